@@ -54,90 +54,33 @@ struct BveF32 {
   }
 };
 
-// FP64 source record shared by the sphere sums: position, q = zeta*A (or f and A for PSE)
+// FP64 source record of the scalar PSE sums
 struct __align__(16) Rec64 {
-  double x, y, z, q;
-  double r;       // second scalar (area for PSE, absolute vorticity for the stream function)
-  long long idx;  // particle index (self-interaction test)
+  double x, y, z, q;  // position and f
+  double r;           // area
+  long long idx;      // particle index
 };
 
 struct BveF64Params {
   const double *x, *y, *z;
   double a2, kden;  // a*a and fl(fl(4 pi) a)
   double *u, *v, *w;
+  const double *q, *area;  // zeta and A
 };
 
-// ASSOC 0: ((a^2 - xi xj) - yi yj) - zi zj   (SphereBVESolver.f90:403-404)
-// ASSOC 1: a^2 - ((xi xj + yi yj) + zi zj)   (SphereBVE.f90:509, sum(xi*xj))
-template <int ASSOC>
-struct BveF64 {
-  struct Tgt {
-    double x, y, z;
-  };
-  struct Acc {
-    double u, v, w;
-  };
-  __device__ static Tgt load(const BveF64Params& p, int64_t i) { return Tgt{p.x[i], p.y[i], p.z[i]}; }
-  __device__ static __forceinline__ void interact(const BveF64Params& p, const Tgt& t,
-                                                  const Rec64& r, Acc& a) {
-    double den;
-    if (ASSOC == 0) {
-      den = __dsub_rn(__dsub_rn(__dsub_rn(p.a2, __dmul_rn(t.x, r.x)), __dmul_rn(t.y, r.y)),
-                      __dmul_rn(t.z, r.z));
-    } else {
-      den = __dsub_rn(p.a2, __dadd_rn(__dadd_rn(__dmul_rn(t.x, r.x), __dmul_rn(t.y, r.y)),
-                                      __dmul_rn(t.z, r.z)));
-    }
-    const double s = -__ddiv_rn(r.q, __dmul_rn(p.kden, den));
-    a.u = __dadd_rn(a.u, __dmul_rn(__dsub_rn(__dmul_rn(t.y, r.z), __dmul_rn(t.z, r.y)), s));
-    a.v = __dadd_rn(a.v, __dmul_rn(__dsub_rn(__dmul_rn(t.z, r.x), __dmul_rn(t.x, r.z)), s));
-    a.w = __dadd_rn(a.w, __dmul_rn(__dsub_rn(__dmul_rn(t.x, r.y), __dmul_rn(t.y, r.x)), s));
-  }
-  __device__ static void store(const BveF64Params& p, int64_t i, int64_t il, const Acc& a) {
-    p.u[il] = a.u;
-    p.v[il] = a.v;
-    p.w[il] = a.w;
-  }
-  static constexpr bool kSkipSelf = true;
-};
+// The FP64 pair itself is BveI64 (seq_i64.cuh).
 
 // ============================================================ planar velocity
 // Reference: planarIncompressibleVelocity, src/PlaneIncompressibleSolver.f90:291-308.
 // (The FP32C form is plane_rel.cuh.)
-struct __align__(16) RecPlane64 {
-  double x, y, q;
-  long long idx;
-};
-
 struct PlaneF64Params {
   const double *x, *y;
   double two_pi, d2;
   double *u, *v;
+  const double *q, *area;  // omega and A
 };
 
-struct PlaneF64 {
-  struct Tgt {
-    double x, y;
-  };
-  struct Acc {
-    double u, v;
-  };
-  __device__ static Tgt load(const PlaneF64Params& p, int64_t i) { return Tgt{p.x[i], p.y[i]}; }
-  __device__ static __forceinline__ void interact(const PlaneF64Params& p, const Tgt& t,
-                                                  const RecPlane64& r, Acc& a) {
-    const double dx = __dsub_rn(t.x, r.x);
-    const double dy = __dsub_rn(t.y, r.y);
-    const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), p.d2);
-    const double s = __ddiv_rn(r.q, __dmul_rn(p.two_pi, r2));
-    a.u = __dsub_rn(a.u, __dmul_rn(dy, s));
-    a.v = __dadd_rn(a.v, __dmul_rn(dx, s));
-  }
-  __device__ static void store(const PlaneF64Params& p, int64_t i, int64_t il, const Acc& a) {
-    p.u[il] = a.u;
-    p.v[il] = a.v;
-  }
-  static constexpr bool kSkipSelf = true;
-};
+// The FP64 pair itself is PlaneI64 (seq_i64.cuh).
 
 // ============================================================ PSE Laplacian
 // Reference: PSESphereLaplacianAtParticles / PSEPlaneLaplacianAtParticles,

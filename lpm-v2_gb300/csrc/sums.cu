@@ -15,6 +15,7 @@
 #include "ops.cuh"
 #include "plane_rel.cuh"
 #include "pse_rel.cuh"
+#include "seq_i64.cuh"
 #include "sort.cuh"
 #include "stream_rel.cuh"
 #include "sums.cuh"
@@ -47,7 +48,6 @@ constexpr int kSweSphereMinB = 2;  // sphere SWE velocity sweep: 2 CTAs per SM (
 // 64-source tiles: the PSE sums' tile cutoff skips 14-25 % more work than with 128 and the
 // sweeps without a cutoff run at the same rate
 constexpr int k64Threads = 128, k64Tile = 64;
-constexpr int kSplit64 = 4;  // lanes per target of the split FP64 sweep (small target sets; 8 was slower)
 
 // ------------------------------------------------------------------ FP64 sequential sweep
 // One thread per target, sources in ascending particle order, one accumulator: the same
@@ -132,87 +132,62 @@ __global__ void __launch_bounds__(k64Threads) seq_fp64_kernel(P p, const Rec* __
   if (valid) Op::store(p, i, il, acc);
 }
 
-// The FP64 sweep for a small target set, S lanes per target.  Lane k of a target's group
-// evaluates sources j = j0 + k of each run of S, on an accumulator of zero, so it holds the
-// term itself (0 + X = X).  The S terms of a run are then added in ascending j, with the same
-// rounding as the sequential sweep, each accumulator component by one lane of the group:
-// lane k keeps components k, k + S, ...  (one FP64 add per lane and term instead of one per
-// component: on GB300's 2 FP64 lanes per clock per SM the adds of all components in every
-// lane cost a quarter of the pipe at S = 4 and three components).  The group's first lane
-// collects the components at the end.  This is for operators whose interact adds exactly one
-// term to each accumulator component (a = a + X, or a = a - X, which is a + (-X)), so the
-// sums stay bit-identical up to the sign of an exact zero.  S times as many warps share the
-// FP64 work.
-template <class Op, class Rec, class P, int S, int THREADS>
-__global__ void __launch_bounds__(THREADS) seq_fp64_split_kernel(P p, const Rec* __restrict__ src,
-                                                                 int64_t ns, int64_t ib, int64_t nt,
-                                                                 int* status) {
-  static_assert(32 % S == 0, "a target's lanes stay in one warp");
-  using Acc = typename Op::Acc;
-  static_assert(sizeof(Acc) % sizeof(double) == 0, "accumulators are doubles");
-  constexpr int NA = static_cast<int>(sizeof(Acc) / sizeof(double));
-  constexpr int NSLOT = (NA + S - 1) / S;  // components per lane
-  __shared__ __align__(128) Rec stage[2][k64Tile];
-  __shared__ __align__(8) uint64_t bars[2];
-  const int k = static_cast<int>(threadIdx.x) % S;
-  const int lane0 = static_cast<int>(threadIdx.x & 31u) - k;  // the group's first lane in the warp
-  const int64_t il = static_cast<int64_t>(blockIdx.x) * (THREADS / S) + threadIdx.x / S;
-  const bool valid = il < nt;
-  const int64_t i = ib + (valid ? il : nt - 1);
-  const typename Op::Tgt t = Op::load(p, i);
-  double slot[NSLOT];  // slot m: component k + m S of the target's sum
-#pragma unroll
-  for (int m = 0; m < NSLOT; ++m) slot[m] = 0.0;
-  const int64_t n_tiles = ceil_div(ns, k64Tile);
-  int64_t tile = 0;
-  pipe_init(bars);
-  uint32_t g = 0;
-  staged_sweep<Rec, k64Tile>(src, 0, n_tiles, stage[0], stage[1], bars, g, status, [&](const Rec* tl) {
-    const int64_t j0 = tile * k64Tile;
-    const int cnt = static_cast<int>(ns - j0 < k64Tile ? ns - j0 : k64Tile);
-    for (int jb = 0; jb < cnt; jb += S) {
-      const int j = jb + k;
-      Acc d{};
-      const bool has = j < cnt && !(Op::kSkipSelf && tl[j < cnt ? j : 0].idx == i);
-      if (has) Op::interact(p, t, tl[j], d);
-      const double* dv = reinterpret_cast<const double*>(&d);
-#pragma unroll
-      for (int q = 0; q < S; ++q) {
-        const bool hq = __shfl_sync(0xffffffffu, has, lane0 + q);
-        double x[NA];
-#pragma unroll
-        for (int c = 0; c < NA; ++c) x[c] = __shfl_sync(0xffffffffu, dv[c], lane0 + q);
-#pragma unroll
-        for (int m = 0; m < NSLOT; ++m) {
-          const int c = k + m * S;
-          double xc = x[0];
-#pragma unroll
-          for (int cc = 1; cc < NA; ++cc) xc = c == cc ? x[cc] : xc;
-          if (hq && c < NA) slot[m] = __dadd_rn(slot[m], xc);
-        }
-      }
+// CTA size of an FP64 sweep over `lanes` threads (one per target, or kSplit64 per target):
+// every CTA does the same work and all of them are resident at once, so an SM's time is its
+// CTA count times the CTA size, and the sweep takes the longest SM's.  Of 128, 64 and 32
+// threads, the size that minimises ceil(CTAs / SMs) x size (the larger on a tie): e.g. at
+// 7,682 targets x 4 lanes, 961 CTAs of 32 threads put at most 7 on an SM (224 thread-slots)
+// where 241 CTAs of 128 put 2 (256).
+int fp64_block_threads(int64_t lanes, int64_t sms) {
+  int best = k64Threads;
+  int64_t best_cost = ceil_div(ceil_div(lanes, k64Threads), sms) * k64Threads;
+  for (int t : {64, 32}) {
+    const int64_t cost = ceil_div(ceil_div(lanes, t), sms) * t;
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = t;
     }
-    ++tile;
-  });
-  Acc acc{};
-  double* av = reinterpret_cast<double*>(&acc);
-#pragma unroll
-  for (int c = 0; c < NA; ++c) av[c] = __shfl_sync(0xffffffffu, slot[c / S], lane0 + c % S);
-  if (valid && k == 0) Op::store(p, i, il, acc);
+  }
+  return best;
 }
 
-// The split sweep at a CTA size of 128, 64 or 32 threads.
-template <class Op, class Rec, class P>
-void launch_split64(int threads, unsigned grid, cudaStream_t stream, const P& p, const Rec* src, int64_t ns,
-                    int64_t ib, int64_t nt, int* status) {
+// Lanes per target of the integer-product sweep: the fewest, from Op::kMinLanes on, that put a warp
+// on every scheduler, at most 8.  kMinLanes is the power of two that holds a lane per component (4
+// BVE, 2 plane), which is as fast as fewer lanes at every size (icos nest 6: 49.1 Ginteractions/s
+// at 4 lanes, 48.5 at 2, 49.2 at 1; quad nest 6: 53.6 at 2, 46.3 at 1).  Below one warp per
+// scheduler twice the lanes win (icos nest 3: 6.5 at 8, 5.0 at 4; quad nest 5: 34.2 at 4, 24.2 at
+// 2), above it they lose (icos nest 4: 27.4 at 4, 23.1 at 8).
+template <class Op>
+int i64_lanes(int64_t nt, int64_t sms) {
+  int s = Op::kMinLanes;
+  while (s < 8 && nt * s < sms * 4 * 32) s *= 2;
+  return s;
+}
+
+template <class Op, int S>
+void launch_i64(const SumJob& job, int64_t sms, const typename Op::Params& p) {
+  const int threads = fp64_block_threads(job.nt * S, sms);
+  const unsigned grid = static_cast<unsigned>(ceil_div(job.nt, threads / S));
+  const typename Op::Rec* src = static_cast<const typename Op::Rec*>(job.src_buf);
   if (threads == 32) {
-    seq_fp64_split_kernel<Op, Rec, P, kSplit64, 32><<<grid, 32, 0, stream>>>(p, src, ns, ib, nt, status);
+    seq_i64_kernel<Op, S, k64Tile, 32><<<grid, 32, 0, job.stream>>>(p, src, job.ns, job.ib, job.nt, job.status);
   } else if (threads == 64) {
-    seq_fp64_split_kernel<Op, Rec, P, kSplit64, 64><<<grid, 64, 0, stream>>>(p, src, ns, ib, nt, status);
+    seq_i64_kernel<Op, S, k64Tile, 64><<<grid, 64, 0, job.stream>>>(p, src, job.ns, job.ib, job.nt, job.status);
   } else {
-    seq_fp64_split_kernel<Op, Rec, P, kSplit64, k64Threads><<<grid, k64Threads, 0, stream>>>(p, src, ns, ib, nt,
-                                                                                             status);
+    seq_i64_kernel<Op, S, k64Tile, k64Threads>
+        <<<grid, k64Threads, 0, job.stream>>>(p, src, job.ns, job.ib, job.nt, job.status);
   }
+}
+
+// The integer-product sweep over the records in job.src_buf.
+template <class Op>
+void launch_i64(const SumJob& job, int64_t sms, const typename Op::Params& p) {
+  const int s = i64_lanes<Op>(job.nt, sms);
+  if constexpr (Op::kMinLanes <= 2) {
+    if (s == 2) return launch_i64<Op, 2>(job, sms, p);
+  }
+  if (s == 4) return launch_i64<Op, 4>(job, sms, p);
+  launch_i64<Op, 8>(job, sms, p);
 }
 
 // The bounding ball (centre, radius) of each FP64 source tile (k64Tile consecutive active
@@ -263,7 +238,7 @@ __global__ void __launch_bounds__(k64Tile) tile_bounds64_kernel(const double* x,
 
 __global__ void prep_rec64_kernel(const double* x, const double* y, const double* z,
                                   const double* s1, const double* area, const int32_t* idx,
-                                  int64_t ns, int pse, Rec64* out) {
+                                  int64_t ns, Rec64* out) {
   const int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (k >= ns) return;
   const int64_t j = idx[k];
@@ -271,13 +246,8 @@ __global__ void prep_rec64_kernel(const double* x, const double* y, const double
   r.x = x[j];
   r.y = y[j];
   r.z = z ? z[j] : 0.0;
-  if (pse) {
-    r.q = s1[j];  // f_j
-    r.r = area[j];
-  } else {
-    r.q = __dmul_rn(s1[j], area[j]);  // zeta_j * A_j, the first product of the Fortran term
-    r.r = 0.0;
-  }
+  r.q = s1[j];  // f_j
+  r.r = area[j];
   r.idx = j;
   out[k] = r;
 }
@@ -289,20 +259,6 @@ __global__ void prep_vec64_kernel(const double* x, const double* y, const double
   if (k >= ns) return;
   const int64_t j = idx[k];
   out[k] = RecVec64{x[j], y[j], z ? z[j] : 0.0, vx[j], vy[j], vz ? vz[j] : 0.0, area[j], static_cast<long long>(j)};
-}
-
-__global__ void prep_plane64_kernel(const double* x, const double* y, const double* omega,
-                                    const double* area, const int32_t* idx, int64_t ns,
-                                    RecPlane64* out) {
-  const int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (k >= ns) return;
-  const int64_t j = idx[k];
-  RecPlane64 r;
-  r.x = x[j];
-  r.y = y[j];
-  r.q = __dmul_rn(omega[j], area[j]);
-  r.idx = j;
-  out[k] = r;
 }
 
 __global__ void prep_stream64_kernel(const double* x, const double* y, const double* z,
@@ -516,7 +472,8 @@ int origin_group(int kind) {
 
 size_t rec_bytes(int kind, int mode) {
   if (mode == LPM_MODE_FP64) {
-    if (kind == kSumPlane) return sizeof(RecPlane64);
+    if (kind == kSumBve || kind == kSumBveMesh) return sizeof(BveI64<0>::Rec);
+    if (kind == kSumPlane) return sizeof(PlaneI64::Rec);
     if (kind == kSumPseDiv || kind == kSumPsePlaneSecond || kind == kSumPsePlaneDdot || kind == kSumPseSphereDdot ||
         kind == kSumSwePlane || kind == kSumSweSphere)
       return sizeof(RecVec64);
@@ -592,25 +549,6 @@ int targets_per_cta(int kind, int shape) {
 }
 
 }  // namespace
-
-// CTA size of an FP64 sweep over `lanes` threads (one per target, or kSplit64 per target):
-// every CTA does the same work and all of them are resident at once, so an SM's time is its
-// CTA count times the CTA size, and the sweep takes the longest SM's.  Of 128, 64 and 32
-// threads, the size that minimises ceil(CTAs / SMs) x size (the larger on a tie): e.g. at
-// 7,682 targets x 4 lanes, 961 CTAs of 32 threads put at most 7 on an SM (224 thread-slots)
-// where 241 CTAs of 128 put 2 (256).
-static int fp64_block_threads(int64_t lanes, int64_t sms) {
-  int best = k64Threads;
-  int64_t best_cost = ceil_div(ceil_div(lanes, k64Threads), sms) * k64Threads;
-  for (int t : {64, 32}) {
-    const int64_t cost = ceil_div(ceil_div(lanes, t), sms) * t;
-    if (cost < best_cost) {
-      best_cost = cost;
-      best = t;
-    }
-  }
-  return best;
-}
 
 int64_t choose_split(int64_t blocks, int64_t tiles, int64_t slots, int64_t max_split) {
   if (blocks < 1) blocks = 1;
@@ -719,14 +657,10 @@ SumPlan plan_sum(int kind, int mode, int64_t ns, int64_t nt, int sm_count, int s
       pl.tperm_offset = align_up(pl.src_bytes, 256);
       pl.src_bytes = pl.tperm_offset + 2 * align_up(static_cast<size_t>(nt) * sizeof(int32_t), 256);
     }
-    // one target per thread and no split (the sum is sequential per target): a target set
-    // too small for one 128-thread CTA per SM takes CTAs of one warp (and, for the BVE and
-    // planar velocity, the split sweep) so that more SMs share the FP64 work.  At one CTA
-    // per SM and above the sequential sweep keeps the FP64 pipe busy (85 % at icos nest 5).
+    // no split: the sum is sequential per target
     const int64_t sms = sm_count > 0 ? sm_count : 152;
-    pl.fp64_small = ceil_div(nt, k64Threads) < sms;
+    pl.sm_count = sms;
     pl.fp64_threads = fp64_block_threads(nt, sms);
-    pl.fp64_split_threads = fp64_block_threads(nt * kSplit64, sms);
     pl.nsplit = 1;
     pl.tiles_per_chunk = pl.n_tiles;
     pl.partial_bytes = 0;
@@ -944,8 +878,6 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
   if (job.mode == LPM_MODE_FP64) {
     const int t64 = plan.fp64_threads;
     const unsigned g = static_cast<unsigned>(ceil_div(job.nt, t64));
-    const int ts = plan.fp64_split_threads;
-    const unsigned gs = static_cast<unsigned>(ceil_div(job.nt, ts / kSplit64));  // the split sweep's grid
     Fp64Cut cut;
     if (fp64_cutoff(job.kind, &cut.unit)) {
       TileBall* bounds = reinterpret_cast<TileBall*>(
@@ -969,44 +901,31 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
     switch (job.kind) {
       case kSumBve:
       case kSumBveMesh: {
-        prep_rec64_kernel<<<prep_grid_ns, pb, 0, job.stream>>>(job.x, job.y, job.z, job.s1, job.area,
-                                                               job.src_idx, job.ns, 0,
-                                                               static_cast<Rec64*>(job.src_buf));
         BveF64Params p{job.x, job.y, job.z, job.radius * job.radius, (4.0 * kPi) * job.radius,
-                       job.out0, job.out1, job.out2};
-        const Rec64* src = static_cast<const Rec64*>(job.src_buf);
-        if (plan.fp64_small) {
-          // a small target set: kSplit64 lanes per target (the terms in parallel, the sum in order)
-          if (job.kind == kSumBve) {
-            launch_split64<BveF64<0>, Rec64>(ts, gs, job.stream, p, src, job.ns, job.ib, job.nt, job.status);
-          } else {
-            launch_split64<BveF64<1>, Rec64>(ts, gs, job.stream, p, src, job.ns, job.ib, job.nt, job.status);
-          }
-        } else if (job.kind == kSumBve) {
-          seq_fp64_kernel<BveF64<0>, Rec64><<<g, t64, 0, job.stream>>>(p, src, job.ns, job.ib, job.nt, job.status);
+                       job.out0, job.out1, job.out2, job.s1, job.area};
+        if (job.kind == kSumBve) {
+          prep_bve_i64_kernel<0><<<prep_grid_ns, pb, 0, job.stream>>>(
+              job.x, job.y, job.z, job.s1, job.area, job.src_idx, job.ns, static_cast<BveI64<0>::Rec*>(job.src_buf));
+          launch_i64<BveI64<0>>(job, plan.sm_count, p);
         } else {
-          seq_fp64_kernel<BveF64<1>, Rec64><<<g, t64, 0, job.stream>>>(p, src, job.ns, job.ib, job.nt, job.status);
+          prep_bve_i64_kernel<1><<<prep_grid_ns, pb, 0, job.stream>>>(
+              job.x, job.y, job.z, job.s1, job.area, job.src_idx, job.ns, static_cast<BveI64<1>::Rec*>(job.src_buf));
+          launch_i64<BveI64<1>>(job, plan.sm_count, p);
         }
         break;
       }
       case kSumPlane: {
-        prep_plane64_kernel<<<prep_grid_ns, pb, 0, job.stream>>>(job.x, job.y, job.s1, job.area, job.src_idx,
-                                                                 job.ns, static_cast<RecPlane64*>(job.src_buf));
-        PlaneF64Params p{job.x, job.y, 2.0 * kPi, job.delta * job.delta, job.out0, job.out1};
-        const RecPlane64* src = static_cast<const RecPlane64*>(job.src_buf);
-        if (plan.fp64_small) {
-          launch_split64<PlaneF64, RecPlane64>(ts, gs, job.stream, p, src, job.ns, job.ib, job.nt, job.status);
-        } else {
-          seq_fp64_kernel<PlaneF64, RecPlane64><<<g, t64, 0, job.stream>>>(p, src, job.ns, job.ib, job.nt,
-                                                                           job.status);
-        }
+        PlaneF64Params p{job.x, job.y, 2.0 * kPi, job.delta * job.delta, job.out0, job.out1, job.s1, job.area};
+        prep_plane_i64_kernel<<<prep_grid_ns, pb, 0, job.stream>>>(
+            job.x, job.y, job.s1, job.area, job.src_idx, job.ns, static_cast<PlaneI64::Rec*>(job.src_buf));
+        launch_i64<PlaneI64>(job, plan.sm_count, p);
         break;
       }
       case kSumPseK8Geo:
       case kSumPseGaussChord:
       case kSumPseK8Chord: {
         prep_rec64_kernel<<<prep_grid_ns, pb, 0, job.stream>>>(job.x, job.y, job.z, job.s1, job.area,
-                                                               job.src_idx, job.ns, 1,
+                                                               job.src_idx, job.ns,
                                                                static_cast<Rec64*>(job.src_buf));
         const double eps2 = job.eps * job.eps;
         PseF64Params p{job.x, job.y, job.z, job.s1, job.eps, eps2, 1.0 / eps2, job.radius, job.out0};
@@ -1031,7 +950,7 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
         if (job.kind == kSumPseGrad) {
           p.scale = 1.0 / eps2;  // MultiplyFieldByScalar(scalarGrad, 1/eps**2)
           prep_rec64_kernel<<<prep_grid_ns, pb, 0, job.stream>>>(job.x, job.y, job.z, job.s1, job.area,
-                                                                 job.src_idx, job.ns, 1,
+                                                                 job.src_idx, job.ns,
                                                                  static_cast<Rec64*>(job.src_buf));
           seq_fp64_kernel<PseGradF64, Rec64><<<g, t64, 0, job.stream>>>(
               p, static_cast<const Rec64*>(job.src_buf), job.ns, job.ib, job.nt, job.status, cut);
@@ -1065,7 +984,7 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
       case kSumPseInterpPlane:
       case kSumPseInterpSphere: {
         prep_rec64_kernel<<<prep_grid_ns, pb, 0, job.stream>>>(job.x, job.y, job.z, job.s1, job.area,
-                                                               job.src_idx, job.ns, 1,
+                                                               job.src_idx, job.ns,
                                                                static_cast<Rec64*>(job.src_buf));
         const double eps2 = job.eps * job.eps;
         PseExtF64Params p{job.x, job.y, job.z, job.s1, job.s2, job.s3, job.eps, eps2, job.eps * eps2,
