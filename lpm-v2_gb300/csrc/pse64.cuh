@@ -1,0 +1,529 @@
+// pse64.cuh -- the FP64 PSE sums: every target over the sources within r = 7, each pair in a form
+// without square root, arctangent or division.
+//
+// Every PSE kernel is E(q) (k0 + k1 q + k2 q^2 + k3 q^3) with q = r^2 = (distance / eps)^2 and
+// E = exp(-q), so a pair needs q, not r:
+//  - chord distances: q = |d|^2 / eps^2;
+//  - great-circle distances: q = theta^2 (a / eps)^2, with theta^2 = 4 asin^2(c / 2) a polynomial
+//    in the squared chord c^2 of the unit directions (Chebyshev interpolation of the function,
+//    within 2^-57 of it; for c up to 0.45, 1.14 and, with the supplement beyond 90 degrees, 2);
+//  - the constants' divisions (eps, 3, pi) are folded into k0..k3;
+//  - E by table and polynomial (P. T. P. Tang, Table-driven implementation of the exponential
+//    function, ACM TOMS 15, 1989): with s = 256 q / ln 2 and i = round(s),
+//    E = 2^-(i / 256) 2^-((s - i) / 256), a table of 256 powers and a polynomial of degree 4
+//    (remainder 4e-17).
+// That is about 32 FP64 instructions a pair for K8 of the great-circle distance, where the
+// reference's expressions take about 150.  The results agree with the reference's to its own rounding
+// (1e-15 of the largest; its exp and atan2 are not CUDA's either), the sum is in the reference's
+// ascending order, one accumulator per target.
+//
+// At r >= 7 each kernel (its polynomial times e^-49) is below 1e-14 of its peak, and the sum
+// leaves those pairs out:
+//  - a CTA is one warp of 32 targets (in curve order, so close together).  It lists the source
+//    tiles whose ball is within reach of its targets' ball, in ascending order;
+//  - in a tile each lane tests its own distance to all 64 sources in FP32 (offsets from the tile's
+//    centre, so that the test is tight wherever the set lies; the limit is widened by the
+//    roundings) and then evaluates only its own: the lanes of a warp work on different sources.
+// A pair with a particle that has no direction (at the origin of a sphere) or no finite position
+// takes the reference's expressions as they stand (Op::Plain), as do all pairs of a reach beyond
+// the polynomials' range.
+//
+// Bound by the FP64 pipe (2 lanes per clock per SM).
+#pragma once
+
+#include "engine.cuh"
+#include "ops.cuh"
+
+namespace lpm {
+
+constexpr int kPse64Tile = 64;
+constexpr int kPse64Stages = 2;
+constexpr int kPse64List = 256;  // tiles listed between two sweeps of a CTA
+constexpr double kPse64Reach = 7.0;
+
+// How q comes from the squared distance in the test space.
+enum { kAngNone = 0, kAngNear = 1, kAngFar = 2, kAngWide = 3 };
+constexpr double kAngNearMax = 0.45, kAngFarMax = 1.13, kAngWideMax = 3.15;  // the largest reach (radians)
+
+__device__ constexpr double kAngleNear[9] = {
+    1.0, 0x1.5555555555528p-4, 0x1.6c16c16c21e06p-7, 0x1.d41d41c32ba47p-10,
+    0x1.4ce1a15af67f7p-12, 0x1.f85ad3dada806p-15, 0x1.8f6711cda66fbp-17, 0x1.3f8984fdb3592p-19,
+    0x1.4ec6f7c8931fap-21};
+__device__ constexpr double kAngleFar[16] = {
+    1.0, 0x1.555555555557dp-4, 0x1.6c16c16c11ab3p-7, 0x1.d41d41d8335acp-10,
+    0x1.4ce19a0a71d18p-12, 0x1.f85dcd29033f7p-15, 0x1.8f0a574238fa0p-17, 0x1.46295d746cb2fp-19,
+    0x1.0de9a232ae937p-21, 0x1.f9dd6ab3b186cp-24, 0x1.678acc7911957p-27, 0x1.3377469b31787p-26,
+    -0x1.0ae9181a54911p-27, 0x1.33d9687615ab8p-28, -0x1.473d3bf6189d6p-30, 0x1.b0132cb15d416p-33};
+__device__ constexpr double kAngleWide[21] = {
+    1.0, 0x1.5555555555539p-4, 0x1.6c16c16c1ad97p-7, 0x1.d41d41d067cd5p-10,
+    0x1.4ce19bc9b7a71p-12, 0x1.f85d52f2033f3p-15, 0x1.8f156d8a2a07fp-17, 0x1.45748f36e7d1bp-19,
+    0x1.16520badb72a2p-21, 0x1.63956078e7873p-24, 0x1.2e4682196d94dp-24, -0x1.0a0a04610a73dp-24,
+    0x1.46010a5d2b1e0p-24, -0x1.169cae1127812p-24, 0x1.7be9e29dcebbcp-25, -0x1.8c9704395f2ddp-26,
+    0x1.3a3073c170e3dp-27, -0x1.6c742eaa3376ap-29, 0x1.2590182d74208p-31, -0x1.2625ff01947f3p-34,
+    0x1.187c20d375371p-38};
+
+// ------------------------------------------------------------------ inputs
+struct __align__(32) TileBall {
+  double x, y, z, r;  // centre and radius in the test space
+};
+
+// The source side of a sum: positions, up to three fields, areas.
+struct Pse64Src {
+  const double *x, *y, *z, *s1, *s2, *s3, *area;
+};
+
+struct Pse64Args {
+  double c;               // s = 256 q / ln 2 per squared distance (chord) or squared angle
+  double k0, k1, k2, k3;  // the kernel as a polynomial in s, with the constants that divide it
+  double reach;           // of the cutoff, in the test space
+  int unit;               // 1: the test space is unit directions
+  int all_plain;          // 1: every pair in the reference's expressions
+  const double *x, *y, *z;  // target positions (z may be null)
+  Pse64Src src;
+  const TileBall* bounds;
+  const float4* side;
+  const double* powers;   // 2^-(i / 256)
+  const int32_t* tperm;   // the targets in curve order, or null: index order
+  int64_t ns, n_tiles, ib, nt;
+  int* status;
+};
+
+// The point of particle i in the test space.  A point at the origin of a sphere has no direction
+// (and atan2(0, 0) puts it at distance 0 from everything); it becomes NaN, which every test reads
+// as "in reach".
+__device__ __forceinline__ double3 cut_point(const double* x, const double* y, const double* z, int64_t i, int unit) {
+  double3 q = make_double3(x[i], y[i], z ? z[i] : 0.0);
+  if (unit) {
+    const double nq = sqrt(q.x * q.x + q.y * q.y + q.z * q.z);
+    const double inv = nq > 0.0 ? 1.0 / nq : __longlong_as_double(0x7ff8000000000000LL);
+    q = make_double3(q.x * inv, q.y * inv, q.z * inv);
+  }
+  return q;
+}
+
+// Whether a test point is NaN or infinite in some component.
+__device__ __forceinline__ bool odd_point(const double3& q) {
+  const double v = (q.x - q.x) + (q.y - q.y) + (q.z - q.z);
+  return !(v == 0.0);
+}
+
+// ------------------------------------------------------------------ a pair's kernel value
+template <int N>
+__device__ __forceinline__ double horner(const double (&c)[N], double v) {
+  double p = c[N - 1];
+#pragma unroll
+  for (int k = N - 2; k >= 0; --k) p = fma(p, v, c[k]);
+  return p;
+}
+
+// 4 asin^2(c / 2) from v = c^2.
+template <int ANG>
+__device__ __forceinline__ double angle2(double v) {
+  if (ANG == kAngNone) return v;
+  if (ANG == kAngNear) return v * horner(kAngleNear, v);
+  if (ANG == kAngFar) return v * horner(kAngleFar, v);
+  if (v <= 2.0) return v * horner(kAngleWide, v);
+  // beyond 90 degrees: the supplement's angle (a kernel that reaches there has eps < 0.45, so
+  // that near the antipode, where this loses digits, it is below e^-40)
+  const double w = fmax(4.0 - v, 0.0);
+  const double t = 3.14159265358979323846 - sqrt(w * horner(kAngleWide, w));
+  return t * t;
+}
+
+template <bool POLY>
+__device__ __forceinline__ double pse64_kernel_value(const Pse64Args& a, double s, const double* powers) {
+  const double big = 6755399441055744.0;  // 1.5 x 2^52: the sum's low word is round(s)
+  const double t = s + big;
+  const int i = __double2loint(t);
+  const double f = s - (t - big);
+  double p = 0x1.3b2ab6fba4e77p-39;  // (-ln 2 / 256)^n / n!
+  p = fma(p, f, -0x1.c6b08d704a0c0p-29);
+  p = fma(p, f, 0x1.ebfbdff82c58fp-19);
+  p = fma(p, f, -0x1.62e42fefa39efp-9);
+  p = fma(p, f, 1.0);
+  const double e = powers[i & 255] * p;
+  const double scaled = __hiloint2double(__double2hiint(e) - ((i >> 8) << 20), __double2loint(e));
+  const double w = POLY ? scaled * fma(fma(fma(a.k3, s, a.k2), s, a.k1), s, a.k0) : scaled * a.k0;
+  // s >= 2^18 (q >= 709; only where the FP32 test underflowed) has left the exponent's range
+  return __double2hiint(s) >= 0x41100000 ? 0.0 : w;
+}
+
+// ------------------------------------------------------------------ operators
+// An operator's record holds the test point (x, y, z), the fields that its pairs need, the
+// particle's index and whether it is odd (odd_point).  add() adds the pair's terms, with w the kernel
+// value over the operator's powers of eps; the accumulators are Plain's, in its units.
+struct Pse64Op {
+  static constexpr bool kPoly = true;   // false: a plain Gaussian
+  static constexpr bool kUnit = false;  // true: great-circle distances
+};
+
+template <int KIND>
+struct PseLap64 : Pse64Op {
+  using Plain = PseF64<KIND>;
+  using Params = PseF64Params;
+  using Acc = typename Plain::Acc;
+  static constexpr int kDim = KIND == kPseK8Chord ? 2 : 3;
+  static constexpr bool kPoly = KIND != kPseGaussChord;
+  static constexpr bool kUnit = KIND == kPseK8Geodesic;
+  struct __align__(16) Rec {
+    double x, y, z, f, area;
+    int32_t idx, odd;
+  };
+  struct Tgt {
+    double f;
+  };
+  __device__ static void fill(Rec& r, const Pse64Src& s, int64_t j) {
+    r.f = s.s1[j];
+    r.area = s.area[j];
+  }
+  __device__ static Tgt load(const Params& p, int64_t i) { return Tgt{p.f[i]}; }
+  __device__ static __forceinline__ void add(const Tgt& t, const Rec& r, double, double, double, double w, Acc& a) {
+    a.l = fma((r.f - t.f) * r.area, w, a.l);
+  }
+  __device__ static Rec64 plain_record(const Pse64Src& s, int64_t j) {
+    return Rec64{s.x[j], s.y[j], s.z ? s.z[j] : 0.0, s.s1[j], s.area[j], static_cast<long long>(j)};
+  }
+};
+
+template <bool SPHERE>
+struct PseInterp64 : Pse64Op {
+  static constexpr bool kUnit = SPHERE;
+  using Plain = PseInterpF64<SPHERE>;
+  using Params = PseExtF64Params;
+  using Acc = typename Plain::Acc;
+  static constexpr int kDim = 3;
+  struct __align__(16) Rec {
+    double x, y, z, fa;
+    int32_t idx, odd;
+    double pad;
+  };
+  struct Tgt {};
+  __device__ static void fill(Rec& r, const Pse64Src& s, int64_t j) {
+    r.fa = __dmul_rn(s.s1[j], s.area[j]);
+    r.pad = 0.0;
+  }
+  __device__ static Tgt load(const Params&, int64_t) { return Tgt{}; }
+  __device__ static __forceinline__ void add(const Tgt&, const Rec& r, double, double, double, double w, Acc& a) {
+    a.s = fma(r.fa, w, a.s);
+  }
+  __device__ static Rec64 plain_record(const Pse64Src& s, int64_t j) { return PseLap64<0>::plain_record(s, j); }
+};
+
+struct PsePlaneGrad64 : Pse64Op {
+  using Plain = PsePlaneGradF64;
+  using Params = PseExtF64Params;
+  using Acc = Plain::Acc;
+  static constexpr int kDim = 2;
+  using Rec = PseLap64<0>::Rec;
+  struct Tgt {
+    double f;
+  };
+  __device__ static void fill(Rec& r, const Pse64Src& s, int64_t j) { PseLap64<0>::fill(r, s, j); }
+  __device__ static Tgt load(const Params& p, int64_t i) { return Tgt{p.s1[i]}; }
+  __device__ static __forceinline__ void add(const Tgt& t, const Rec& r, double dx, double dy, double, double w,
+                                             Acc& a) {
+    const double g = (r.f + t.f) * r.area * w;
+    a.gx = fma(g, dx, a.gx);
+    a.gy = fma(g, dy, a.gy);
+  }
+  __device__ static Rec64 plain_record(const Pse64Src& s, int64_t j) { return PseLap64<0>::plain_record(s, j); }
+};
+
+template <class Base>  // PsePlaneSecondF64 or PsePlaneDdotF64
+struct PlaneD464 : Pse64Op {
+  using Plain = Base;
+  using Params = PseExtF64Params;
+  using Acc = typename Base::Acc;
+  static constexpr int kDim = 2;
+  struct __align__(16) Rec {
+    double x, y, z, va, vb, area;
+    int32_t idx, odd;
+    double pad[3];  // an odd number of 16-byte units: lanes that read different records share fewer banks
+  };
+  struct Tgt {
+    double a, b;
+  };
+  __device__ static void fill(Rec& r, const Pse64Src& s, int64_t j) {
+    r.va = s.s1[j];
+    r.vb = s.s2[j];
+    r.area = s.area[j];
+    r.pad[0] = r.pad[1] = r.pad[2] = 0.0;
+  }
+  __device__ static Tgt load(const Params& p, int64_t i) { return Tgt{p.s1[i], p.s2[i]}; }
+  __device__ static __forceinline__ void add(const Tgt& t, const Rec& r, double dx, double dy, double, double w,
+                                             Acc& a) {
+    const double g = r.area * w, gx = g * dx, gy = g * dy, sa = r.va + t.a, sb = r.vb + t.b;
+    a.ax = fma(sa, gx, a.ax);
+    a.ay = fma(sa, gy, a.ay);
+    a.bx = fma(sb, gx, a.bx);
+    a.by = fma(sb, gy, a.by);
+  }
+  __device__ static RecVec64 plain_record(const Pse64Src& s, int64_t j) {
+    return RecVec64{s.x[j], s.y[j], s.z ? s.z[j] : 0.0, s.s1[j], s.s2[j], s.s3 ? s.s3[j] : 0.0, s.area[j],
+                    static_cast<long long>(j)};
+  }
+};
+
+// The sphere's first-derivative operators use the raw differences x_i - x_j beside the angle.
+struct PseVecRec64 {
+  double x, y, z, rx, ry, rz, a, b, c, area;
+  int32_t idx, odd;
+};
+
+template <class Base>
+struct PseSphereVec64 : Pse64Op {
+  static constexpr bool kUnit = true;
+  using Plain = Base;
+  using Acc = typename Base::Acc;
+  static constexpr int kDim = 3;
+  struct __align__(16) Rec : PseVecRec64 {
+    double pad[3];
+  };
+  __device__ static void fill(Rec& r, const Pse64Src& s, int64_t j) {
+    r.rx = s.x[j];
+    r.ry = s.y[j];
+    r.rz = s.z[j];
+    r.a = s.s1[j];
+    r.b = s.s2 ? s.s2[j] : 0.0;
+    r.c = s.s3 ? s.s3[j] : 0.0;
+    r.area = s.area[j];
+    r.pad[0] = r.pad[1] = r.pad[2] = 0.0;
+  }
+};
+
+struct PseGrad64 : PseSphereVec64<PseGradF64> {
+  using Params = PseVecF64Params;
+  struct Tgt {
+    double x, y, z, f;
+  };
+  __device__ static Tgt load(const Params& p, int64_t i) { return Tgt{p.x[i], p.y[i], p.z[i], p.f[i]}; }
+  __device__ static __forceinline__ void add(const Tgt& t, const Rec& r, double, double, double, double w, Acc& a) {
+    const double g = (r.a + t.f) * r.area * w;
+    a.g0 = fma(g, t.x - r.rx, a.g0);
+    a.g1 = fma(g, t.y - r.ry, a.g1);
+    a.g2 = fma(g, t.z - r.rz, a.g2);
+  }
+  __device__ static Rec64 plain_record(const Pse64Src& s, int64_t j) { return PseLap64<0>::plain_record(s, j); }
+};
+
+struct PseDiv64 : PseSphereVec64<PseDivF64> {
+  using Params = PseVecF64Params;
+  struct Tgt {
+    double x, y, z, vx, vy, vz;
+  };
+  __device__ static Tgt load(const Params& p, int64_t i) {
+    return Tgt{p.x[i], p.y[i], p.z[i], p.vx[i], p.vy[i], p.vz[i]};
+  }
+  // (P d) . V = d . V - (x . d) (x . V)
+  __device__ static __forceinline__ void add(const Tgt& t, const Rec& r, double, double, double, double w, Acc& a) {
+    const double dx = t.x - r.rx, dy = t.y - r.ry, dz = t.z - r.rz;
+    const double vx = r.a + t.vx, vy = r.b + t.vy, vz = r.c + t.vz;
+    const double dv = fma(dx, vx, fma(dy, vy, dz * vz));
+    const double xd = fma(t.x, dx, fma(t.y, dy, t.z * dz)), xv = fma(t.x, vx, fma(t.y, vy, t.z * vz));
+    a.d = fma(fma(-xd, xv, dv) * r.area, w, a.d);
+  }
+  __device__ static RecVec64 plain_record(const Pse64Src& s, int64_t j) {
+    return PlaneD464<PsePlaneSecondF64>::plain_record(s, j);
+  }
+};
+
+struct PseSphereDdot64 : PseSphereVec64<PseSphereDdotF64> {
+  using Params = PseExtF64Params;
+  struct Tgt {
+    double x, y, z, u, v;
+  };
+  __device__ static Tgt load(const Params& p, int64_t i) {
+    return Tgt{p.x[i], p.y[i], p.z[i], p.s1[i], p.s2[i]};
+  }
+  __device__ static __forceinline__ void add(const Tgt& t, const Rec& r, double, double, double, double w, Acc& a) {
+    const double g = r.area * w;
+    const double gx = g * (t.x - r.rx), gy = g * (t.y - r.ry), gz = g * (t.z - r.rz);
+    const double su = r.a + t.u, sv = r.b + t.v, sw = r.c + t.v;  // w_j with v_i, as the reference
+    a.ux = fma(su, gx, a.ux);
+    a.uy = fma(su, gy, a.uy);
+    a.uz = fma(su, gz, a.uz);
+    a.vx = fma(sv, gx, a.vx);
+    a.vy = fma(sv, gy, a.vy);
+    a.vz = fma(sv, gz, a.vz);
+    a.wx = fma(sw, gx, a.wx);
+    a.wy = fma(sw, gy, a.wy);
+    a.wz = fma(sw, gz, a.wz);
+  }
+  __device__ static RecVec64 plain_record(const Pse64Src& s, int64_t j) {
+    return PlaneD464<PsePlaneSecondF64>::plain_record(s, j);
+  }
+};
+
+// A pair in the reference's expressions.
+template <class Op>
+__device__ __noinline__ typename Op::Acc pse64_plain(const typename Op::Params& p, const Pse64Src& s, int64_t i,
+                                                     int64_t j, typename Op::Acc a) {
+  Op::Plain::interact(p, Op::Plain::load(p, i), Op::plain_record(s, j), a);
+  return a;
+}
+
+// ------------------------------------------------------------------ prep
+// Records, FP32 offsets from the tile's centre and ball of one tile; one CTA per tile.  The radius
+// is widened by 1e-9 of itself and of the centre's size, which covers the rounding of the tests; an
+// odd particle leaves the centre alone and makes the radius infinite.  CTA 0 also writes the
+// powers.
+template <class Op>
+__global__ void __launch_bounds__(kPse64Tile) pse64_prep_kernel(Pse64Src s, const int32_t* idx, int64_t ns, int unit,
+                                                                typename Op::Rec* out, float4* side, TileBall* bounds,
+                                                                double* powers) {
+  __shared__ double red[4][kPse64Tile];
+  const int tid = threadIdx.x;
+  const int64_t k = static_cast<int64_t>(blockIdx.x) * kPse64Tile + tid;
+  const bool valid = k < ns;
+  const int32_t j = valid ? idx[k] : 0;
+  const double3 q = valid ? cut_point(s.x, s.y, s.z, j, unit) : make_double3(0.0, 0.0, 0.0);
+  const bool odd = odd_point(q);
+  red[0][tid] = odd ? 0.0 : q.x;
+  red[1][tid] = odd ? 0.0 : q.y;
+  red[2][tid] = odd ? 0.0 : q.z;
+  red[3][tid] = valid && !odd ? 1.0 : 0.0;
+  __syncthreads();
+  for (int w = kPse64Tile / 2; w > 0; w >>= 1) {
+    if (tid < w) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c) red[c][tid] += red[c][tid + w];
+    }
+    __syncthreads();
+  }
+  const double cnt = red[3][0] > 0.0 ? red[3][0] : 1.0;
+  const double cx = red[0][0] / cnt, cy = red[1][0] / cnt, cz = red[2][0] / cnt;
+  const double dx = q.x - cx, dy = q.y - cy, dz = q.z - cz;
+  __syncthreads();
+  red[0][tid] = odd ? __longlong_as_double(0x7ff0000000000000LL)
+                    : valid ? sqrt(dx * dx + dy * dy + dz * dz) : 0.0;
+  __syncthreads();
+  for (int w = kPse64Tile / 2; w > 0; w >>= 1) {
+    if (tid < w) red[0][tid] = fmax(red[0][tid], red[0][tid + w]);
+    __syncthreads();
+  }
+  if (tid == 0) {
+    const double sz = fabs(cx) + fabs(cy) + fabs(cz);
+    bounds[blockIdx.x] = TileBall{cx, cy, cz, red[0][0] * (1.0 + 1e-9) + 1e-9 * sz};
+  }
+  typename Op::Rec r{};
+  if (valid) {
+    Op::fill(r, s, j);
+    r.x = q.x;
+    r.y = q.y;
+    r.z = q.z;
+    r.idx = j;
+    r.odd = odd ? 1 : 0;
+  }
+  out[k] = r;
+  const float nan = __int_as_float(0x7fffffff);
+  side[k] = odd ? make_float4(nan, nan, nan, 0.f)
+                : make_float4(static_cast<float>(dx), static_cast<float>(dy), static_cast<float>(dz), 0.f);
+  if (blockIdx.x == 0) {
+    for (int e = tid; e < 256; e += kPse64Tile) powers[e] = exp2(-static_cast<double>(e) / 256.0);
+  }
+}
+
+// ------------------------------------------------------------------ sweep
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+template <class Op, int ANG>
+__global__ void __launch_bounds__(32) pse64_sweep_kernel(typename Op::Params p, Pse64Args a,
+                                                         const typename Op::Rec* __restrict__ src) {
+  using Rec = typename Op::Rec;
+  using Acc = typename Op::Acc;
+  __shared__ TilePipe<Rec, kPse64Tile, kPse64Stages, float4, kPse64Tile> pp;
+  __shared__ double powers[256];
+  __shared__ int32_t list[kPse64List];
+  const int lane = threadIdx.x;
+  const int64_t k = static_cast<int64_t>(blockIdx.x) * 32 + lane;
+  const bool valid = k < a.nt;
+  const int64_t kk = valid ? k : a.nt - 1;
+  const int64_t i = a.tperm ? static_cast<int64_t>(a.tperm[kk]) : a.ib + kk;
+  const typename Op::Tgt t = Op::load(p, i);
+  const double3 tp = cut_point(a.x, a.y, a.z, i, a.unit);
+  const bool odd = a.all_plain || odd_point(tp);
+  for (int e = lane; e < 256; e += 32) powers[e] = a.powers[e];
+  tile_pipe_init(pp);  // (synchronises)
+  // the ball around the warp's targets (NaN or infinite: in reach of everything)
+  const double wx = warp_sum(tp.x) / 32.0, wy = warp_sum(tp.y) / 32.0, wz = warp_sum(tp.z) / 32.0;
+  double far = (tp.x - wx) * (tp.x - wx) + (tp.y - wy) * (tp.y - wy) + (tp.z - wz) * (tp.z - wz);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) far = fmax(far, __shfl_xor_sync(0xffffffffu, far, o));
+  const double wr = sqrt(far) * (1.0 + 1e-9) + 1e-9 * (fabs(wx) + fabs(wy) + fabs(wz)) + a.reach;
+
+  Acc acc{};
+  uint32_t g = 0;
+  int cnt = 0;
+  for (int64_t w0 = 0; w0 < a.n_tiles; w0 += 32) {
+    const int64_t tl = w0 + lane;
+    bool in = tl < a.n_tiles;
+    if (in) {
+      const TileBall b = a.bounds[tl];
+      const double dx = wx - b.x, dy = wy - b.y, dz = wz - b.z, lim = wr + b.r;
+      in = !(dx * dx + dy * dy + dz * dz > lim * lim);
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, in);
+    if (in) list[cnt + __popc(m & ((1u << lane) - 1u))] = static_cast<int32_t>(tl);
+    cnt += __popc(m);
+    if (cnt <= kPse64List - 32 && w0 + 32 < a.n_tiles) continue;
+    __syncwarp();
+    int q = 0;
+    const bool ok = warp_sweep_tiles(
+        src, [&](int64_t e) { return static_cast<int64_t>(list[e]); }, cnt, pp, g, a.status, default_wait(), a.side,
+        [&](const Rec* rec, const float4* side) {
+          const int64_t tile = list[q++];
+          const TileBall b = a.bounds[tile];
+          const float ox = static_cast<float>(tp.x - b.x), oy = static_cast<float>(tp.y - b.y),
+                      oz = static_cast<float>(tp.z - b.z);
+          // the offsets' and the test's roundings: a few 2^-24 of the offsets, which are at most
+          // the target's own and the tile's radius (a tile beyond the reach of all is rejected
+          // whatever its size)
+          const float lim = static_cast<float>(a.reach) * 1.00001f +
+                            1e-6f * (fabsf(ox) + fabsf(oy) + fabsf(oz) + static_cast<float>(b.r));
+          const float lim2 = lim * lim;
+          const int64_t left = a.ns - tile * kPse64Tile;
+          uint32_t mask[2];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t bits = 0;
+#pragma unroll 8
+            for (int j = 0; j < 32; ++j) {
+              const float4 s = side[h * 32 + j];
+              const float dx = ox - s.x, dy = oy - s.y, dz = oz - s.z;
+              if (!(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > lim2)) bits |= 1u << j;
+            }
+            if (odd) bits = 0xffffffffu;
+            const int64_t n = left - 32 * h;  // sources of the tile's half
+            mask[h] = n >= 32 ? bits : (n > 0 ? bits & ((1u << n) - 1u) : 0u);
+          }
+#pragma unroll 1
+          for (int h = 0; h < 2; ++h) {
+            uint32_t bits = mask[h];
+            while (bits) {
+              const int j = __ffs(static_cast<int>(bits)) - 1;
+              bits &= bits - 1u;
+              const Rec& r = rec[h * 32 + j];
+              if (odd || r.odd) {
+                acc = pse64_plain<Op>(p, a.src, i, r.idx, acc);
+                continue;
+              }
+              const double dx = tp.x - r.x, dy = tp.y - r.y, dz = Op::kDim == 3 ? tp.z - r.z : 0.0;
+              const double d2 = Op::kDim == 3 ? fma(dx, dx, fma(dy, dy, dz * dz)) : fma(dx, dx, dy * dy);
+              const double w = pse64_kernel_value<Op::kPoly>(a, angle2<ANG>(d2) * a.c, powers);
+              Op::add(t, r, dx, dy, dz, w, acc);
+            }
+          }
+          __syncwarp();
+        });
+    if (!ok) return;  // a wait gave up: the status word is set and the outputs are not used
+    cnt = 0;
+    __syncwarp();
+  }
+  if (valid) Op::Plain::store(p, i, i - a.ib, acc);
+}
+
+}  // namespace lpm

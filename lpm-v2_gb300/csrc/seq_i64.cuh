@@ -282,6 +282,19 @@ __global__ void __launch_bounds__(THREADS) seq_i64_kernel(typename Op::Params p,
   double slot[NSLOT];  // slot m: component k + m S of the target's sum
 #pragma unroll
   for (int m = 0; m < NSLOT; ++m) slot[m] = 0.0;
+  // The terms of the last run: their additions, a chain of S, wait for the next run's products to
+  // run beside.
+  double run[S][NSLOT];
+#pragma unroll
+  for (int q = 0; q < S; ++q)
+#pragma unroll
+    for (int m = 0; m < NSLOT; ++m) run[q][m] = 0.0;
+  auto add_run = [&]() {
+#pragma unroll
+    for (int q = 0; q < S; ++q)
+#pragma unroll
+      for (int m = 0; m < NSLOT; ++m) slot[m] = __dadd_rn(slot[m], run[q][m]);
+  };
   const int64_t n_tiles = ceil_div(ns, TILE);
   int64_t tile = 0;
   pipe_init(bars);
@@ -296,8 +309,11 @@ __global__ void __launch_bounds__(THREADS) seq_i64_kernel(typename Op::Params p,
       // the warp's targets or sources ask for care, or a pair turns out to need it
       bool care = __any_sync(0xffffffffu, (t.flags | r.flags) != 0);
       if (!care) {
+        add_run();
         const bool ok = Op::template terms<false>(p, t, r, x) || !has;
         care = __any_sync(0xffffffffu, !ok);
+      } else {
+        add_run();
       }
       if (care) {
         const bool ok = Op::template terms<true>(p, t, r, x);
@@ -313,15 +329,15 @@ __global__ void __launch_bounds__(THREADS) seq_i64_kernel(typename Op::Params p,
         for (int c = 0; c < NA; ++c) y[c] = __shfl_sync(0xffffffffu, x[c], lane0 + q);
 #pragma unroll
         for (int m = 0; m < NSLOT; ++m) {
-          double yc = y[m * S];
+          run[q][m] = y[m * S];
 #pragma unroll
-          for (int c = m * S + 1; c < NA && c < (m + 1) * S; ++c) yc = k == c - m * S ? y[c] : yc;
-          slot[m] = __dadd_rn(slot[m], yc);
+          for (int c = m * S + 1; c < NA && c < (m + 1) * S; ++c) run[q][m] = k == c - m * S ? y[c] : run[q][m];
         }
       }
     }
     ++tile;
   });
+  add_run();
   double acc[NA];
 #pragma unroll
   for (int c = 0; c < NA; ++c) acc[c] = __shfl_sync(0xffffffffu, slot[c / S], lane0 + c % S);

@@ -14,6 +14,7 @@
 #include "engine.cuh"
 #include "ops.cuh"
 #include "plane_rel.cuh"
+#include "pse64.cuh"
 #include "pse_rel.cuh"
 #include "seq_i64.cuh"
 #include "sort.cuh"
@@ -45,94 +46,42 @@ constexpr int kBetaThreads = 128, kBetaTpt = 4, kBetaTile = 256, kBetaMinB = 4;
 constexpr int kSweMinB = 3;        // planar SWE velocity sweep: 128 x 4 targets, 3 CTAs per SM
 constexpr int kSweSphereMinB = 2;  // sphere SWE velocity sweep: 2 CTAs per SM (no spills; 10 % over 3)
 // FP64 sequential sweep shape
-// 64-source tiles: the PSE sums' tile cutoff skips 14-25 % more work than with 128 and the
-// sweeps without a cutoff run at the same rate
+// (64-source tiles for the PSE sums' cutoff; the sweeps without one run at the same rate at 128)
 constexpr int k64Threads = 128, k64Tile = 64;
 
 // ------------------------------------------------------------------ FP64 sequential sweep
 // One thread per target, sources in ascending particle order, one accumulator: the same
 // summation order as the Fortran j loop, hence bit-identical sums.
-//
-// The PSE kernels all carry exp(-r^2), r = distance / eps: at r >= 7 each kernel (its
-// polynomial times e^-49) is below 1e-14 of its peak, far below the FP64 sums' 1e-12
-// agreement with the reference (whose exp is not CUDA's anyway; the all-pairs oracle tests
-// hold that bound with the cutoff).  For those a warp skips a whole source tile when every
-// one of its targets is farther than the tile's radius plus `reach` from the tile's centre,
-// in the space the distance is measured in:
-//   - unit directions for the great-circle kernels (reach 7 eps / radius; the angle is never
-//     shorter than the chord of the unit directions);
-//   - raw positions for the chord and planar ones (reach 7 eps).
-// The pairs it keeps are summed in the reference's order.  The FP32C sweeps cut at the same
-// r^2 = 49 (PseRel::kCutR2).
-struct __align__(32) TileBall {
-  double x, y, z, r;  // centre and radius in the test space
-};
-
-struct Fp64Cut {
-  const TileBall* bounds = nullptr;  // per source tile
-  const double *x = nullptr, *y = nullptr, *z = nullptr;  // target positions (z may be null)
-  double reach = 0.0;
-  int unit = 0;  // 1: the test space is unit directions
-  // the targets in curve order (nt global indices), or nullptr for index order: a warp then
-  // holds 32 targets close together and skips more tiles; each target's own sum is unchanged
-  const int32_t* tperm = nullptr;
-};
-
-// The point of particle i in the test space.  A point at the origin has no direction (and
-// atan2(0, 0) puts it at distance 0 from everything): it becomes NaN, which the tests below
-// read as "in reach", so nothing is skipped for it.
-__device__ __forceinline__ double3 cut_point(const double* x, const double* y, const double* z, int64_t i,
-                                             int unit) {
-  double3 q = make_double3(x[i], y[i], z ? z[i] : 0.0);
-  if (unit) {
-    const double nq = sqrt(q.x * q.x + q.y * q.y + q.z * q.z);
-    const double inv = nq > 0.0 ? 1.0 / nq : __longlong_as_double(0x7ff8000000000000LL);
-    q = make_double3(q.x * inv, q.y * inv, q.z * inv);
-  }
-  return q;
-}
-
 template <class Op, class Rec, class P>
 __global__ void __launch_bounds__(k64Threads) seq_fp64_kernel(P p, const Rec* __restrict__ src,
                                                               int64_t ns, int64_t ib, int64_t nt,
-                                                              int* status, Fp64Cut cut = Fp64Cut{}) {
+                                                              int* status) {
   __shared__ __align__(128) Rec stage[2][k64Tile];
   __shared__ __align__(8) uint64_t bars[2];
-  const int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const bool valid = k < nt;
-  const int64_t i = cut.tperm ? static_cast<int64_t>(cut.tperm[valid ? k : nt - 1]) : ib + (valid ? k : nt - 1);
-  const int64_t il = i - ib;  // the target's place in the outputs
+  const int64_t il = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const bool valid = il < nt;
+  const int64_t i = ib + (valid ? il : nt - 1);
   const typename Op::Tgt t = Op::load(p, i);
   typename Op::Acc acc{};
   const int64_t n_tiles = ceil_div(ns, k64Tile);
-  const double3 tp = cut.bounds ? cut_point(cut.x, cut.y, cut.z, i, cut.unit) : make_double3(0.0, 0.0, 0.0);
   int64_t tile = 0;
   pipe_init(bars);
   uint32_t g = 0;
   staged_sweep<Rec, k64Tile>(src, 0, n_tiles, stage[0], stage[1], bars, g, status,
                              [&](const Rec* tl) {
-                               bool run = true;
-                               if (cut.bounds) {
-                                 const TileBall b = cut.bounds[tile];
-                                 const double dx = tp.x - b.x, dy = tp.y - b.y, dz = tp.z - b.z;
-                                 const double lim = b.r + cut.reach;
-                                 run = __any_sync(0xffffffffu, !(dx * dx + dy * dy + dz * dz > lim * lim));
-                               }
-                               if (run) {
-                                 const int64_t j0 = tile * k64Tile;
-                                 const int cnt = static_cast<int>(ns - j0 < k64Tile ? ns - j0 : k64Tile);
-                                 for (int j = 0; j < cnt; ++j) {
-                                   const Rec& r = tl[j];
-                                   if (Op::kSkipSelf && r.idx == i) continue;
-                                   Op::interact(p, t, r, acc);
-                                 }
+                               const int64_t j0 = tile * k64Tile;
+                               const int cnt = static_cast<int>(ns - j0 < k64Tile ? ns - j0 : k64Tile);
+                               for (int j = 0; j < cnt; ++j) {
+                                 const Rec& r = tl[j];
+                                 if (Op::kSkipSelf && r.idx == i) continue;
+                                 Op::interact(p, t, r, acc);
                                }
                                ++tile;
                              });
   if (valid) Op::store(p, i, il, acc);
 }
 
-// CTA size of an FP64 sweep over `lanes` threads (one per target, or kSplit64 per target):
+// CTA size of an FP64 sweep over `lanes` threads (one or several per target):
 // every CTA does the same work and all of them are resident at once, so an SM's time is its
 // CTA count times the CTA size, and the sweep takes the longest SM's.  Of 128, 64 and 32
 // threads, the size that minimises ceil(CTAs / SMs) x size (the larger on a tie): e.g. at
@@ -190,67 +139,8 @@ void launch_i64(const SumJob& job, int64_t sms, const typename Op::Params& p) {
   launch_i64<Op, 8>(job, sms, p);
 }
 
-// The bounding ball (centre, radius) of each FP64 source tile (k64Tile consecutive active
-// sources) in the cutoff's test space; one CTA of k64Tile threads per tile.  The radius is
-// widened by 1e-9 of itself and of the centre's size, which covers the rounding of the test.
-__global__ void __launch_bounds__(k64Tile) tile_bounds64_kernel(const double* x, const double* y, const double* z,
-                                                                const int32_t* idx, int64_t ns, int unit,
-                                                                TileBall* bounds) {
-  __shared__ double red[4][k64Tile];
-  const int tid = threadIdx.x;
-  const int64_t k = static_cast<int64_t>(blockIdx.x) * k64Tile + tid;
-  const bool valid = k < ns;
-  const double3 q = valid ? cut_point(x, y, z, idx[k], unit) : make_double3(0.0, 0.0, 0.0);
-  // a source without a direction (NaN point) leaves the centre alone and makes the radius
-  // infinite: the tile is in reach of every target
-  const bool dirless = valid && !(q.x == q.x && q.y == q.y && q.z == q.z);
-  red[0][tid] = dirless ? 0.0 : q.x;
-  red[1][tid] = dirless ? 0.0 : q.y;
-  red[2][tid] = dirless ? 0.0 : q.z;
-  red[3][tid] = valid && !dirless ? 1.0 : 0.0;
-  __syncthreads();
-  for (int w = k64Tile / 2; w > 0; w >>= 1) {
-    if (tid < w) {
-#pragma unroll
-      for (int c = 0; c < 4; ++c) red[c][tid] += red[c][tid + w];
-    }
-    __syncthreads();
-  }
-  const double cnt = red[3][0] > 0.0 ? red[3][0] : 1.0;
-  const double cx = red[0][0] / cnt, cy = red[1][0] / cnt, cz = red[2][0] / cnt;
-  __syncthreads();
-  red[0][tid] = dirless ? __longlong_as_double(0x7ff0000000000000LL)
-                : valid ? sqrt((q.x - cx) * (q.x - cx) + (q.y - cy) * (q.y - cy) + (q.z - cz) * (q.z - cz))
-                        : 0.0;
-  __syncthreads();
-  for (int w = k64Tile / 2; w > 0; w >>= 1) {
-    if (tid < w) red[0][tid] = fmax(red[0][tid], red[0][tid + w]);
-    __syncthreads();
-  }
-  if (tid == 0) {
-    const double sz = fabs(cx) + fabs(cy) + fabs(cz);
-    bounds[blockIdx.x] = TileBall{cx, cy, cz, red[0][0] * (1.0 + 1e-9) + 1e-9 * sz};
-  }
-}
-
 // ------------------------------------------------------------------ prep kernels
 // Gather the active particles (src_idx) into source records; records ns..npad-1 are inert.
-
-__global__ void prep_rec64_kernel(const double* x, const double* y, const double* z,
-                                  const double* s1, const double* area, const int32_t* idx,
-                                  int64_t ns, Rec64* out) {
-  const int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (k >= ns) return;
-  const int64_t j = idx[k];
-  Rec64 r;
-  r.x = x[j];
-  r.y = y[j];
-  r.z = z ? z[j] : 0.0;
-  r.q = s1[j];  // f_j
-  r.r = area[j];
-  r.idx = j;
-  out[k] = r;
-}
 
 __global__ void prep_vec64_kernel(const double* x, const double* y, const double* z, const double* vx,
                                   const double* vy, const double* vz, const double* area, const int32_t* idx,
@@ -394,8 +284,7 @@ __global__ void finish_stream_kernel(const double* partial, int64_t nsplit, int6
   }
 }
 
-// The FP64 kinds whose kernel decays as exp(-r^2) (the PSE operators), whose sweep skips
-// source tiles beyond r = 10; *unit tells whether the distance is a great-circle one.
+// The FP64 kinds whose kernel decays as exp(-r^2) (the PSE operators, pse64.cuh); *unit tells whether the distance is a great-circle one.
 bool fp64_cutoff(int kind, int* unit) {
   switch (kind) {
     case kSumPseK8Geo:
@@ -419,6 +308,7 @@ bool fp64_cutoff(int kind, int* unit) {
 }
 
 int tile_of(int kind, int mode) {
+  static_assert(kPse64Tile == k64Tile, "one tile size");
   if (mode == LPM_MODE_FP64) return k64Tile;
   switch (kind) {
     case kSumBve:
@@ -474,12 +364,12 @@ size_t rec_bytes(int kind, int mode) {
   if (mode == LPM_MODE_FP64) {
     if (kind == kSumBve || kind == kSumBveMesh) return sizeof(BveI64<0>::Rec);
     if (kind == kSumPlane) return sizeof(PlaneI64::Rec);
-    if (kind == kSumPseDiv || kind == kSumPsePlaneSecond || kind == kSumPsePlaneDdot || kind == kSumPseSphereDdot ||
-        kind == kSumSwePlane || kind == kSumSweSphere)
-      return sizeof(RecVec64);
+    if (kind == kSumPseGrad || kind == kSumPseDiv || kind == kSumPseSphereDdot) return sizeof(PseGrad64::Rec);
+    if (kind == kSumPsePlaneSecond || kind == kSumPsePlaneDdot) return sizeof(PlaneD464<PsePlaneSecondF64>::Rec);
+    if (kind == kSumSwePlane || kind == kSumSweSphere) return sizeof(RecVec64);
     if (kind == kSumSphereStream || kind == kSumPlaneStream || kind == kSumBetaPlane || kind == kSumBetaStream)
       return sizeof(RecStream64);
-    return sizeof(Rec64);
+    return sizeof(PseLap64<kPseK8Geodesic>::Rec);  // the scalar PSE sums
   }
   switch (kind) {
     case kSumBve:
@@ -651,9 +541,10 @@ SumPlan plan_sum(int kind, int mode, int64_t ns, int64_t nt, int sm_count, int s
   if (mode == LPM_MODE_FP64) {
     int unit = 0;
     if (fp64_cutoff(kind, &unit)) {
-      // the tiles' bounding balls follow the records, then the targets' curve order (two
-      // lists of nt int32, as for the FP32C PSE sums)
-      pl.src_bytes = align_up(pl.src_bytes, 256) + static_cast<size_t>(pl.n_tiles) * sizeof(TileBall);
+      // FP32 offsets, balls and the table of powers follow the records, then the targets' curve
+      // order (two lists of nt int32, as for the FP32C PSE sums)
+      pl.src_bytes = align_up(pl.src_bytes, 256) + static_cast<size_t>(pl.n_tiles) * kPse64Tile * sizeof(float4) +
+                     static_cast<size_t>(pl.n_tiles) * sizeof(TileBall) + 256 * sizeof(double);
       pl.tperm_offset = align_up(pl.src_bytes, 256);
       pl.src_bytes = pl.tperm_offset + 2 * align_up(static_cast<size_t>(nt) * sizeof(int32_t), 256);
     }
@@ -867,6 +758,81 @@ int launch_plane_pse_rel(const SumJob& job, const SumPlan& plan, int64_t npad) {
 }
 }  // namespace
 
+namespace {
+// The PSE kernels over pi as polynomials in q = r^2 (times e^-q).
+constexpr double kK8[4] = {40.0, -40.0, 10.0, -2.0 / 3.0};      // bivariateLaplacianKernel8
+constexpr double kK1[4] = {-20.0, 20.0, -5.0, 1.0 / 3.0};       // bivariateFirstDerivativeKernel8
+constexpr double kDelta8[4] = {4.0, -6.0, 2.0, -1.0 / 6.0};     // bivariateDeltaKernel8
+constexpr double kGauss[4] = {4.0, 0.0, 0.0, 0.0};
+
+// An FP64 PSE sum (pse64.cuh): the targets' curve order, prep and sweep.  `over` divides the kernel
+// (the operator's powers of eps).
+template <class Op>
+int launch_pse64(const SumJob& job, const SumPlan& plan, const typename Op::Params& p, const double (&poly)[4],
+                 double over) {
+  using Rec = typename Op::Rec;
+  const int64_t npad = plan.n_tiles * kPse64Tile;
+  char* base = static_cast<char*>(job.src_buf);
+  const size_t side_off = align_up(static_cast<size_t>(npad) * rec_bytes(job.kind, job.mode), 256);
+  const size_t ball_off = side_off + static_cast<size_t>(npad) * sizeof(float4);
+  const size_t power_off = ball_off + static_cast<size_t>(plan.n_tiles) * sizeof(TileBall);
+  static_assert(kPse64Tile * sizeof(float4) % 256 == 0 && sizeof(TileBall) % 8 == 0, "aligned parts");
+  Rec* recs = reinterpret_cast<Rec*>(base);
+  float4* side = reinterpret_cast<float4*>(base + side_off);
+  TileBall* bounds = reinterpret_cast<TileBall*>(base + ball_off);
+  double* powers = reinterpret_cast<double*>(base + power_off);
+
+  Pse64Args a;
+  int unit = 0;
+  fp64_cutoff(job.kind, &unit);
+  const double per_s = std::log(2.0) / 256.0;  // q of one unit of s
+  const double scale = unit ? job.radius / job.eps : 1.0 / job.eps;
+  a.c = scale * scale / per_s;
+  a.k0 = poly[0] / kPi / over;
+  a.k1 = poly[1] * per_s / kPi / over;
+  a.k2 = poly[2] * per_s * per_s / kPi / over;
+  a.k3 = poly[3] * per_s * per_s * per_s / kPi / over;
+  a.reach = kPse64Reach * job.eps / (unit ? job.radius : 1.0);
+  a.unit = unit;
+  a.all_plain = unit && a.reach > kAngWideMax;
+  a.x = job.x;
+  a.y = job.y;
+  a.z = job.z;
+  a.src = Pse64Src{job.x, job.y, job.z, job.s1, job.s2, job.s3, job.area};
+  a.bounds = bounds;
+  a.side = side;
+  a.powers = powers;
+  a.ns = job.ns;
+  a.n_tiles = plan.n_tiles;
+  a.ib = job.ib;
+  a.nt = job.nt;
+  a.status = job.status;
+  // targets in curve order when the job brings sort scratch (the host-buffer calls)
+  const bool sphere = unit || (job.kind == kSumPseGaussChord && job.z);
+  LPM_TRY(sorted_targets(job, plan, [&](const int32_t* in, int32_t* out) {
+    return sphere ? curve_sort(job.stream, job.nt, in, job.x, job.y, job.z, 1.0 / job.radius, job.sort_scratch,
+                               job.sort_bytes, out)
+                  : curve_sort2d(job.stream, job.nt, in, job.x, job.y, job.sort_scratch, job.sort_bytes, out);
+  }, &a.tperm));
+  pse64_prep_kernel<Op><<<static_cast<unsigned>(plan.n_tiles), kPse64Tile, 0, job.stream>>>(
+      a.src, job.src_idx, job.ns, unit, recs, side, bounds, powers);
+  const unsigned grid = static_cast<unsigned>(ceil_div(job.nt, 32));
+  if constexpr (Op::kUnit) {
+    if (a.reach <= kAngNearMax) {
+      pse64_sweep_kernel<Op, kAngNear><<<grid, 32, 0, job.stream>>>(p, a, recs);
+    } else if (a.reach <= kAngFarMax) {
+      pse64_sweep_kernel<Op, kAngFar><<<grid, 32, 0, job.stream>>>(p, a, recs);
+    } else {
+      pse64_sweep_kernel<Op, kAngWide><<<grid, 32, 0, job.stream>>>(p, a, recs);
+    }
+  } else {
+    pse64_sweep_kernel<Op, kAngNone><<<grid, 32, 0, job.stream>>>(p, a, recs);
+  }
+  LPM_CUDA_TRY(cudaGetLastError());
+  return LPM_OK;
+}
+}  // namespace
+
 int launch_sum(const SumJob& job, const SumPlan& plan) {
   const int pb = 256;
   const unsigned prep_grid_ns = static_cast<unsigned>(ceil_div(job.ns > 0 ? job.ns : 1, pb));
@@ -878,26 +844,6 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
   if (job.mode == LPM_MODE_FP64) {
     const int t64 = plan.fp64_threads;
     const unsigned g = static_cast<unsigned>(ceil_div(job.nt, t64));
-    Fp64Cut cut;
-    if (fp64_cutoff(job.kind, &cut.unit)) {
-      TileBall* bounds = reinterpret_cast<TileBall*>(
-          static_cast<char*>(job.src_buf) +
-          align_up(static_cast<size_t>(plan.n_tiles) * k64Tile * rec_bytes(job.kind, job.mode), 256));
-      tile_bounds64_kernel<<<static_cast<unsigned>(plan.n_tiles), k64Tile, 0, job.stream>>>(
-          job.x, job.y, job.z, job.src_idx, job.ns, cut.unit, bounds);
-      cut.bounds = bounds;
-      cut.x = job.x;
-      cut.y = job.y;
-      cut.z = job.z;
-      cut.reach = std::sqrt(static_cast<double>(PseRel::kCutR2)) * job.eps / (cut.unit ? job.radius : 1.0);
-      // targets in curve order when the job brings sort scratch (the host-buffer calls)
-      const bool sphere = cut.unit || (job.kind == kSumPseGaussChord && job.z);
-      LPM_TRY(sorted_targets(job, plan, [&](const int32_t* in, int32_t* out) {
-        return sphere ? curve_sort(job.stream, job.nt, in, job.x, job.y, job.z, 1.0 / job.radius, job.sort_scratch,
-                                   job.sort_bytes, out)
-                      : curve_sort2d(job.stream, job.nt, in, job.x, job.y, job.sort_scratch, job.sort_bytes, out);
-      }, &cut.tperm));
-    }
     switch (job.kind) {
       case kSumBve:
       case kSumBveMesh: {
@@ -924,23 +870,11 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
       case kSumPseK8Geo:
       case kSumPseGaussChord:
       case kSumPseK8Chord: {
-        prep_rec64_kernel<<<prep_grid_ns, pb, 0, job.stream>>>(job.x, job.y, job.z, job.s1, job.area,
-                                                               job.src_idx, job.ns,
-                                                               static_cast<Rec64*>(job.src_buf));
         const double eps2 = job.eps * job.eps;
         PseF64Params p{job.x, job.y, job.z, job.s1, job.eps, eps2, 1.0 / eps2, job.radius, job.out0};
-        const Rec64* src = static_cast<const Rec64*>(job.src_buf);
-        if (job.kind == kSumPseK8Geo) {
-          seq_fp64_kernel<PseF64<kPseK8Geodesic>, Rec64><<<g, t64, 0, job.stream>>>(
-              p, src, job.ns, job.ib, job.nt, job.status, cut);
-        } else if (job.kind == kSumPseGaussChord) {
-          seq_fp64_kernel<PseF64<kPseGaussChord>, Rec64><<<g, t64, 0, job.stream>>>(
-              p, src, job.ns, job.ib, job.nt, job.status, cut);
-        } else {
-          seq_fp64_kernel<PseF64<kPseK8Chord>, Rec64><<<g, t64, 0, job.stream>>>(
-              p, src, job.ns, job.ib, job.nt, job.status, cut);
-        }
-        break;
+        if (job.kind == kSumPseK8Geo) return launch_pse64<PseLap64<kPseK8Geodesic>>(job, plan, p, kK8, eps2);
+        if (job.kind == kSumPseGaussChord) return launch_pse64<PseLap64<kPseGaussChord>>(job, plan, p, kGauss, eps2);
+        return launch_pse64<PseLap64<kPseK8Chord>>(job, plan, p, kK8, eps2);
       }
       case kSumPseGrad:
       case kSumPseDiv: {
@@ -949,20 +883,10 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
                           job.eps * eps2, job.radius, 0.0, job.out0, job.out1, job.out2};
         if (job.kind == kSumPseGrad) {
           p.scale = 1.0 / eps2;  // MultiplyFieldByScalar(scalarGrad, 1/eps**2)
-          prep_rec64_kernel<<<prep_grid_ns, pb, 0, job.stream>>>(job.x, job.y, job.z, job.s1, job.area,
-                                                                 job.src_idx, job.ns,
-                                                                 static_cast<Rec64*>(job.src_buf));
-          seq_fp64_kernel<PseGradF64, Rec64><<<g, t64, 0, job.stream>>>(
-              p, static_cast<const Rec64*>(job.src_buf), job.ns, job.ib, job.nt, job.status, cut);
-        } else {
-          p.scale = 1.0 / job.eps;  // MultiplyFieldByScalar(divergence, 1/eps)
-          prep_vec64_kernel<<<prep_grid_ns, pb, 0, job.stream>>>(job.x, job.y, job.z, job.s1, job.s2, job.s3,
-                                                                 job.area, job.src_idx, job.ns,
-                                                                 static_cast<RecVec64*>(job.src_buf));
-          seq_fp64_kernel<PseDivF64, RecVec64><<<g, t64, 0, job.stream>>>(
-              p, static_cast<const RecVec64*>(job.src_buf), job.ns, job.ib, job.nt, job.status, cut);
+          return launch_pse64<PseGrad64>(job, plan, p, kK1, eps2);
         }
-        break;
+        p.scale = 1.0 / job.eps;  // MultiplyFieldByScalar(divergence, 1/eps)
+        return launch_pse64<PseDiv64>(job, plan, p, kK1, job.eps * eps2);
       }
       case kSumSphereStream:
       case kSumPlaneStream: {
@@ -982,29 +906,28 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
       }
       case kSumPsePlaneGrad:
       case kSumPseInterpPlane:
-      case kSumPseInterpSphere: {
-        prep_rec64_kernel<<<prep_grid_ns, pb, 0, job.stream>>>(job.x, job.y, job.z, job.s1, job.area,
-                                                               job.src_idx, job.ns,
-                                                               static_cast<Rec64*>(job.src_buf));
-        const double eps2 = job.eps * job.eps;
-        PseExtF64Params p{job.x, job.y, job.z, job.s1, job.s2, job.s3, job.eps, eps2, job.eps * eps2,
-                          job.radius, job.radius2, 0.0, 1.0 / job.eps, job.out0, job.out1, job.out2, job.out3};
-        const Rec64* src = static_cast<const Rec64*>(job.src_buf);
-        if (job.kind == kSumPsePlaneGrad) {
-          seq_fp64_kernel<PsePlaneGradF64, Rec64><<<g, t64, 0, job.stream>>>(p, src, job.ns, job.ib, job.nt,
-                                                                                    job.status, cut);
-        } else if (job.kind == kSumPseInterpPlane) {
-          seq_fp64_kernel<PseInterpF64<false>, Rec64><<<g, t64, 0, job.stream>>>(p, src, job.ns, job.ib,
-                                                                                        job.nt, job.status, cut);
-        } else {
-          seq_fp64_kernel<PseInterpF64<true>, Rec64><<<g, t64, 0, job.stream>>>(p, src, job.ns, job.ib,
-                                                                                       job.nt, job.status, cut);
-        }
-        break;
-      }
+      case kSumPseInterpSphere:
       case kSumPsePlaneSecond:
       case kSumPsePlaneDdot:
-      case kSumPseSphereDdot:
+      case kSumPseSphereDdot: {
+        const double eps2 = job.eps * job.eps, eps3 = job.eps * eps2;
+        PseExtF64Params p{job.x, job.y, job.z, job.s1, job.s2, job.s3, job.eps, eps2, eps3,
+                          job.radius, job.radius2, 0.0, 1.0 / job.eps, job.out0, job.out1, job.out2, job.out3};
+        switch (job.kind) {
+          case kSumPsePlaneGrad:
+            return launch_pse64<PsePlaneGrad64>(job, plan, p, kK1, eps3);
+          case kSumPseInterpPlane:
+            return launch_pse64<PseInterp64<false>>(job, plan, p, kDelta8, eps2);
+          case kSumPseInterpSphere:
+            return launch_pse64<PseInterp64<true>>(job, plan, p, kDelta8, eps2);
+          case kSumPsePlaneSecond:
+            return launch_pse64<PlaneD464<PsePlaneSecondF64>>(job, plan, p, kK1, eps3);
+          case kSumPsePlaneDdot:
+            return launch_pse64<PlaneD464<PsePlaneDdotF64>>(job, plan, p, kK1, eps3);
+          default:
+            return launch_pse64<PseSphereDdot64>(job, plan, p, kK1, eps3);
+        }
+      }
       case kSumSwePlane:
       case kSumSweSphere: {
         prep_vec64_kernel<<<prep_grid_ns, pb, 0, job.stream>>>(job.x, job.y, job.z, job.s1, job.s2, job.s3,
@@ -1014,29 +937,14 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
         PseExtF64Params p{job.x, job.y, job.z, job.s1, job.s2, job.s3, job.eps, eps2, job.eps * eps2,
                           job.radius, job.radius2, 0.0, 1.0 / job.eps, job.out0, job.out1, job.out2, job.out3};
         const RecVec64* src = static_cast<const RecVec64*>(job.src_buf);
-        switch (job.kind) {
-          case kSumPsePlaneSecond:
-            seq_fp64_kernel<PsePlaneSecondF64, RecVec64><<<g, t64, 0, job.stream>>>(p, src, job.ns, job.ib,
-                                                                                          job.nt, job.status, cut);
-            break;
-          case kSumPsePlaneDdot:
-            seq_fp64_kernel<PsePlaneDdotF64, RecVec64><<<g, t64, 0, job.stream>>>(p, src, job.ns, job.ib,
-                                                                                        job.nt, job.status, cut);
-            break;
-          case kSumPseSphereDdot:
-            seq_fp64_kernel<PseSphereDdotF64, RecVec64><<<g, t64, 0, job.stream>>>(p, src, job.ns, job.ib,
-                                                                                         job.nt, job.status, cut);
-            break;
-          case kSumSwePlane:
-            p.k0 = 2.0 * kPi;  // 2.0_kreal * PI
-            seq_fp64_kernel<SwePlaneF64, RecVec64><<<g, t64, 0, job.stream>>>(p, src, job.ns, job.ib,
-                                                                                    job.nt, job.status);
-            break;
-          default:
-            p.k0 = ((4.0 * kPi) * job.radius) * job.radius;  // 4.0_kreal * PI * radius * radius
-            seq_fp64_kernel<SweSphereF64, RecVec64><<<g, t64, 0, job.stream>>>(p, src, job.ns, job.ib,
-                                                                                     job.nt, job.status);
-            break;
+        if (job.kind == kSumSwePlane) {
+          p.k0 = 2.0 * kPi;  // 2.0_kreal * PI
+          seq_fp64_kernel<SwePlaneF64, RecVec64><<<g, t64, 0, job.stream>>>(p, src, job.ns, job.ib, job.nt,
+                                                                            job.status);
+        } else {
+          p.k0 = ((4.0 * kPi) * job.radius) * job.radius;  // 4.0_kreal * PI * radius * radius
+          seq_fp64_kernel<SweSphereF64, RecVec64><<<g, t64, 0, job.stream>>>(p, src, job.ns, job.ib, job.nt,
+                                                                             job.status);
         }
         break;
       }
