@@ -24,9 +24,10 @@
 //  - each lane tests its own distance to the 64 sources of each listed tile in FP32 (offsets from
 //    the tile's centre, so that the test is tight wherever the set lies; the limit is widened by
 //    the roundings) and keeps a bit per source;
-//  - then each lane walks its own bits through up to 64 tiles: the lanes of a warp work on
-//    different sources, and take about as many each.  At cubed nest 6 a warp takes 1.04 x the mean
-//    number of pairs in reach of a target; tile by tile it took 1.31 x, whole tiles 1.9 x.
+//  - then each lane walks its own bits through up to 48 tiles, two pairs at a time: the lanes of a
+//    warp work on different sources, and take about as many each.  At cubed nest 6 a warp takes
+//    1.02 x the mean number of pairs in reach of a target; tile by tile it would take 1.31 x, whole
+//    tiles 1.9 x.  Two pairs, because a warp alone waits about 80 clocks for each FP64 result.
 // A pair with a particle that has no direction (at the origin of a sphere) or no finite position
 // takes the reference's expressions as they stand (Op::Plain), as do all pairs of a reach beyond
 // the polynomials' range.
@@ -41,7 +42,8 @@ namespace lpm {
 
 constexpr int kPse64Tile = 64;
 constexpr int kPse64Stages = 2;
-constexpr int kPse64List = 64;  // tiles listed and tested before their pairs are evaluated
+constexpr int kPse64List = 64;  // tiles listed before they are tested
+constexpr int kPse64Mine = 48;  // tiles with sources of its own that a lane holds before they are evaluated
 constexpr double kPse64Reach = 7.0;
 
 // How q comes from the squared distance in the test space.
@@ -439,7 +441,8 @@ __global__ void __launch_bounds__(32) pse64_sweep_kernel(typename Op::Params p, 
   using Rec = typename Op::Rec;
   using Acc = typename Op::Acc;
   __shared__ TilePipe<float4, kPse64Tile, kPse64Stages> pp;
-  __shared__ uint64_t mine[kPse64List][32];  // the lanes' sources of a listed tile
+  __shared__ uint64_t mine[kPse64Mine][32];   // the lanes' sources, a tile's at a time
+  __shared__ int32_t tile_of[kPse64Mine][32];  // and of which tile
   __shared__ double powers[256];
   __shared__ int32_t list[kPse64List];
   const int lane = threadIdx.x;
@@ -460,6 +463,53 @@ __global__ void __launch_bounds__(32) pse64_sweep_kernel(typename Op::Params p, 
   const double wr = sqrt(far) * (1.0 + 1e-9) + 1e-9 * (fabs(wx) + fabs(wy) + fabs(wz)) + a.reach;
 
   Acc acc{};
+  int held = 0;  // entries of mine and tile_of that this lane holds
+  // Evaluates the held sources in ascending order.
+  auto evaluate = [&]() {
+    int e = 0;
+    uint64_t bits = 0;
+    const Rec* base = src;
+    // the lane's next source, or null
+    auto next = [&]() -> const Rec* {
+      if (bits == 0) {
+        if (e == held) return nullptr;
+        bits = mine[e][lane];  // never zero
+        base = src + static_cast<int64_t>(tile_of[e][lane]) * kPse64Tile;
+        ++e;
+      }
+      const int j = __ffsll(static_cast<long long>(bits)) - 1;
+      bits &= bits - 1;
+      return base + j;
+    };
+    const Rec *at0 = next(), *at1 = next();
+    Rec r0 = *(at0 ? at0 : src), r1 = *(at1 ? at1 : src);
+    while (at0) {
+      const Rec n0 = r0, n1 = r1;
+      const bool two = at1 != nullptr;
+      at0 = next();
+      at1 = next();
+      r0 = *(at0 ? at0 : src);  // on their way while this pair of pairs is evaluated
+      r1 = *(at1 ? at1 : src);
+      if (odd || n0.odd || n1.odd) {
+        acc = pse64_plain<Op>(p, a.src, i, n0.idx, acc);
+        if (two) acc = pse64_plain<Op>(p, a.src, i, n1.idx, acc);
+        continue;
+      }
+      const double x0 = tp.x - n0.x, y0 = tp.y - n0.y, z0 = Op::kDim == 3 ? tp.z - n0.z : 0.0;
+      const double x1 = tp.x - n1.x, y1 = tp.y - n1.y, z1 = Op::kDim == 3 ? tp.z - n1.z : 0.0;
+      const double q0 = Op::kDim == 3 ? fma(x0, x0, fma(y0, y0, z0 * z0)) : fma(x0, x0, y0 * y0);
+      const double q1 = Op::kDim == 3 ? fma(x1, x1, fma(y1, y1, z1 * z1)) : fma(x1, x1, y1 * y1);
+      const double w0 = pse64_kernel_value<Op::kPoly>(a, angle2<ANG>(q0) * a.c, powers);
+      const double w1 = pse64_kernel_value<Op::kPoly>(a, angle2<ANG>(q1) * a.c, powers);
+      Op::add(t, n0, x0, y0, z0, w0, acc);
+      Acc more = acc;
+      Op::add(t, n1, x1, y1, z1, w1, more);
+      if (two) acc = more;
+    }
+    held = 0;
+    __syncwarp();
+  };
+
   uint32_t g = 0;
   int cnt = 0;
   for (int64_t w0 = 0; w0 < a.n_tiles; w0 += 32) {
@@ -503,37 +553,19 @@ __global__ void __launch_bounds__(32) pse64_sweep_kernel(typename Op::Params p, 
             const int64_t n = left - 32 * h;
             half[h] = n >= 32 ? bits : (n > 0 ? bits & ((1u << n) - 1u) : 0u);
           }
-          mine[q++][lane] = (static_cast<uint64_t>(half[1]) << 32) | half[0];
+          ++q;
+          if ((half[0] | half[1]) != 0) {
+            mine[held][lane] = (static_cast<uint64_t>(half[1]) << 32) | half[0];
+            tile_of[held][lane] = static_cast<int32_t>(tile);
+            ++held;
+          }
+          if (__any_sync(0xffffffffu, held == kPse64Mine)) evaluate();
         });
     if (!ok) return;  // a wait gave up: the status word is set and the outputs are not used
-    int e = -1;
-    uint64_t bits = 0;
-    // the next source of this lane, or null
-    auto next = [&]() -> const Rec* {
-      while (bits == 0 && e + 1 < cnt) bits = mine[++e][lane];
-      if (bits == 0) return nullptr;
-      const int j = __ffsll(static_cast<long long>(bits)) - 1;
-      bits &= bits - 1;
-      return src + static_cast<int64_t>(list[e]) * kPse64Tile + j;
-    };
-    const Rec* at = next();
-    Rec r = *(at ? at : src);
-    while (at) {
-      const Rec now = r;
-      at = next();
-      r = *(at ? at : src);  // on its way while this pair is evaluated
-      if (odd || now.odd) {
-        acc = pse64_plain<Op>(p, a.src, i, now.idx, acc);
-        continue;
-      }
-      const double dx = tp.x - now.x, dy = tp.y - now.y, dz = Op::kDim == 3 ? tp.z - now.z : 0.0;
-      const double d2 = Op::kDim == 3 ? fma(dx, dx, fma(dy, dy, dz * dz)) : fma(dx, dx, dy * dy);
-      const double w = pse64_kernel_value<Op::kPoly>(a, angle2<ANG>(d2) * a.c, powers);
-      Op::add(t, now, dx, dy, dz, w, acc);
-    }
     cnt = 0;
     __syncwarp();
   }
+  evaluate();
   if (valid) Op::Plain::store(p, i, i - a.ib, acc);
 }
 
