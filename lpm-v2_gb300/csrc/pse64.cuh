@@ -14,8 +14,9 @@
 //    (remainder 4e-17).
 // That is about 32 FP64 instructions a pair for K8 of the great-circle distance, where the
 // reference's expressions take about 150.  The results agree with the reference's to its own rounding
-// (1e-15 of the largest; its exp and atan2 are not CUDA's either), the sum is in the reference's
-// ascending order, one accumulator per target.
+// (1e-15 of the largest; its exp and atan2 are not CUDA's either).  A lane's sum is in the reference's
+// ascending order; small target sets have up to 8 lanes per target, each summing its part of every
+// tile, and add the parts at the end.
 //
 // At r >= 7 each kernel (its polynomial times e^-49) is below 1e-14 of its peak, and the sum
 // leaves those pairs out:
@@ -32,7 +33,11 @@
 // takes the reference's expressions as they stand (Op::Plain), as do all pairs of a reach beyond
 // the polynomials' range.
 //
-// Bound by the FP64 pipe (2 lanes per clock per SM).
+// Bound by the FP64 pipe (2 lanes per clock per SM): 73-77 % busy at cubed nest 6, the rest being
+// the last warps of an SM.  Host calls on GB300, ms, before (the reference's expressions over whole
+// tiles) and after: cubed nest 4 K8 7.1 -> 0.38, gradient 7.5 -> 0.43, double dot 13.5 -> 0.48; nest 6
+// K8 37 -> 4.4, Gaussian 12.7 -> 1.8, gradient 40 -> 5.3, divergence 49 -> 6.3, double dot 67 -> 6.8,
+// interpolation 37 -> 4.6; quad nest 6 K8 7.3 -> 1.2, gradient 8.4 -> 1.3, second partials 11.5 -> 1.5.
 #pragma once
 
 #include "engine.cuh"
@@ -45,6 +50,9 @@ constexpr int kPse64Stages = 2;
 constexpr int kPse64List = 64;  // tiles listed before they are tested
 constexpr int kPse64Mine = 48;  // tiles with sources of its own that a lane holds before they are evaluated
 constexpr double kPse64Reach = 7.0;
+// A set of up to this many sources (a few tiles) leaves nothing out: particles may then be so far
+// apart, against eps, that what lies beyond r = 7 is all there is.
+constexpr int64_t kPse64AllPairs = 4 * kPse64Tile;
 
 // How q comes from the squared distance in the test space.
 enum { kAngNone = 0, kAngNear = 1, kAngFar = 2, kAngWide = 3 };
@@ -149,8 +157,8 @@ __device__ __forceinline__ double pse64_kernel_value(const Pse64Args& a, double 
   const double e = powers[i & 255] * p;
   const double scaled = __hiloint2double(__double2hiint(e) - ((i >> 8) << 20), __double2loint(e));
   const double w = POLY ? scaled * fma(fma(fma(a.k3, s, a.k2), s, a.k1), s, a.k0) : scaled * a.k0;
-  // s >= 2^18 (q >= 709; only where the FP32 test underflowed) has left the exponent's range
-  return __double2hiint(s) >= 0x41100000 ? 0.0 : w;
+  // s >= 1020 x 256 (q >= 707, where the kernel is below 1e-300) leaves the exponent's range
+  return __double2hiint(s) >= 0x410fe000 ? 0.0 : w;
 }
 
 // ------------------------------------------------------------------ operators
@@ -435,7 +443,8 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-template <class Op, int ANG>
+// S lanes per target.
+template <class Op, int ANG, int S>
 __global__ void __launch_bounds__(32) pse64_sweep_kernel(typename Op::Params p, Pse64Args a,
                                                          const typename Op::Rec* __restrict__ src) {
   using Rec = typename Op::Rec;
@@ -446,8 +455,10 @@ __global__ void __launch_bounds__(32) pse64_sweep_kernel(typename Op::Params p, 
   __shared__ double powers[256];
   __shared__ int32_t list[kPse64List];
   const int lane = threadIdx.x;
-  const int64_t k = static_cast<int64_t>(blockIdx.x) * 32 + lane;
+  const int64_t k = static_cast<int64_t>(blockIdx.x) * (32 / S) + lane / S;
   const bool valid = k < a.nt;
+  // this lane's sources of a tile: the (lane modulo S)-th of S consecutive parts
+  const uint64_t part = (~0ull >> (64 - 64 / S)) << (lane % S * (64 / S));
   const int64_t kk = valid ? k : a.nt - 1;
   const int64_t i = a.tperm ? static_cast<int64_t>(a.tperm[kk]) : a.ib + kk;
   const typename Op::Tgt t = Op::load(p, i);
@@ -554,8 +565,9 @@ __global__ void __launch_bounds__(32) pse64_sweep_kernel(typename Op::Params p, 
             half[h] = n >= 32 ? bits : (n > 0 ? bits & ((1u << n) - 1u) : 0u);
           }
           ++q;
-          if ((half[0] | half[1]) != 0) {
-            mine[held][lane] = (static_cast<uint64_t>(half[1]) << 32) | half[0];
+          const uint64_t bits = ((static_cast<uint64_t>(half[1]) << 32) | half[0]) & part;
+          if (bits != 0) {
+            mine[held][lane] = bits;
             tile_of[held][lane] = static_cast<int32_t>(tile);
             ++held;
           }
@@ -566,7 +578,15 @@ __global__ void __launch_bounds__(32) pse64_sweep_kernel(typename Op::Params p, 
     __syncwarp();
   }
   evaluate();
-  if (valid) Op::Plain::store(p, i, i - a.ib, acc);
+  if constexpr (S > 1) {  // the parts' sums
+    constexpr int NA = static_cast<int>(sizeof(Acc) / sizeof(double));
+    double* av = reinterpret_cast<double*>(&acc);
+#pragma unroll
+    for (int c = 0; c < NA; ++c)
+#pragma unroll
+      for (int o = 1; o < S; o <<= 1) av[c] += __shfl_xor_sync(0xffffffffu, av[c], o);
+  }
+  if (valid && lane % S == 0) Op::Plain::store(p, i, i - a.ib, acc);
 }
 
 }  // namespace lpm

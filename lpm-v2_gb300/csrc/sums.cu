@@ -765,6 +765,23 @@ constexpr double kK1[4] = {-20.0, 20.0, -5.0, 1.0 / 3.0};       // bivariateFirs
 constexpr double kDelta8[4] = {4.0, -6.0, 2.0, -1.0 / 6.0};     // bivariateDeltaKernel8
 constexpr double kGauss[4] = {4.0, 0.0, 0.0, 0.0};
 
+template <class Op, int S>
+void launch_pse64_sweep(const SumJob& job, int ang, const typename Op::Params& p, const Pse64Args& a,
+                        const typename Op::Rec* recs) {
+  const unsigned grid = static_cast<unsigned>(ceil_div(job.nt, 32 / S));
+  if constexpr (Op::kUnit) {
+    if (ang == kAngNear) {
+      pse64_sweep_kernel<Op, kAngNear, S><<<grid, 32, 0, job.stream>>>(p, a, recs);
+    } else if (ang == kAngFar) {
+      pse64_sweep_kernel<Op, kAngFar, S><<<grid, 32, 0, job.stream>>>(p, a, recs);
+    } else {
+      pse64_sweep_kernel<Op, kAngWide, S><<<grid, 32, 0, job.stream>>>(p, a, recs);
+    }
+  } else {
+    pse64_sweep_kernel<Op, kAngNone, S><<<grid, 32, 0, job.stream>>>(p, a, recs);
+  }
+}
+
 // An FP64 PSE sum (pse64.cuh): the targets' curve order, prep and sweep.  `over` divides the kernel
 // (the operator's powers of eps).
 template <class Op>
@@ -795,6 +812,11 @@ int launch_pse64(const SumJob& job, const SumPlan& plan, const typename Op::Para
   a.reach = kPse64Reach * job.eps / (unit ? job.radius : 1.0);
   a.unit = unit;
   a.all_plain = unit && a.reach > kAngWideMax;
+  int ang = !unit ? kAngNone : a.reach <= kAngNearMax ? kAngNear : a.reach <= kAngFarMax ? kAngFar : kAngWide;
+  if (job.ns <= kPse64AllPairs) {
+    a.reach = 1e300;
+    if (unit) ang = kAngWide;
+  }
   a.x = job.x;
   a.y = job.y;
   a.z = job.z;
@@ -816,17 +838,20 @@ int launch_pse64(const SumJob& job, const SumPlan& plan, const typename Op::Para
   }, &a.tperm));
   pse64_prep_kernel<Op><<<static_cast<unsigned>(plan.n_tiles), kPse64Tile, 0, job.stream>>>(
       a.src, job.src_idx, job.ns, unit, recs, side, bounds, powers);
-  const unsigned grid = static_cast<unsigned>(ceil_div(job.nt, 32));
-  if constexpr (Op::kUnit) {
-    if (a.reach <= kAngNearMax) {
-      pse64_sweep_kernel<Op, kAngNear><<<grid, 32, 0, job.stream>>>(p, a, recs);
-    } else if (a.reach <= kAngFarMax) {
-      pse64_sweep_kernel<Op, kAngFar><<<grid, 32, 0, job.stream>>>(p, a, recs);
-    } else {
-      pse64_sweep_kernel<Op, kAngWide><<<grid, 32, 0, job.stream>>>(p, a, recs);
-    }
+  // Lanes per target: the fewest that put three warps on every scheduler, at most 8.  Measured at 1,
+  // 2, 4 and 8 lanes (K8, host call, ms): cubed nest 3 1.17, 0.63, 0.36, 0.25; nest 5 1.55, 1.24,
+  // 1.43, 1.26; nest 6 5.21, 4.44, 4.46, 4.60; nest 7 21.7, 21.6, 22.4, 23.7; quad nest 4 0.43, 0.36,
+  // 0.29, 0.27; nest 6 1.07, 1.20, 1.19, 1.25.  One warp can use a quarter of an SM's FP64 pipe.
+  int lanes = 1;
+  while (lanes < 8 && job.nt * lanes < 3 * plan.sm_count * 4 * 32) lanes *= 2;
+  if (lanes == 1) {
+    launch_pse64_sweep<Op, 1>(job, ang, p, a, recs);
+  } else if (lanes == 2) {
+    launch_pse64_sweep<Op, 2>(job, ang, p, a, recs);
+  } else if (lanes == 4) {
+    launch_pse64_sweep<Op, 4>(job, ang, p, a, recs);
   } else {
-    pse64_sweep_kernel<Op, kAngNone><<<grid, 32, 0, job.stream>>>(p, a, recs);
+    launch_pse64_sweep<Op, 8>(job, ang, p, a, recs);
   }
   LPM_CUDA_TRY(cudaGetLastError());
   return LPM_OK;
