@@ -79,7 +79,7 @@ struct EnsArgs {
   int n_items;
   int* head;
   const BveRel::Rec* src;
-  const BveRel::Origin* org;
+  const BveRel::Group* org;
   const double *x, *y, *z;
   const double* inv_a;  // per instance
   double* partial;      // [slot][3][targets per item]
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(THREADS, MINB) ensemble_sweep_kernel(EnsArgs a
     const BveF32::Params prm{a.x, a.y, a.z, a.inv_a[it.inst]};
     BveX2::Pair pr[NP];
     float2 hx[NP], hy[NP], hz[NP], lx[NP], ly[NP], lz[NP];
-    bve_load_pairs<NP>(prm, it.t0, it.nt, THREADS, pr);
+    bve_load_pairs<NP>(prm, it.t0, it.nt, pr);
 #pragma unroll
     for (int p = 0; p < NP; ++p) hx[p] = hy[p] = hz[p] = lx[p] = ly[p] = lz[p] = make_float2(0.f, 0.f);
     int64_t tile = it.tile0;
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(THREADS, MINB) ensemble_sweep_kernel(EnsArgs a
     for (int p = 0; p < NP; ++p) {
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const int l = (2 * p + h) * THREADS + threadIdx.x;
+        const int l = bve_target<TPT>(2 * p + h);
         if (l < it.nt) {
           slot[0 * TB + l] = static_cast<double>(h ? hx[p].y : hx[p].x) + static_cast<double>(h ? lx[p].y : lx[p].x);
           slot[1 * TB + l] = static_cast<double>(h ? hy[p].y : hy[p].x) + static_cast<double>(h ? ly[p].y : ly[p].x);
@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(kTile) ensemble_prep_kernel(const int32_t* til
                                                               const int32_t* sorted, const double* x, const double* y,
                                                               const double* z, const double* zeta, const double* area,
                                                               const double* radius, BveRel::Rec* out,
-                                                              BveRel::Origin* org) {
+                                                              BveRel::Group* org) {
   const int64_t t = blockIdx.x;
   const int k = tile_inst[t];
   const int64_t local = (t - tile_off[k]) * kTile + threadIdx.x;
@@ -274,7 +274,7 @@ struct lpm_ensemble {
   int32_t* tile_inst = nullptr;
   int64_t *d_tile_off = nullptr, *d_src_start = nullptr, *d_ns_k = nullptr;
   BveRel::Rec* rec = nullptr;
-  BveRel::Origin* org = nullptr;
+  BveRel::Group* org = nullptr;
   Item* items = nullptr;
   int* queue = nullptr;
   int n_items = 0;

@@ -25,6 +25,17 @@
 
 namespace lpm {
 
+// rel1 and rel2 (bve_rel.cuh) from an origin with a low part (planar sets lie anywhere).
+__device__ __forceinline__ float2 rel1x2(float2 ph, float2 pl, float oh, float ol) {
+  return __fadd2_rn(__fadd2_rn(ph, make_float2(-oh, -oh)), __fadd2_rn(pl, make_float2(-ol, -ol)));
+}
+__device__ __forceinline__ void rel2(float ph, float pl, float oh, float ol, float& rh, float& rl) {
+  rel2(ph, __fadd_rn(pl, -ol), oh, rh, rl);
+}
+__device__ __forceinline__ void rel2x2(float2 ph, float2 pl, float oh, float ol, float2& rh, float2& rl) {
+  rel2x2(ph, __fadd2_rn(pl, make_float2(-ol, -ol)), oh, rh, rl);
+}
+
 struct PlaneRel {
   struct __align__(16) Rec {
     float4 a;  // -sx_hi, -sx_hi, -sy_hi, -sy_hi

@@ -244,9 +244,9 @@ __global__ void __launch_bounds__(THREADS, MINB) pse_rel_sweep_kernel(PseRelArgs
       bool in_reach = false;
 #pragma unroll
       for (int p = 0; p < NP; ++p) {
-        tx[p] = rel1x2(pr[p].xh, pr[p].xl, o.hi.x, o.lo.x);
-        ty[p] = rel1x2(pr[p].yh, pr[p].yl, o.hi.y, o.lo.y);
-        tz[p] = rel1x2(pr[p].zh, pr[p].zl, o.hi.z, o.lo.z);
+        tx[p] = rel1x2(pr[p].xh, pr[p].xl, o.hi.x);
+        ty[p] = rel1x2(pr[p].yh, pr[p].yl, o.hi.y);
+        tz[p] = rel1x2(pr[p].zh, pr[p].zl, o.hi.z);
         const float2 n2 = __ffma2_rn(tz[p], tz[p], __ffma2_rn(ty[p], ty[p], __fmul2_rn(tx[p], tx[p])));
         in_reach |= (n2.x < reach * reach) | (n2.y < reach * reach);
       }
@@ -269,9 +269,9 @@ __global__ void __launch_bounds__(THREADS, MINB) pse_rel_sweep_kernel(PseRelArgs
         float2 txh[NP], tyh[NP], tzh[NP], txl[NP], tyl[NP], tzl[NP];
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
-          rel2x2(pr[p].xh, pr[p].xl, o.hi.x, o.lo.x, txh[p], txl[p]);
-          rel2x2(pr[p].yh, pr[p].yl, o.hi.y, o.lo.y, tyh[p], tyl[p]);
-          rel2x2(pr[p].zh, pr[p].zl, o.hi.z, o.lo.z, tzh[p], tzl[p]);
+          rel2x2(pr[p].xh, pr[p].xl, o.hi.x, txh[p], txl[p]);
+          rel2x2(pr[p].yh, pr[p].yl, o.hi.y, tyh[p], tyl[p]);
+          rel2x2(pr[p].zh, pr[p].zl, o.hi.z, tzh[p], tzl[p]);
         }
         for (int j = 0; j < G; ++j) {
           const float4 ra = gr[j].a, rb = gr[j].b, rc = gr[j].c, rd = gr[j].d, re = gr[j].e;
@@ -333,11 +333,12 @@ __global__ void __launch_bounds__(TILE) pse_rel_prep_kernel(const double* x, con
   const int32_t j = valid ? sorted[k] : 0;
   double px = 0.0, py = 0.0, pz = 0.0;
   if (valid) pse_position<ANG>(x, y, z, j, inv_a, px, py, pz);
-  const GroupFrame fr = sphere_group_frame<TILE, PseRel::kGroup>(valid, px, py, pz, 0.0);
+  const SplitPoint sp = split_point(px, py, pz);
+  const GroupFrame fr = sphere_group_frame<TILE, PseRel::kGroup>(valid, sp, 0.0);
   PseRel::Rec r;
   if (valid) {
     float hi[3], lo[3];
-    group_offsets(fr, px, py, pz, hi, lo);
+    group_offsets(fr, sp, hi, lo);
     const float ar = __double2float_rn(area[j]);
     r.a = make_float4(-hi[0], -hi[0], -hi[1], -hi[1]);
     r.b = make_float4(-hi[2], -hi[2], ar, ar);

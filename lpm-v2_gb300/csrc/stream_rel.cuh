@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(THREADS, MINB) stream_rel_sweep_kernel(SweepAr
   float2 hr[NP], lr[NP], ha[NP], la[NP], ar[NP], aa[NP];
   const int64_t first = static_cast<int64_t>(blockIdx.x) * (THREADS * TPT);
   const int64_t count = a.nt - first < THREADS * TPT ? a.nt - first : THREADS * TPT;
-  bve_load_pairs<NP>(a.p, a.ib + first, count, THREADS, pr);
+  bve_load_pairs<NP>(a.p, a.ib + first, count, pr);
 #pragma unroll
   for (int p = 0; p < NP; ++p) hr[p] = lr[p] = ha[p] = la[p] = ar[p] = aa[p] = make_float2(0.f, 0.f);
 
@@ -146,9 +146,9 @@ __global__ void __launch_bounds__(THREADS, MINB) stream_rel_sweep_kernel(SweepAr
       float2 tx[NP], ty[NP], tz[NP];
 #pragma unroll
       for (int p = 0; p < NP; ++p) {
-        tx[p] = rel1x2(pr[p].xh, pr[p].xl, o.hi.x, o.lo.x);
-        ty[p] = rel1x2(pr[p].yh, pr[p].yl, o.hi.y, o.lo.y);
-        tz[p] = rel1x2(pr[p].zh, pr[p].zl, o.hi.z, o.lo.z);
+        tx[p] = rel1x2(pr[p].xh, pr[p].xl, o.hi.x);
+        ty[p] = rel1x2(pr[p].yh, pr[p].yl, o.hi.y);
+        tz[p] = rel1x2(pr[p].zh, pr[p].zl, o.hi.z);
       }
       // far: every target of the warp beyond 3R (and off the centroid of a zero-radius group)
       const float rg = fabsf(o.hi.w);
@@ -212,9 +212,9 @@ __global__ void __launch_bounds__(THREADS, MINB) stream_rel_sweep_kernel(SweepAr
         float2 txh[NP], tyh[NP], tzh[NP], txl[NP], tyl[NP], tzl[NP];
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
-          rel2x2(pr[p].xh, pr[p].xl, o.hi.x, o.lo.x, txh[p], txl[p]);
-          rel2x2(pr[p].yh, pr[p].yl, o.hi.y, o.lo.y, tyh[p], tyl[p]);
-          rel2x2(pr[p].zh, pr[p].zl, o.hi.z, o.lo.z, tzh[p], tzl[p]);
+          rel2x2(pr[p].xh, pr[p].xl, o.hi.x, txh[p], txl[p]);
+          rel2x2(pr[p].yh, pr[p].yl, o.hi.y, tyh[p], tyl[p]);
+          rel2x2(pr[p].zh, pr[p].zl, o.hi.z, tzh[p], tzl[p]);
         }
 #pragma unroll 1
         for (int j0 = 0; j0 < G; j0 += FL) {
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(THREADS, MINB) stream_rel_sweep_kernel(SweepAr
   for (int p = 0; p < NP; ++p) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const int64_t il = first + (2 * p + h) * THREADS + threadIdx.x;
+      const int64_t il = first + bve_target<TPT>(2 * p + h);
       if (il < a.nt) {
         a.partial[(chunk * 2 + 0) * a.nt + il] =
             static_cast<double>(h ? hr[p].y : hr[p].x) + static_cast<double>(h ? lr[p].y : lr[p].x);
@@ -276,11 +276,12 @@ __global__ void __launch_bounds__(TILE) stream_rel_prep_kernel(const double* x, 
     pz = z[j] * inv_a;
     cj = fma(px, px, fma(py, py, fma(pz, pz, -1.0)));
   }
-  const GroupFrame f = sphere_group_frame<TILE, BveRel::kGroup>(valid, px, py, pz, cj);
+  const SplitPoint sp = split_point(px, py, pz);
+  const GroupFrame f = sphere_group_frame<TILE, BveRel::kGroup>(valid, sp, cj);
   StreamRel::Rec r;
   if (valid) {
     float hi[3], lo[3];
-    group_offsets(f, px, py, pz, hi, lo);
+    group_offsets(f, sp, hi, lo);
     const float nc = __double2float_rn(-cj);
     const double wr = qr[j] * area[j], wa = qa[j] * area[j];
     const float sr = __double2float_rn(wr * scale_r), sa = __double2float_rn(wa * scale_a);
@@ -507,7 +508,7 @@ __global__ void __launch_bounds__(THREADS, MINB) sphere_swe_rel_sweep_kernel(Swe
   float2 hs[NP][NC], ls[NP][NC];
   const int64_t first = static_cast<int64_t>(blockIdx.x) * (THREADS * TPT);
   const int64_t count = a.nt - first < THREADS * TPT ? a.nt - first : THREADS * TPT;
-  bve_load_pairs<NP>(a.p, a.ib + first, count, THREADS, pr);
+  bve_load_pairs<NP>(a.p, a.ib + first, count, pr);
 #pragma unroll
   for (int p = 0; p < NP; ++p)
 #pragma unroll
@@ -541,9 +542,9 @@ __global__ void __launch_bounds__(THREADS, MINB) sphere_swe_rel_sweep_kernel(Swe
       float2 tx[NP], ty[NP], tz[NP];
 #pragma unroll
       for (int p = 0; p < NP; ++p) {
-        tx[p] = rel1x2(pr[p].xh, pr[p].xl, o.hi.x, o.lo.x);
-        ty[p] = rel1x2(pr[p].yh, pr[p].yl, o.hi.y, o.lo.y);
-        tz[p] = rel1x2(pr[p].zh, pr[p].zl, o.hi.z, o.lo.z);
+        tx[p] = rel1x2(pr[p].xh, pr[p].xl, o.hi.x);
+        ty[p] = rel1x2(pr[p].yh, pr[p].yl, o.hi.y);
+        tz[p] = rel1x2(pr[p].zh, pr[p].zl, o.hi.z);
       }
       if (o.hi.w <= 0.f || !warp_near<NP>(tx, ty, tz, o.hi.w)) {  // -R: compact, taken as far
         // compact or far group: d = t_hi - s_hi
@@ -565,9 +566,9 @@ __global__ void __launch_bounds__(THREADS, MINB) sphere_swe_rel_sweep_kernel(Swe
         float2 txh[NP], tyh[NP], tzh[NP], txl[NP], tyl[NP], tzl[NP];
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
-          rel2x2(pr[p].xh, pr[p].xl, o.hi.x, o.lo.x, txh[p], txl[p]);
-          rel2x2(pr[p].yh, pr[p].yl, o.hi.y, o.lo.y, tyh[p], tyl[p]);
-          rel2x2(pr[p].zh, pr[p].zl, o.hi.z, o.lo.z, tzh[p], tzl[p]);
+          rel2x2(pr[p].xh, pr[p].xl, o.hi.x, txh[p], txl[p]);
+          rel2x2(pr[p].yh, pr[p].yl, o.hi.y, tyh[p], tyl[p]);
+          rel2x2(pr[p].zh, pr[p].zl, o.hi.z, tzh[p], tzl[p]);
         }
         for (int j = 0; j < G; ++j) {
           const float4 ra = gr[j].a, rb = gr[j].b, rc = gr[j].c, rd = gr[j].d, re = gr[j].e;
@@ -598,7 +599,7 @@ __global__ void __launch_bounds__(THREADS, MINB) sphere_swe_rel_sweep_kernel(Swe
   for (int p = 0; p < NP; ++p) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const int64_t il = first + (2 * p + h) * THREADS + threadIdx.x;
+      const int64_t il = first + bve_target<TPT>(2 * p + h);
       if (il < a.nt) {
 #pragma unroll
         for (int c = 0; c < NC; ++c)

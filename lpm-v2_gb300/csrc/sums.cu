@@ -523,7 +523,8 @@ SumPlan plan_sum(int kind, int mode, int64_t ns, int64_t nt, int sm_count, int s
                       sizeof(BveRel::Origin) == sizeof(BetaStreamRel::Origin),
                   "one origin layout size");
     pl.src_bytes = align_up(pl.src_bytes, 256) +
-                   static_cast<size_t>(pl.n_tiles) * (tile / origin_group(kind)) * sizeof(BveRel::Origin);
+                   static_cast<size_t>(pl.n_tiles) * (tile / origin_group(kind)) *
+                       (kind == kSumBve || kind == kSumBveMesh ? sizeof(BveRel::Group) : sizeof(BveRel::Origin));
   }
   if (mode == LPM_MODE_FP32C && pse_culls_tiles(kind)) {
     // the tiles' balls follow the group origins
@@ -1009,7 +1010,7 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
         src_list = job.sorted;
       }
       BveRel::Rec* recs = static_cast<BveRel::Rec*>(job.src_buf);
-      BveRel::Origin* org = reinterpret_cast<BveRel::Origin*>(
+      BveRel::Group* org = reinterpret_cast<BveRel::Group*>(
           static_cast<char*>(job.src_buf) + align_up(static_cast<size_t>(npad) * sizeof(BveRel::Rec), 256));
       bve_rel_prep_kernel<kBveTile><<<static_cast<unsigned>(plan.n_tiles), kBveTile, 0, job.stream>>>(
           job.x, job.y, job.z, job.s1, job.area, src_list, job.ns, inv_a, -1.0 / (2.0 * kPi * job.radius), recs,
