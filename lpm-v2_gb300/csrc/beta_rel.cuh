@@ -66,10 +66,7 @@ __global__ void __launch_bounds__(THREADS, MINB) beta_rel_sweep_kernel(BetaRelAr
   __shared__ __align__(8) uint64_t bars[2];
 
   const int64_t chunk = blockIdx.y;
-  const int64_t tile0 = chunk * a.tiles_per_chunk;
-  int64_t ntl = a.n_tiles - tile0;
-  if (ntl > a.tiles_per_chunk) ntl = a.tiles_per_chunk;
-  if (ntl < 0) ntl = 0;
+  const ChunkTiles ct = chunk_tiles(a.n_tiles);
 
   BetaTgt tg[2 * NP];
   float hu[2 * NP], lu[2 * NP], hv[2 * NP], lv[2 * NP];
@@ -86,8 +83,8 @@ __global__ void __launch_bounds__(THREADS, MINB) beta_rel_sweep_kernel(BetaRelAr
 
   pipe_init(bars);
   uint32_t g = 0;
-  int64_t tile = tile0;
-  staged_sweep<Rec, TILE>(a.src, tile0, ntl, stage[0], stage[1], bars, g, a.status, [&](const Rec* tl) {
+  int64_t tile = ct.first;
+  staged_sweep<Rec, TILE>(a.src, ct.first, ct.count, stage[0], stage[1], bars, g, a.status, [&](const Rec* tl) {
     float au[2 * NP], av[2 * NP];
 #pragma unroll
     for (int t = 0; t < 2 * NP; ++t) au[t] = av[t] = 0.f;
@@ -170,13 +167,13 @@ __global__ void __launch_bounds__(THREADS, MINB) beta_rel_sweep_kernel(BetaRelAr
         }
       }
     }
-    ++tile;
+    tile += ct.step;
 #pragma unroll
     for (int t = 0; t < 2 * NP; ++t) {
       comp_add(hu[t], lu[t], au[t]);
       comp_add(hv[t], lv[t], av[t]);
     }
-  });
+  }, ct.step);
 
 #pragma unroll
   for (int p = 0; p < NP; ++p) {
@@ -356,10 +353,7 @@ __global__ void __launch_bounds__(THREADS, MINB) beta_stream_rel_sweep_kernel(Be
   __shared__ __align__(8) float2 ln_tab[32];
 
   const int64_t chunk = blockIdx.y;
-  const int64_t tile0 = chunk * a.tiles_per_chunk;
-  int64_t ntl = a.n_tiles - tile0;
-  if (ntl > a.tiles_per_chunk) ntl = a.tiles_per_chunk;
-  if (ntl < 0) ntl = 0;
+  const ChunkTiles ct = chunk_tiles(a.n_tiles);
 
   BetaTgt tg[2 * NP];
   float hr[2 * NP], lr[2 * NP], ha[2 * NP], la[2 * NP];
@@ -377,8 +371,8 @@ __global__ void __launch_bounds__(THREADS, MINB) beta_stream_rel_sweep_kernel(Be
   ln_tab_load(ln_tab);
   pipe_init(bars);
   uint32_t g = 0;
-  int64_t tile = tile0;
-  staged_sweep<Rec, TILE>(a.src, tile0, ntl, stage[0], stage[1], bars, g, a.status, [&](const Rec* tl) {
+  int64_t tile = ct.first;
+  staged_sweep<Rec, TILE>(a.src, ct.first, ct.count, stage[0], stage[1], bars, g, a.status, [&](const Rec* tl) {
     const BetaStreamRel::Origin* og = a.org + tile * GPT;
 #pragma unroll 1
     for (int g0 = 0; g0 < TILE; g0 += G) {
@@ -496,8 +490,8 @@ __global__ void __launch_bounds__(THREADS, MINB) beta_stream_rel_sweep_kernel(Be
         }
       }
     }
-    ++tile;
-  });
+    tile += ct.step;
+  }, ct.step);
 
 #pragma unroll
   for (int p = 0; p < NP; ++p) {

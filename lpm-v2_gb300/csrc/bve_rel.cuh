@@ -29,7 +29,7 @@
 // fma(dz,dz, fma(dy,dy, fma(dx,dx, -c_i))), one operation less per pair.
 // Then  q = |d|^2 - c_i - c_j,  w = S_j / q,  D += w d  with c = |p|^2 - 1 and
 // S_j = -zeta_j A_j / (2 pi a) as in BveF32; u = D x p_i in FP64.
-// A group whose warp is far (every target at |t - o| >= 3R, compact or not) takes the
+// A group whose warp is far (every target at |t - o| >= 3R, 1.5R if it is compact) takes the
 // expanded form in a basis (o, e1, e2) of the group, e1 and e2 about orthonormal to o: with the
 // source p_j = (1 + c) o + a e1 + b e2 and h = q/2 = 1 - p_i.p_j,
 //   h = C - c gamma - a alpha - b beta,   alpha = p_i.e1, beta = p_i.e2, gamma = p_i.o, C = 1 - gamma,
@@ -40,8 +40,7 @@
 // B_j/2 - t.s_j and four sums) took 8, 2 and 4.  Any basis does: the records solve for (a, b, c) in
 // the rounded one, alpha = t.e1 + o.e1 carries the group constant o.e1 (about 2^-25), and gamma =
 // |o|^2 + k - ct, C = ct + k with ct = (|t|^2 - c_i)/2 and k = (1 - |o|^2)/2, so no term loses
-// digits: |h| >= 2R^2, C and the products are at most a few h at the 3R boundary, and q stays
-// within a few ulps.  A compact group with a target of the warp near it keeps d = t_hi - s_hi
+// digits: C and the products are at most a few h at the 3R boundary, and q stays within a few ulps.  A compact group with a target of the warp near it keeps d = t_hi - s_hi
 // (10-11 operations; it contains the self pairs), any other near group the two-float form (17).
 // Forming the targets' offsets, projections and the near test cost about 25 per pair and group.
 // Targets keep their original order (only sources are sorted), so no scatter is needed.
@@ -62,7 +61,7 @@ struct BveRel {
     float4 e;  // -sx_lo, -sy_lo, -sz_lo, -c_j  (near forms)
   };
   struct __align__(16) Origin {
-    float4 hi;  // o.x, o.y, o.z, R (the group radius about o; -R for a compact group)
+    float4 hi;  // o.x, o.y, o.z, R (the group radius about o; -R/2 for a compact group)
     float4 lo;  // 0, 0, 0, 1 if every c_j of the group is negligible
   };
   // The BVE sweep's group record: the origin and the far form's basis.
@@ -149,18 +148,25 @@ __device__ __forceinline__ void bve_load_pairs(const BveF32::Params& prm, int64_
 }
 
 // Whether any target of the warp lies within kNearFactor R of a group origin (t = t_hi,
-// the offsets from it).  Every lane of the warp must call it.
+// the offsets from it); n2 returns |t|^2.  Every lane of the warp must call it.
 template <int NP>
 __device__ __forceinline__ bool warp_near(const float2 (&tx)[NP], const float2 (&ty)[NP], const float2 (&tz)[NP],
-                                          float r) {
+                                          float r, float2 (&n2)[NP]) {
   const float lim = (BveRel::kNearFactor * r) * (BveRel::kNearFactor * r);
   bool near = false;
 #pragma unroll
   for (int p = 0; p < NP; ++p) {
-    const float2 n2 = __ffma2_rn(tz[p], tz[p], __ffma2_rn(ty[p], ty[p], __fmul2_rn(tx[p], tx[p])));
-    near |= (n2.x < lim) | (n2.y < lim);
+    n2[p] = __ffma2_rn(tz[p], tz[p], __ffma2_rn(ty[p], ty[p], __fmul2_rn(tx[p], tx[p])));
+    near |= (n2[p].x < lim) | (n2[p].y < lim);
   }
   return __any_sync(0xffffffffu, near);
+}
+
+template <int NP>
+__device__ __forceinline__ bool warp_near(const float2 (&tx)[NP], const float2 (&ty)[NP], const float2 (&tz)[NP],
+                                          float r) {
+  float2 n2[NP];
+  return warp_near<NP>(tx, ty, tz, r, n2);
 }
 
 // One staged tile against NP target pairs: FP32 partials of D added into (ax, ay, az).  The far
@@ -182,15 +188,16 @@ __device__ __forceinline__ void bve_rel_tile(const BveRel::Rec* __restrict__ tl,
       ty[p] = rel1x2(pr[p].yh, pr[p].yl, o.hi.y);
       tz[p] = rel1x2(pr[p].zh, pr[p].zl, o.hi.z);
     }
-    if (!warp_near<NP>(tx, ty, tz, fabsf(o.hi.w))) {
+    float2 n2[NP];
+    if (!warp_near<NP>(tx, ty, tz, fabsf(o.hi.w), n2)) {
       // far group: h = C - c gamma - a alpha - b beta, D += t W + e1 A + e2 B
       const float4 e1 = gp.e1, e2 = gp.e2;
       float2 al[NP], be[NP], ga[NP], cc[NP], ww[NP], va[NP], vb[NP];
 #pragma unroll
       for (int p = 0; p < NP; ++p) {
-        const float2 n2 = __ffma2_rn(tz[p], tz[p], __ffma2_rn(ty[p], ty[p], __ffma2_rn(tx[p], tx[p], pr[p].nc)));
-        cc[p] = __ffma2_rn(n2, make_float2(0.5f, 0.5f), make_float2(o.lo.x, o.lo.x));
-        ga[p] = __ffma2_rn(n2, make_float2(-0.5f, -0.5f), make_float2(o.lo.y, o.lo.y));
+        const float2 nq = __fadd2_rn(n2[p], pr[p].nc);  // |t|^2 - c_i
+        cc[p] = __ffma2_rn(nq, make_float2(0.5f, 0.5f), make_float2(o.lo.x, o.lo.x));
+        ga[p] = __ffma2_rn(nq, make_float2(-0.5f, -0.5f), make_float2(o.lo.y, o.lo.y));
         al[p] = __ffma2_rn(tx[p], make_float2(e1.x, e1.x), make_float2(e1.w, e1.w));
         al[p] = __ffma2_rn(ty[p], make_float2(e1.y, e1.y), al[p]);
         al[p] = __ffma2_rn(tz[p], make_float2(e1.z, e1.z), al[p]);
@@ -320,7 +327,7 @@ __device__ __forceinline__ void bve_merge_pairs(const float2 (&ax)[NP], const fl
   }
 }
 
-template <int THREADS, int TPT, int TILE, int MINB>
+template <int THREADS, int TPT, int TILE, int MINB, bool DECOUPLED>
 __global__ void __launch_bounds__(THREADS, MINB) bve_rel_sweep_kernel(SweepArgs<BveF32> a,
                                                                       const BveRel::Group* __restrict__ org) {
   static_assert(TPT % 2 == 0, "targets come in pairs");
@@ -328,14 +335,10 @@ __global__ void __launch_bounds__(THREADS, MINB) bve_rel_sweep_kernel(SweepArgs<
   constexpr int NP = TPT / 2;
   constexpr int GPT = TILE / BveRel::kGroup;
   using Rec = BveRel::Rec;
-  __shared__ __align__(128) Rec stage[2][TILE];
-  __shared__ __align__(8) uint64_t bars[2];
+  __shared__ TilePipe<Rec, TILE, 2> pipe;  // (its full barriers serve the block-synchronous pipeline too)
 
   const int64_t chunk = blockIdx.y;
-  const int64_t tile0 = chunk * a.tiles_per_chunk;
-  int64_t ntl = a.n_tiles - tile0;
-  if (ntl > a.tiles_per_chunk) ntl = a.tiles_per_chunk;
-  if (ntl < 0) ntl = 0;
+  const ChunkTiles ct = chunk_tiles(a.n_tiles);
 
   BveX2::Pair pr[NP];
   float2 hx[NP], hy[NP], hz[NP], lx[NP], ly[NP], lz[NP];
@@ -345,18 +348,26 @@ __global__ void __launch_bounds__(THREADS, MINB) bve_rel_sweep_kernel(SweepArgs<
 #pragma unroll
   for (int p = 0; p < NP; ++p) hx[p] = hy[p] = hz[p] = lx[p] = ly[p] = lz[p] = make_float2(0.f, 0.f);
 
-  pipe_init(bars);
   uint32_t g = 0;
-  int64_t tile = tile0;
+  int64_t tile = ct.first;
   const Rec* src = reinterpret_cast<const Rec*>(a.src);
-  staged_sweep<Rec, TILE>(src, tile0, ntl, stage[0], stage[1], bars, g, a.status, a.wait, [&](const Rec* tl) {
+  auto body = [&](const Rec* tl) {
     float2 ax[NP], ay[NP], az[NP];
 #pragma unroll
     for (int p = 0; p < NP; ++p) ax[p] = ay[p] = az[p] = make_float2(0.f, 0.f);
     bve_rel_tile<NP, TILE, (NP >= 3 ? 4 : 2)>(tl, org + tile * GPT, pr, ax, ay, az);
-    ++tile;
+    tile += ct.step;
     bve_merge_pairs<NP>(ax, ay, az, hx, hy, hz, lx, ly, lz);
-  });
+  };
+  if constexpr (DECOUPLED) {
+    tile_pipe_init(pipe);
+    warp_sweep_tiles(src, [ct](int64_t k) { return ct.first + k * ct.step; }, ct.count, pipe, g, a.status, a.wait,
+                     static_cast<const Rec*>(nullptr), body);
+  } else {
+    pipe_init(pipe.full);
+    staged_sweep<Rec, TILE>(src, ct.first, ct.count, pipe.stage[0], pipe.stage[1], pipe.full, g, a.status, a.wait, body,
+                            ct.step);
+  }
 
 #pragma unroll
   for (int p = 0; p < NP; ++p) {
@@ -619,7 +630,13 @@ __device__ __forceinline__ void bve_rel_prep_tile(const double* x, const double*
   if (threadIdx.x % BveRel::kGroup == 0) {
     BveRel::Group g;
     g.o = group_origin(f);
-    g.o.hi.w = f.compact ? -f.radius : f.radius;  // the sign marks a compact group
+    // The sign marks a compact group, whose far form starts at 1.5 R: there |h| >= R^2 / 8 and the
+    // expanded form's roundings are at most about 20 x 2^-24 of it, at the nearest of the group's
+    // sources alone, while the difference form near a compact group carries an absolute 2^-24 R
+    // in d for all of them.  Measured at icosahedral nests 5, 6, 7 against FP64 (relative L2 of the
+    // velocity): 1.86e-7, 8.60e-8, 4.95e-8 from 3 R on, 1.73e-7, 7.95e-8, 4.65e-8 from 1.5 R on, and
+    // 3, 3 and 1 % faster.
+    g.o.hi.w = f.compact ? -0.5f * f.radius : f.radius;
     if (b.singular) g.o.hi.w = 1e15f;             // near every target
     g.o.lo.x = b.k;
     g.o.lo.y = 1.f - b.k;  // |o|^2 + k

@@ -2,15 +2,14 @@
 //
 // Layout: sources are compacted (active particles only) into an array of fixed-size
 // records, padded with inert records to a multiple of the tile size.  A CTA owns a block of
-// targets (held in registers) and a contiguous range of source tiles (one split-K chunk) --
+// targets (held in registers) and a share of the source tiles (one split-K chunk, chunk_tiles) --
 // or, for the sums with a distance cutoff, a round-robin share of the tiles within reach of
 // its targets (sweep_culled_share, at the end of this file).
 // Tiles are staged into shared memory by 1-D TMA bulk copies (cp.async.bulk), and every
 // thread then sweeps a tile with broadcast shared-memory reads.  Two pipelines:
 //  - staged_sweep: two stages, block-synchronous (every warp finishes a tile before its stage
 //    is refilled; two block barriers per tile);
-//  - warp_sweep / warp_sweep_tiles: S stages, warp-decoupled, over a contiguous range or a
-//    list of tiles.  Each stage has a "full" mbarrier (the copy's
+//  - warp_sweep_tiles: S stages, warp-decoupled, over a list of tiles.  Each stage has a "full" mbarrier (the copy's
 //    transaction count) and an "empty" one (one arrival per warp when it is done with the
 //    tile).  Thread 0 refills a stage as soon as every warp has released it, so warps that
 //    skip a tile's work run ahead by up to S - 1 tiles instead of waiting at a barrier.
@@ -38,20 +37,21 @@ __device__ __forceinline__ void pipe_init(uint64_t* bars) {
 // is called once per tile by every thread of the block.  `g` counts the tiles this CTA has
 // pushed through the pipeline so far (identical in every thread): tile g uses stage g & 1
 // and completes phase (g >> 1) & 1 of that stage's barrier, so one CTA can run many sweeps
-// (a persistent kernel) on barriers initialised once.  Returns false on a timeout.
+// (a persistent kernel) on barriers initialised once.  With `step` the tiles are tile0,
+// tile0 + step, ... (chunk_tiles below).  Returns false on a timeout.
 template <class Rec, int TILE, class Body>
 __device__ __forceinline__ bool staged_sweep(const Rec* __restrict__ src, int64_t tile0,
                                              int64_t ntl, Rec* stage0, Rec* stage1,
                                              uint64_t* bars, uint32_t& g, int* status, const WaitCfg& w,
-                                             Body&& body) {
+                                             Body&& body, int64_t step = 1) {
   constexpr uint32_t kBytes = TILE * sizeof(Rec);
   static_assert(kBytes % 16 == 0, "tile bytes must be a multiple of 16");
   if (threadIdx.x == 0) {
     for (int64_t k = 0; k < ntl && k < 2; ++k) {
       const uint32_t gk = g + static_cast<uint32_t>(k);
-      if (tile0 + k == w.skip_tile) continue;
+      if (tile0 + k * step == w.skip_tile) continue;
       mbar_arrive_expect_tx(&bars[gk & 1u], kBytes);
-      tma_load_1d((gk & 1u) ? stage1 : stage0, src + (tile0 + k) * TILE, kBytes, &bars[gk & 1u]);
+      tma_load_1d((gk & 1u) ? stage1 : stage0, src + (tile0 + k * step) * TILE, kBytes, &bars[gk & 1u]);
     }
   }
   bool ok = true;
@@ -67,15 +67,15 @@ __device__ __forceinline__ bool staged_sweep(const Rec* __restrict__ src, int64_
     }
     body(s ? stage1 : stage0);
     __syncthreads();  // every thread is done with stage s
-    if (threadIdx.x == 0 && k + 2 < ntl && tile0 + k + 2 != w.skip_tile) {
+    if (threadIdx.x == 0 && k + 2 < ntl && tile0 + (k + 2) * step != w.skip_tile) {
       mbar_arrive_expect_tx(&bars[s], kBytes);
-      tma_load_1d(s ? stage1 : stage0, src + (tile0 + k + 2) * TILE, kBytes, &bars[s]);
+      tma_load_1d(s ? stage1 : stage0, src + (tile0 + (k + 2) * step) * TILE, kBytes, &bars[s]);
     }
   }
   if (!ok && threadIdx.x == 0) {
     // let copies that are still in flight land before the CTA moves on (bounded again)
     for (int64_t kk = k; kk < ntl && kk < k + 2; ++kk) {
-      if (tile0 + kk == w.skip_tile) continue;  // never issued
+      if (tile0 + kk * step == w.skip_tile) continue;  // never issued
       const uint32_t gk = g + static_cast<uint32_t>(kk);
       mbar_wait_bounded(&bars[gk & 1u], (gk >> 1) & 1u, status, w.ns);
     }
@@ -87,9 +87,22 @@ __device__ __forceinline__ bool staged_sweep(const Rec* __restrict__ src, int64_
 template <class Rec, int TILE, class Body>
 __device__ __forceinline__ bool staged_sweep(const Rec* __restrict__ src, int64_t tile0,
                                              int64_t ntl, Rec* stage0, Rec* stage1,
-                                             uint64_t* bars, uint32_t& g, int* status, Body&& body) {
+                                             uint64_t* bars, uint32_t& g, int* status, Body&& body,
+                                             int64_t step = 1) {
   return staged_sweep<Rec, TILE>(src, tile0, ntl, stage0, stage1, bars, g, status, default_wait(),
-                                 static_cast<Body&&>(body));
+                                 static_cast<Body&&>(body), step);
+}
+
+// The source tiles of a split-K chunk (chunk blockIdx.y of gridDim.y): every gridDim.y-th tile from
+// the blockIdx.y-th on.  The tiles near a target block are consecutive in curve order and cost about
+// 1.4 x a far one, so consecutive chunks would give one CTA of each block all of them (icosahedral
+// nest 5, 9 chunks of 9 tiles: the sweep waited for CTAs whose groups were all near).
+struct ChunkTiles {
+  int64_t first, step, count;
+};
+__device__ __forceinline__ ChunkTiles chunk_tiles(int64_t n_tiles) {
+  const int64_t c = blockIdx.y, step = gridDim.y;
+  return ChunkTiles{c, step, n_tiles > c ? (n_tiles - c + step - 1) / step : 0};
 }
 
 // Shared memory of an S-stage warp-decoupled pipeline.  With NSIDE > 0 each stage also holds
@@ -192,15 +205,6 @@ __device__ __forceinline__ bool warp_sweep_tiles(const Rec* __restrict__ src, Ti
   }
   g += static_cast<uint32_t>(ntl);
   return all;
-}
-
-// The sweep over the contiguous tiles [tile0, tile0 + ntl).
-template <class Rec, int TILE, int S, class Side, int NSIDE, class Body>
-__device__ __forceinline__ bool warp_sweep(const Rec* __restrict__ src, int64_t tile0, int64_t ntl,
-                                           TilePipe<Rec, TILE, S, Side, NSIDE>& pp, uint32_t& g, int* status,
-                                           const WaitCfg& w, const Side* __restrict__ side_src, Body&& body) {
-  return warp_sweep_tiles(src, [tile0](int64_t k) { return tile0 + k; }, ntl, pp, g, status, w, side_src,
-                          static_cast<Body&&>(body));
 }
 
 // ---------------------------------------------------------------- tile culling (cutoff sums)

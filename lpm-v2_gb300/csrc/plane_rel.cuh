@@ -77,10 +77,7 @@ __global__ void __launch_bounds__(THREADS, MINB) plane_rel_sweep_kernel(PlaneRel
   __shared__ __align__(8) uint64_t bars[2];
 
   const int64_t chunk = blockIdx.y;
-  const int64_t tile0 = chunk * a.tiles_per_chunk;
-  int64_t ntl = a.n_tiles - tile0;
-  if (ntl > a.tiles_per_chunk) ntl = a.tiles_per_chunk;
-  if (ntl < 0) ntl = 0;
+  const ChunkTiles ct = chunk_tiles(a.n_tiles);
 
   PlaneRel::Pair pr[NP];
   float2 hu[NP], hv[NP], lu[NP], lv[NP];
@@ -106,8 +103,8 @@ __global__ void __launch_bounds__(THREADS, MINB) plane_rel_sweep_kernel(PlaneRel
 
   pipe_init(bars);
   uint32_t g = 0;
-  int64_t tile = tile0;
-  staged_sweep<Rec, TILE>(a.src, tile0, ntl, stage[0], stage[1], bars, g, a.status, [&](const Rec* tl) {
+  int64_t tile = ct.first;
+  staged_sweep<Rec, TILE>(a.src, ct.first, ct.count, stage[0], stage[1], bars, g, a.status, [&](const Rec* tl) {
     float2 au[NP], av[NP];
 #pragma unroll
     for (int p = 0; p < NP; ++p) au[p] = av[p] = make_float2(0.f, 0.f);
@@ -178,7 +175,7 @@ __global__ void __launch_bounds__(THREADS, MINB) plane_rel_sweep_kernel(PlaneRel
         av[p] = __fadd2_rn(av[p], gv[p]);
       }
     }
-    ++tile;
+    tile += ct.step;
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
       comp_add(hu[p].x, lu[p].x, au[p].x);
@@ -186,7 +183,7 @@ __global__ void __launch_bounds__(THREADS, MINB) plane_rel_sweep_kernel(PlaneRel
       comp_add(hv[p].x, lv[p].x, av[p].x);
       comp_add(hv[p].y, lv[p].y, av[p].y);
     }
-  });
+  }, ct.step);
 
 #pragma unroll
   for (int p = 0; p < NP; ++p) {
@@ -560,10 +557,7 @@ __global__ void __launch_bounds__(THREADS, MINB) plane_swe_rel_sweep_kernel(Plan
   __shared__ __align__(8) uint64_t bars[2];
 
   const int64_t chunk = blockIdx.y;
-  const int64_t tile0 = chunk * a.tiles_per_chunk;
-  int64_t ntl = a.n_tiles - tile0;
-  if (ntl > a.tiles_per_chunk) ntl = a.tiles_per_chunk;
-  if (ntl < 0) ntl = 0;
+  const ChunkTiles ct = chunk_tiles(a.n_tiles);
 
   PlaneRel::Pair pr[NP];
   float2 hs[NP][NC], ls[NP][NC];
@@ -590,8 +584,8 @@ __global__ void __launch_bounds__(THREADS, MINB) plane_swe_rel_sweep_kernel(Plan
 
   pipe_init(bars);
   uint32_t g = 0;
-  int64_t tile = tile0;
-  staged_sweep<Rec, TILE>(a.src, tile0, ntl, stage[0], stage[1], bars, g, a.status, [&](const Rec* tl) {
+  int64_t tile = ct.first;
+  staged_sweep<Rec, TILE>(a.src, ct.first, ct.count, stage[0], stage[1], bars, g, a.status, [&](const Rec* tl) {
     float2 acc[NP][NC];
 #pragma unroll
     for (int p = 0; p < NP; ++p)
@@ -662,7 +656,7 @@ __global__ void __launch_bounds__(THREADS, MINB) plane_swe_rel_sweep_kernel(Plan
         }
       }
     }
-    ++tile;
+    tile += ct.step;
 #pragma unroll
     for (int p = 0; p < NP; ++p)
 #pragma unroll
@@ -670,7 +664,7 @@ __global__ void __launch_bounds__(THREADS, MINB) plane_swe_rel_sweep_kernel(Plan
         comp_add(hs[p][c].x, ls[p][c].x, acc[p][c].x);
         comp_add(hs[p][c].y, ls[p][c].y, acc[p][c].y);
       }
-  });
+  }, ct.step);
 
 #pragma unroll
   for (int p = 0; p < NP; ++p) {

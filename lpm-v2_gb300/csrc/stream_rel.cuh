@@ -122,10 +122,7 @@ __global__ void __launch_bounds__(THREADS, MINB) stream_rel_sweep_kernel(SweepAr
   __shared__ __align__(8) float2 ln_tab[32];
 
   const int64_t chunk = blockIdx.y;
-  const int64_t tile0 = chunk * a.tiles_per_chunk;
-  int64_t ntl = a.n_tiles - tile0;
-  if (ntl > a.tiles_per_chunk) ntl = a.tiles_per_chunk;
-  if (ntl < 0) ntl = 0;
+  const ChunkTiles ct = chunk_tiles(a.n_tiles);
 
   BveX2::Pair pr[NP];
   float2 hr[NP], lr[NP], ha[NP], la[NP], ar[NP], aa[NP];
@@ -138,7 +135,7 @@ __global__ void __launch_bounds__(THREADS, MINB) stream_rel_sweep_kernel(SweepAr
   ln_tab_load(ln_tab);
   tile_pipe_init(pipe);
   uint32_t g = 0;
-  warp_sweep(src, tile0, ntl, pipe, g, a.status, default_wait(), org, [&](const Rec* tl, const BveRel::Origin* og) {
+  warp_sweep_tiles(src, [ct](int64_t k) { return ct.first + k * ct.step; }, ct.count, pipe, g, a.status, default_wait(), org, [&](const Rec* tl, const BveRel::Origin* og) {
 #pragma unroll 1
     for (int g0 = 0; g0 < TILE; g0 += G) {
       const BveRel::Origin o = og[g0 / G];
@@ -340,10 +337,7 @@ __global__ void __launch_bounds__(THREADS, MINB) plane_stream_rel_sweep_kernel(P
   __shared__ __align__(8) float2 ln_tab[32];
 
   const int64_t chunk = blockIdx.y;
-  const int64_t tile0 = chunk * a.tiles_per_chunk;
-  int64_t ntl = a.n_tiles - tile0;
-  if (ntl > a.tiles_per_chunk) ntl = a.tiles_per_chunk;
-  if (ntl < 0) ntl = 0;
+  const ChunkTiles ct = chunk_tiles(a.n_tiles);
 
   PlaneRel::Pair pr[NP];
   float2 hs[NP], ls[NP], hk[NP], lk[NP];
@@ -371,8 +365,8 @@ __global__ void __launch_bounds__(THREADS, MINB) plane_stream_rel_sweep_kernel(P
   ln_tab_load(ln_tab);
   pipe_init(bars);
   uint32_t g = 0;
-  int64_t tile = tile0;
-  staged_sweep<Rec, TILE>(a.src, tile0, ntl, stage[0], stage[1], bars, g, a.status, [&](const Rec* tl) {
+  int64_t tile = ct.first;
+  staged_sweep<Rec, TILE>(a.src, ct.first, ct.count, stage[0], stage[1], bars, g, a.status, [&](const Rec* tl) {
     const PlaneRel::Origin* og = a.org + tile * GPT;
 #pragma unroll 1
     for (int g0 = 0; g0 < TILE; g0 += G) {
@@ -456,8 +450,8 @@ __global__ void __launch_bounds__(THREADS, MINB) plane_stream_rel_sweep_kernel(P
         }
       }
     }
-    ++tile;
-  });
+    tile += ct.step;
+  }, ct.step);
 
   constexpr double kLn2 = 0.69314718055994530942;
 #pragma unroll
@@ -499,10 +493,7 @@ __global__ void __launch_bounds__(THREADS, MINB) sphere_swe_rel_sweep_kernel(Swe
   __shared__ __align__(8) uint64_t bars[2];
 
   const int64_t chunk = blockIdx.y;
-  const int64_t tile0 = chunk * a.tiles_per_chunk;
-  int64_t ntl = a.n_tiles - tile0;
-  if (ntl > a.tiles_per_chunk) ntl = a.tiles_per_chunk;
-  if (ntl < 0) ntl = 0;
+  const ChunkTiles ct = chunk_tiles(a.n_tiles);
 
   BveX2::Pair pr[NP];
   float2 hs[NP][NC], ls[NP][NC];
@@ -516,8 +507,8 @@ __global__ void __launch_bounds__(THREADS, MINB) sphere_swe_rel_sweep_kernel(Swe
 
   pipe_init(bars);
   uint32_t g = 0;
-  int64_t tile = tile0;
-  staged_sweep<Rec, TILE>(src, tile0, ntl, stage[0], stage[1], bars, g, a.status, [&](const Rec* tl) {
+  int64_t tile = ct.first;
+  staged_sweep<Rec, TILE>(src, ct.first, ct.count, stage[0], stage[1], bars, g, a.status, [&](const Rec* tl) {
     float2 ac[NP][NC];
 #pragma unroll
     for (int p = 0; p < NP; ++p)
@@ -585,7 +576,7 @@ __global__ void __launch_bounds__(THREADS, MINB) sphere_swe_rel_sweep_kernel(Swe
         }
       }
     }
-    ++tile;
+    tile += ct.step;
 #pragma unroll
     for (int p = 0; p < NP; ++p)
 #pragma unroll
@@ -593,7 +584,7 @@ __global__ void __launch_bounds__(THREADS, MINB) sphere_swe_rel_sweep_kernel(Swe
         comp_add(hs[p][c].x, ls[p][c].x, ac[p][c].x);
         comp_add(hs[p][c].y, ls[p][c].y, ac[p][c].y);
       }
-  });
+  }, ct.step);
 
 #pragma unroll
   for (int p = 0; p < NP; ++p) {

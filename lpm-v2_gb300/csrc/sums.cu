@@ -30,11 +30,14 @@ constexpr double kPi = 3.1415926535897932384626433832795027975;
 // FP32C sweep shapes (threads per CTA, targets per thread, tile, min CTAs per SM)
 constexpr int kBveTile = 256;
 // Shapes of the sphere-BVE FP32C sweep the autotuner chooses from: threads per CTA,
-// targets per thread (in pairs), CTAs per SM.  All fit without register spills.
+// targets per thread (in pairs), CTAs per SM, and whether its warps run decoupled (they lose less
+// to the near groups that some of them meet: icosahedral nest 5 7 % faster than the
+// block-synchronous pipeline, nest 6 2 %; at nest 7, with few near groups, 0.5 % slower).
 struct BveShape {
   int threads, tpt, minb;
+  bool decoupled;
 };
-constexpr BveShape kBveShapes[] = {{128, 4, 4}, {256, 4, 2}, {128, 6, 2}, {128, 8, 2}};
+constexpr BveShape kBveShapes[] = {{128, 4, 4, true}, {128, 4, 4, false}, {128, 6, 2, true}, {128, 8, 2, false}};
 constexpr int kBveShapeCount = sizeof(kBveShapes) / sizeof(kBveShapes[0]);
 constexpr int kPlaneThreads = 128, kPlaneTpt = 4, kPlaneTile = 256, kPlaneMinB = 4;
 // PSE sweeps (warp-decoupled pipeline): 256-source tiles in two stages; the divergence, whose
@@ -1029,16 +1032,16 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
       const dim3 grid(static_cast<unsigned>(ceil_div(job.nt, sh.threads * sh.tpt)), static_cast<unsigned>(plan.nsplit));
       switch (plan.shape) {
         case 0:
-          bve_rel_sweep_kernel<128, 4, kBveTile, 4><<<grid, 128, 0, job.stream>>>(a, org);
+          bve_rel_sweep_kernel<128, 4, kBveTile, 4, true><<<grid, 128, 0, job.stream>>>(a, org);
           break;
         case 1:
-          bve_rel_sweep_kernel<256, 4, kBveTile, 2><<<grid, 256, 0, job.stream>>>(a, org);
+          bve_rel_sweep_kernel<128, 4, kBveTile, 4, false><<<grid, 128, 0, job.stream>>>(a, org);
           break;
         case 2:
-          bve_rel_sweep_kernel<128, 6, kBveTile, 2><<<grid, 128, 0, job.stream>>>(a, org);
+          bve_rel_sweep_kernel<128, 6, kBveTile, 2, true><<<grid, 128, 0, job.stream>>>(a, org);
           break;
         default:
-          bve_rel_sweep_kernel<128, 8, kBveTile, 2><<<grid, 128, 0, job.stream>>>(a, org);
+          bve_rel_sweep_kernel<128, 8, kBveTile, 2, false><<<grid, 128, 0, job.stream>>>(a, org);
           break;
       }
       finish_bve_kernel<<<fin_grid, pb, 0, job.stream>>>(job.partial, plan.nsplit, job.nt, job.ib, job.x,
@@ -1390,16 +1393,22 @@ int autotune_bve_shape(const SumJob& job, int sm_count, int* shape) {
     const SumPlan p = plan_sum(j.kind, j.mode, j.ns, j.nt, sm_count, sh);
     rc = launch_sum(j, p);  // warm-up (and sort) run
     if (rc != LPM_OK) break;
-    cudaEventRecord(e0, j.stream);
-    rc = launch_sum(j, p);
-    cudaEventRecord(e1, j.stream);
-    if (rc != LPM_OK) break;
-    if (cudaEventSynchronize(e1) != cudaSuccess) {
-      rc = set_error(LPM_ERR_CUDA, "autotune: %s", cudaGetErrorString(cudaGetLastError()));
-      break;
+    float ms = 3.4e38f;
+    for (int again = 0; again < 3 && rc == LPM_OK; ++again) {  // the best of three: single runs scatter by a few percent
+      cudaEventRecord(e0, j.stream);
+      rc = launch_sum(j, p);
+      cudaEventRecord(e1, j.stream);
+      if (rc != LPM_OK) break;
+      if (cudaEventSynchronize(e1) != cudaSuccess) {
+        rc = set_error(LPM_ERR_CUDA, "autotune: %s", cudaGetErrorString(cudaGetLastError()));
+        break;
+      }
+      float one = 0.f;
+      cudaEventElapsedTime(&one, e0, e1);
+      ms = std::min(ms, one);
+      if (one > 5.f) break;  // a long sum's single run is good enough
     }
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, e0, e1);
+    if (rc != LPM_OK) break;
     if (ms < best_ms) {
       best_ms = ms;
       best = sh;
