@@ -1,7 +1,7 @@
-// pse_rel.cuh -- the sphere PSE operators in FP32C on the group-relative layout of the BVE
-// sweep (bve_rel.cuh), with a group-level cutoff: the Laplacian (K8 of the great-circle
-// distance, or the Gaussian of the chord), the gradient and the divergence (K1, the first-
-// derivative kernel, of the great-circle distance).
+// pse_rel.cuh -- the sphere PSE derivatives in FP32C on the group-relative layout of the BVE
+// sweep (bve_rel.cuh), with a group-level cutoff: the gradient and the divergence (K1, the first-
+// derivative kernel, of the great-circle distance), and the K8 Laplacian for an eps beyond the
+// angle polynomials of pse_lap.cuh.
 //
 // Reference, src/PSEDirectSum.f90 (kernels :611-640):
 //   PSESphereLaplacianAtParticles (:502-535)  L_i = eps^-4 sum_j (f_j - f_i) A_j K8(r)
@@ -33,7 +33,7 @@
 
 namespace lpm {
 
-enum PseRelOp { kPseOpLapK8 = 0, kPseOpLapGauss = 1, kPseOpGrad = 2, kPseOpDiv = 3 };
+enum PseRelOp { kPseOpLapK8 = 0, kPseOpGrad = 1, kPseOpDiv = 2 };
 enum PseRelAngle { kPseAngleSeries = 0, kPseAngleAsin = 1, kPseAngleChord = 2 };
 
 struct PseRel {
@@ -130,7 +130,7 @@ __device__ __forceinline__ void pse_pair(float2 dx, float2 dy, float2 dz, float2
     k = __fmul2_rn(poly, k);
   }
   const float2 wk = __fmul2_rn(hi2(rb), k);  // A_j K
-  if (OP == kPseOpLapK8 || OP == kPseOpLapGauss) {
+  if (OP == kPseOpLapK8) {
     // f_j - f_i = (f_j,hi - f_i,hi) + (f_j,lo - f_i,lo)
     const float2 df = __fadd2_rn(__fadd2_rn(lo2(rc), make_float2(-t.e0.x, -t.e0.y)),
                                  __fadd2_rn(hi2(rc), make_float2(-t.e1.x, -t.e1.y)));

@@ -15,6 +15,7 @@
 #include "ops.cuh"
 #include "plane_rel.cuh"
 #include "pse64.cuh"
+#include "pse_lap.cuh"
 #include "pse_rel.cuh"
 #include "seq_i64.cuh"
 #include "sort.cuh"
@@ -44,6 +45,7 @@ constexpr int kPlaneThreads = 128, kPlaneTpt = 4, kPlaneTile = 256, kPlaneMinB =
 // sweep holds more per-target state (128 registers), runs faster on 128-source tiles in four
 constexpr int kPseThreads = 128, kPseTpt = 4, kPseTile = 256, kPseMinB = 4, kPseStages = 2;
 constexpr int kPseDivTile = 128, kPseDivStages = 4;
+constexpr int kLapMinB = 4;
 constexpr int kStreamThreads = 128, kStreamTpt = 4, kStreamTile = 256, kStreamMinB = 4;
 constexpr int kBetaThreads = 128, kBetaTpt = 4, kBetaTile = 256, kBetaMinB = 4;
 constexpr int kSweMinB = 3;        // planar SWE velocity sweep: 128 x 4 targets, 3 CTAs per SM
@@ -340,7 +342,6 @@ int tile_of(int kind, int mode) {
 // the sweeps that share its layout, 64 for the PSE sweeps (their cutoff's granularity) and
 // the planar and beta-plane ones.
 int origin_group(int kind) {
-  static_assert(PseRel::kGroup == PlanePseRel::kGroup, "the Gaussian-chord kind serves the sphere and the plane");
   switch (kind) {
     case kSumBve:
     case kSumBveMesh:
@@ -353,7 +354,7 @@ int origin_group(int kind) {
     case kSumPseDiv:
       return PseRel::kGroup;
     case kSumPseK8Chord:
-      return PlanePseRel::kGroup;
+      return PseLap::kGroup;
     case kSumBetaPlane:
       return BetaRel::kGroup;
     case kSumBetaStream:
@@ -395,9 +396,12 @@ size_t rec_bytes(int kind, int mode) {
     case kSumPseGaussChord:
     case kSumPseGrad:
     case kSumPseDiv:
-      return sizeof(PseRel::Rec);  // also covers the planar record of the Gaussian-chord kind
+      static_assert(sizeof(PseLap::Rec) <= sizeof(PseRel::Rec) && sizeof(PseLap::Group) == sizeof(BveRel::Origin) &&
+                        PseLap::kGroup == PseRel::kGroup,
+                    "the Laplacians' layout fits the derivatives'");
+      return sizeof(PseRel::Rec);
     default:
-      return sizeof(PlanePseRel::Rec);
+      return sizeof(PseLap::Rec);
   }
 }
 
@@ -478,6 +482,9 @@ bool pse_culls_tiles(int kind) {
          kind == kSumPseDiv;
 }
 
+// The FP32C Laplacians (pse_lap.cuh), whose targets are split into floats once per call.
+bool pse_lap_kind(int kind) { return kind == kSumPseK8Geo || kind == kSumPseGaussChord || kind == kSumPseK8Chord; }
+
 // Shares per target block of a culled sweep: about six waves of CTAs in all, at most 32 per
 // block.  A block's in-reach work is split evenly, but tiles differ in cost (near and partly
 // reached groups), so finer CTAs balance the SMs better until the per-CTA scan of the tile
@@ -537,6 +544,10 @@ SumPlan plan_sum(int kind, int mode, int64_t ns, int64_t nt, int sm_count, int s
     pl.tperm_offset = align_up(pl.src_bytes, 256);
     pl.src_bytes = pl.tperm_offset + 2 * align_up(static_cast<size_t>(nt) * sizeof(int32_t), 256);
   }
+  if (mode == LPM_MODE_FP32C && pse_lap_kind(kind)) {
+    pl.tgt_offset = align_up(pl.src_bytes, 256);
+    pl.src_bytes = pl.tgt_offset + static_cast<size_t>(nt) * sizeof(PseLap::Tgt);
+  }
   if (mode == LPM_MODE_FP32C && kind == kSumSphereStream) {
     // the sources' own zeta A (2 x nt) and the two totals follow the group origins
     pl.src_bytes = align_up(pl.src_bytes, 256) + align_up(2 * static_cast<size_t>(nt) * sizeof(double), 256) +
@@ -585,6 +596,7 @@ SumPlan plan_sum(int kind, int mode, int64_t ns, int64_t nt, int sm_count, int s
     pl.aux_n_tiles = pp.n_tiles;
     pl.aux_tiles_per_chunk = pp.tiles_per_chunk;
     pl.aux_nsplit = pp.nsplit;
+    pl.aux_tgt_offset = pp.tgt_offset;
     pl.aux_src_offset = align_up(pl.src_bytes, 256);
     pl.src_bytes = pl.aux_src_offset + pp.src_bytes;
     pl.partial_bytes = std::max(pl.partial_bytes, pp.partial_bytes);
@@ -685,12 +697,8 @@ int launch_pse_rel(const SumJob& job, const SumPlan& plan, int64_t npad) {
   a.wait = job.wait;
   const bool series = job.eps <= 0.06 * job.radius;  // the asin^2 series angle (pse_rel.cuh)
   switch (job.kind) {
-    case kSumPseK8Geo:
-      if (series) pse_rel_launch<kPseOpLapK8, kPseAngleSeries>(job, plan, src_list, a);
-      else pse_rel_launch<kPseOpLapK8, kPseAngleAsin>(job, plan, src_list, a);
-      break;
-    case kSumPseGaussChord:
-      pse_rel_launch<kPseOpLapGauss, kPseAngleChord>(job, plan, src_list, a);
+    case kSumPseK8Geo:  // beyond the reach of the Laplacian's own angle polynomials
+      pse_rel_launch<kPseOpLapK8, kPseAngleAsin>(job, plan, src_list, a);
       break;
     case kSumPseGrad:
       if (series) pse_rel_launch<kPseOpGrad, kPseAngleSeries>(job, plan, src_list, a);
@@ -706,57 +714,85 @@ int launch_pse_rel(const SumJob& job, const SumPlan& plan, int64_t npad) {
 }  // namespace
 
 namespace {
-int launch_plane_pse_rel(const SumJob& job, const SumPlan& plan, int64_t npad) {
+template <bool SPHERE, bool K8, int ANG>
+void pse_lap_launch(const SumJob& job, const SumPlan& plan, const int32_t* src_list, double inv_a, const PseLapArgs& a) {
+  const unsigned prep = static_cast<unsigned>(plan.n_tiles + ceil_div(job.nt, kPseTile));
+  pse_lap_prep_kernel<SPHERE, ANG, kPseTile><<<prep, kPseTile, 0, job.stream>>>(
+      job.x, job.y, job.z, job.s1, job.area, src_list, job.ns, plan.n_tiles, inv_a, a.c_cut, a.tperm, job.ib, job.nt,
+      const_cast<PseLap::Rec*>(a.src), const_cast<PseLap::Group*>(a.grp), const_cast<float4*>(a.tball),
+      const_cast<PseLap::Tgt*>(a.tgt));
+  const dim3 grid(static_cast<unsigned>(ceil_div(job.nt, kPseThreads * kPseTpt)), static_cast<unsigned>(plan.nsplit));
+  pse_lap_sweep_kernel<SPHERE, K8, ANG, kPseThreads, kPseTpt, kPseTile, kLapMinB, kPseStages>
+      <<<grid, kPseThreads, 0, job.stream>>>(a);
+}
+
+// An FP32C Laplacian (pse_lap.cuh): the curve orders, prep and sweep.
+int launch_pse_lap(const SumJob& job, const SumPlan& plan, int64_t npad) {
+  const bool sphere = job.z != nullptr && job.kind != kSumPseK8Chord;
+  const double inv_a = sphere ? 1.0 / job.radius : 1.0;
+  const double scale = job.eps * inv_a;  // eps in the positions' unit
+  const double cut = std::sqrt(static_cast<double>(PseRel::kCutR2)) * scale;
+  if (job.kind == kSumPseK8Geo && cut > kLapFarMax) return launch_pse_rel(job, plan, npad);
   const int32_t* src_list = job.src_idx;
   const int32_t* tperm = nullptr;
-  auto sort2 = [&](const int32_t* in, int32_t* out) {
-    return curve_sort2d(job.stream, job.nt, in, job.x, job.y, job.sort_scratch, job.sort_bytes, out);
+  auto sort_of = [&](int64_t n, const int32_t* in, int32_t* out) {
+    return sphere ? curve_sort(job.stream, n, in, job.x, job.y, job.z, inv_a, job.sort_scratch, job.sort_bytes, out)
+                  : curve_sort2d(job.stream, n, in, job.x, job.y, job.sort_scratch, job.sort_bytes, out);
   };
+  auto sort_targets = [&](const int32_t* in, int32_t* out) { return sort_of(job.nt, in, out); };
   if (targets_cover_sources(job, plan)) {
-    // one sort: every particle along the curve over their bounding box, the sources picked
-    // out of it in that order
-    LPM_TRY(sorted_targets(job, plan, sort2, &tperm));
+    // one sort: every particle in curve order, the sources picked out of it in that order
+    // (the same order as a sort of their own, whose keys are the same function of position)
+    LPM_TRY(sorted_targets(job, plan, sort_targets, &tperm));
     LPM_TRY(select_in_order(job.stream, job.n, tperm, job.ns, job.src_idx, job.sort_scratch, job.sort_bytes,
                             job.sorted));
     src_list = job.sorted;
   } else {
     if (job.sort_scratch) {
-      LPM_TRY(curve_sort2d(job.stream, job.ns, job.src_idx, job.x, job.y, job.sort_scratch, job.sort_bytes,
-                           job.sorted));
+      LPM_TRY(sort_of(job.ns, job.src_idx, job.sorted));
       src_list = job.sorted;
     }
-    LPM_TRY(sorted_targets(job, plan, sort2, &tperm));
+    LPM_TRY(sorted_targets(job, plan, sort_targets, &tperm));
   }
-  PlanePseRelArgs a;
-  a.tperm = tperm;
-  a.x = job.x;
-  a.y = job.y;
-  a.f = job.s1;
-  a.ks2 = static_cast<float>(1.0 / (job.eps * job.eps));
-  a.c_cut = static_cast<float>(std::sqrt(static_cast<double>(PseRel::kCutR2)) * job.eps);
-  a.src = static_cast<PlanePseRel::Rec*>(job.src_buf);
-  a.org = reinterpret_cast<PlaneRel::Origin*>(static_cast<char*>(job.src_buf) +
-                                              align_up(static_cast<size_t>(npad) * sizeof(PlanePseRel::Rec), 256));
-  // the tile balls follow the origins (plan_sum)
-  a.tball = reinterpret_cast<const float4*>(
-      reinterpret_cast<const char*>(a.org) +
-      align_up(static_cast<size_t>(plan.n_tiles) * (kPseTile / PlanePseRel::kGroup) * sizeof(PlaneRel::Origin), 256));
+  char* base = static_cast<char*>(job.src_buf);
+  const size_t grp_off = align_up(static_cast<size_t>(npad) * sizeof(PseLap::Rec), 256);
+  const size_t ball_off =
+      align_up(grp_off + static_cast<size_t>(plan.n_tiles) * (kPseTile / PseLap::kGroup) * sizeof(PseLap::Group), 256);
+  PseLapArgs a;
+  a.src = reinterpret_cast<const PseLap::Rec*>(base);
+  a.grp = reinterpret_cast<const PseLap::Group*>(base + grp_off);
+  a.tball = reinterpret_cast<const float4*>(base + ball_off);
+  a.tgt = reinterpret_cast<const PseLap::Tgt*>(base + plan.tgt_offset);
+  a.c_cut = static_cast<float>(cut);
+  // y = -log2(e) r^2 as a polynomial in the squared chord: r^2 = v / scale^2, or theta^2 / scale^2 with
+  // theta^2 = 4 asin^2(sqrt(v) / 2) interpolated at the Chebyshev nodes of [0, 0.2] and [0, 1.3]
+  // (4.4e-9 and 6.7e-9 relative); both stay monotonic beyond, where the kernel is zero
+  constexpr double kNear[4] = {0.9999999957139412, 0.08333401828821702, 0.011094097040298852, 0.0019196358256262074};
+  constexpr double kFar[7] = {1.0000000054898175,     0.08333292065778725,    0.011116116508061118,
+                              0.001763274276537942,   0.00036433929246890823, 1.1828733148294194e-05,
+                              3.4221076886605545e-05};
+  const double ks = -1.4426950408889634 / (scale * scale);
+  const int ang = job.kind != kSumPseK8Geo ? kLapChord : (cut <= kLapNearMax ? kLapNear : kLapFar);
+  for (int k = 0; k < 7; ++k) {
+    const double c = ang == kLapChord ? (k == 0 ? 1.0 : 0.0) : (ang == kLapNear ? (k < 4 ? kNear[k] : 0.0) : kFar[k]);
+    a.q[k] = static_cast<float>(ks * c);
+  }
   a.n_tiles = plan.n_tiles;
-  a.tiles_per_chunk = plan.tiles_per_chunk;
   a.ib = job.ib;
   a.nt = job.nt;
+  a.tperm = tperm;
   a.partial = job.partial;
   a.status = job.status;
-  plane_pse_rel_prep_kernel<kPseTile><<<static_cast<unsigned>(plan.n_tiles), kPseTile, 0, job.stream>>>(
-      job.x, job.y, job.s1, job.area, src_list, job.ns, const_cast<PlanePseRel::Rec*>(a.src),
-      const_cast<PlaneRel::Origin*>(a.org), const_cast<float4*>(a.tball));
-  const dim3 grid(static_cast<unsigned>(ceil_div(job.nt, kPseThreads * kPseTpt)), static_cast<unsigned>(plan.nsplit));
-  if (job.kind == kSumPseK8Chord) {
-    plane_pse_rel_sweep_kernel<true, kPseThreads, kPseTpt, kPseTile, kPseMinB, kPseStages>
-        <<<grid, kPseThreads, 0, job.stream>>>(a);
+  a.wait = job.wait;
+  if (!sphere) {
+    if (job.kind == kSumPseK8Chord) pse_lap_launch<false, true, kLapChord>(job, plan, src_list, inv_a, a);
+    else pse_lap_launch<false, false, kLapChord>(job, plan, src_list, inv_a, a);
+  } else if (job.kind == kSumPseGaussChord) {
+    pse_lap_launch<true, false, kLapChord>(job, plan, src_list, inv_a, a);
+  } else if (ang == kLapNear) {
+    pse_lap_launch<true, true, kLapNear>(job, plan, src_list, inv_a, a);
   } else {
-    plane_pse_rel_sweep_kernel<false, kPseThreads, kPseTpt, kPseTile, kPseMinB, kPseStages>
-        <<<grid, kPseThreads, 0, job.stream>>>(a);
+    pse_lap_launch<true, true, kLapFar>(job, plan, src_list, inv_a, a);
   }
   return LPM_OK;
 }
@@ -1084,13 +1120,7 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
     case kSumPseK8Chord: {
       const double e4 = (job.eps * job.eps) * (job.eps * job.eps);
       const double cscale = (job.kind == kSumPseGaussChord ? 4.0 : 1.0) / kPi / e4;
-      if (job.z && (job.kind == kSumPseK8Geo || job.kind == kSumPseGaussChord)) {
-        // sphere: group-relative sweep with the r^2 >= 49 group cutoff (pse_rel.cuh)
-        LPM_TRY(launch_pse_rel(job, plan, npad));
-      } else {
-        // plane: the 2-D group-relative sweep with the same cutoff (plane_rel.cuh)
-        LPM_TRY(launch_plane_pse_rel(job, plan, npad));
-      }
+      LPM_TRY(launch_pse_lap(job, plan, npad));
       finish_scalar_kernel<<<fin_grid, pb, 0, job.stream>>>(job.partial, plan.nsplit, job.nt, cscale, job.out0);
       break;
     }
@@ -1252,7 +1282,8 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
       pp.n_tiles = plan.aux_n_tiles;
       pp.tiles_per_chunk = plan.aux_tiles_per_chunk;
       pp.nsplit = plan.aux_nsplit;
-      LPM_TRY(launch_pse_rel(jp, pp, plan.aux_n_tiles * kPseTile));
+      pp.tgt_offset = plan.aux_tgt_offset;
+      LPM_TRY(launch_pse_lap(jp, pp, plan.aux_n_tiles * kPseTile));
       finish_scalar_kernel<<<fin_grid, pb, 0, job.stream>>>(job.partial, pp.nsplit, job.nt,
                                                             1.0 / (kPi * job.eps * job.eps), job.out3);
       break;
@@ -1329,7 +1360,8 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
       pp.n_tiles = plan.aux_n_tiles;
       pp.tiles_per_chunk = plan.aux_tiles_per_chunk;
       pp.nsplit = plan.aux_nsplit;
-      LPM_TRY(launch_plane_pse_rel(jp, pp, plan.aux_n_tiles * kPseTile));
+      pp.tgt_offset = plan.aux_tgt_offset;
+      LPM_TRY(launch_pse_lap(jp, pp, plan.aux_n_tiles * kPseTile));
       const double e4 = (job.eps * job.eps) * (job.eps * job.eps);
       finish_scalar_kernel<<<fin_grid, pb, 0, job.stream>>>(job.partial, pp.nsplit, job.nt, 1.0 / kPi / e4,
                                                             job.out3);

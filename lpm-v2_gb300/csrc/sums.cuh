@@ -21,10 +21,11 @@ struct SumPlan {
   // a second sweep of the same job (the planar SWE surface-height Laplacian): its tiles and
   // split, its source records at src_buf + aux_src_offset; it reuses the partials
   int64_t aux_n_tiles = 0, aux_tiles_per_chunk = 0, aux_nsplit = 0;
-  size_t aux_src_offset = 0;
+  size_t aux_src_offset = 0, aux_tgt_offset = 0;
   // FP32C PSE sums: the targets' curve order (two lists of nt int32: [ib, ib + nt) and its
   // sorted permutation) at src_buf + tperm_offset; 0 when the sweep takes targets in order
   size_t tperm_offset = 0;
+  size_t tgt_offset = 0;  // FP32C Laplacians: the targets as floats (PseLap::Tgt) at src_buf + tgt_offset
 };
 
 enum SumKind : int {
