@@ -1,5 +1,7 @@
-// hilbert.cuh -- index along a Hilbert curve of a cell of a 2^10 x 2^10 x 2^10 grid (3-D)
-// or of a 2^16 x 2^16 grid (2-D).
+// hilbert.cuh -- index along a Hilbert curve of a cell of a 2^16 x 2^16 grid (2-D), of a direction on
+// the cube around the sphere, and of a cell of a 2^10 x 2^10 x 2^10 grid (3-D; the orders below do
+// not use it: where that curve leaves the sphere's shell and enters it again elsewhere, consecutive
+// sources lie in two pieces).
 //
 // J. Skilling, "Programming the Hilbert curve", AIP Conf. Proc. 707, 381 (2004): the cell
 // coordinates are turned in place into the "transpose" of the Hilbert index (undo the
@@ -80,6 +82,43 @@ __host__ __device__ inline uint32_t hilbert_index2d(uint32_t x0, uint32_t x1) {
   X[0] ^= t;
   X[1] ^= t;
   return (spread16(X[0]) << 1) | spread16(X[1]);
+}
+
+// The curve index (kSphereCurveBits bits) of a point's direction: the six faces of the cube around
+// the sphere in turn, on each a 2-D Hilbert curve over 2^10 x 2^10 cells, laid so that one face's
+// curve ends at the cube's corner where the next one's starts.  The faces' gnomonic coordinates are
+// evened out by u (1.273 - 0.273 |u|), about (4 / pi) atan u.  Groups of 32 of 98,304 even sources have a
+// mean radius of 0.052 (95 % below 0.067) in this order, 0.076 (0.159) along the 3-D curve.
+constexpr int kSphereCurveBits = 23;
+
+__host__ __device__ inline uint32_t sphere_curve_index(float x, float y, float z) {
+  const float ax = x < 0.f ? -x : x, ay = y < 0.f ? -y : y, az = z < 0.f ? -z : z;
+  uint32_t face;
+  float m, u, v;  // the largest component, and the face's coordinates along and across its curve
+  if (ax >= ay && ax >= az) {
+    m = ax;
+    face = x < 0.f ? 0u : 5u;
+    u = x < 0.f ? z : -y;
+    v = x < 0.f ? y : -z;
+  } else if (ay >= az) {
+    m = ay;
+    face = y < 0.f ? 1u : 3u;
+    u = y < 0.f ? -z : z;
+    v = x;
+  } else {
+    m = az;
+    face = z < 0.f ? 2u : 4u;
+    u = z < 0.f ? y : x;
+    v = z < 0.f ? x : -y;
+  }
+  const float inv = m > 0.f ? 1.f / m : 0.f;
+  uint32_t c[2];
+  for (int k = 0; k < 2; ++k) {
+    const float w = (k == 0 ? u : v) * inv, wa = w < 0.f ? -w : w;
+    const float q = (w * (1.273f - 0.273f * wa) + 1.f) * 32768.f;
+    c[k] = q > 0.f ? (q < 65535.f ? static_cast<uint32_t>(q) : 65535u) : 0u;  // (NaN: 0)
+  }
+  return (face << 20) | (hilbert_index2d(c[0], c[1]) >> 12);
 }
 
 }  // namespace lpm

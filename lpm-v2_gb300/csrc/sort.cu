@@ -1,13 +1,11 @@
 // sort.cu -- spatial (Hilbert-curve) ordering of the source particles on the device.
 //
-// The FP32C sweeps store every source relative to the origin of its group (64 or 128
-// consecutive sources), so groups must be spatially compact: sources are ordered by the 30-bit index, along a 3-D
-// Hilbert curve over a 2^10 grid per axis, of the cell holding their unit-scaled position,
-// with a device radix sort (CUB).  Consecutive Hilbert cells are face neighbours, so a group
-// of consecutive sources forms one connected patch (a Hilbert-curve order jumps across the grid at
-// its octant boundaries, which leaves some groups in two distant pieces).  The order only
-// affects rounding (the FP32C sum is order-independent to its error bound); FP64 sums keep
-// the reference's ascending order.
+// The FP32C sweeps store every source relative to the origin of its group (32 to 128
+// consecutive sources), so groups must be spatially compact: sources are ordered by an index along a
+// Hilbert curve with a device radix sort (CUB).  On the sphere the curve runs over the faces of the
+// cube around it (sphere_curve_index), 23 bits, three passes of the sort; in the plane over a 2^16
+// grid on the bounding box.  The order only affects rounding (the FP32C sum is order-independent to
+// its error bound); FP64 sums keep the reference's ascending order.
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_select.cuh>
 
@@ -18,26 +16,17 @@
 namespace lpm {
 namespace {
 
-__device__ __forceinline__ uint32_t quant10(double p) {
-  double t = (p + 1.0) * 512.0;
-  t = t < 0.0 ? 0.0 : (t > 1023.0 ? 1023.0 : t);
-  return static_cast<uint32_t>(t);
-}
-
-__device__ __forceinline__ uint32_t cell_key(double px, double py, double pz) {
-  return hilbert_index30(quant10(px), quant10(py), quant10(pz));
-}
-
 __global__ void curve_keys_kernel(int64_t ns, const int32_t* idx, const double* x, const double* y,
                                    const double* z, double inv_a, uint32_t* keys, int32_t* vals) {
   const int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (k >= ns) return;
   const int32_t j = idx[k];
-  keys[k] = cell_key(x[j] * inv_a, y[j] * inv_a, z ? z[j] * inv_a : 0.0);
+  keys[k] = sphere_curve_index(static_cast<float>(x[j] * inv_a), static_cast<float>(y[j] * inv_a),
+                               z ? static_cast<float>(z[j] * inv_a) : 0.f);
   vals[k] = j;
 }
 
-// 64-bit keys: the group in the high bits, the curve index of the group-scaled position low.
+// 64-bit keys: the group in the high bits, the curve index of the position low.
 __global__ void grouped_curve_keys_kernel(int64_t ns, const int32_t* idx, const int32_t* grp, const double* x,
                                            const double* y, const double* z, const double* inv_a, uint64_t* keys,
                                            int32_t* vals) {
@@ -46,7 +35,8 @@ __global__ void grouped_curve_keys_kernel(int64_t ns, const int32_t* idx, const 
   const int32_t j = idx[k];
   const int32_t g = grp[k];
   const double s = inv_a[g];
-  keys[k] = (static_cast<uint64_t>(g) << 30) | cell_key(x[j] * s, y[j] * s, z[j] * s);
+  keys[k] = (static_cast<uint64_t>(g) << kSphereCurveBits) |
+            sphere_curve_index(static_cast<float>(x[j] * s), static_cast<float>(y[j] * s), static_cast<float>(z[j] * s));
   vals[k] = j;
 }
 
@@ -125,7 +115,7 @@ __global__ void curve2d_keys_kernel(int64_t ns, const int32_t* idx, const double
 int end_bit_for(int n_groups) {
   int b = 0;
   while ((1 << b) < n_groups) ++b;
-  return 30 + b;
+  return kSphereCurveBits + b;
 }
 
 }  // namespace
@@ -166,7 +156,7 @@ size_t curve_sort_bytes(int64_t ns) {
   size_t temp = 0;
   cub::DeviceRadixSort::SortPairs(nullptr, temp, static_cast<const uint32_t*>(nullptr), static_cast<uint32_t*>(nullptr),
                                   static_cast<const int32_t*>(nullptr), static_cast<int32_t*>(nullptr),
-                                  static_cast<int>(ns), 0, 30);
+                                  static_cast<int>(ns), 0, kSphereCurveBits);
   // keys in/out + values in
   return align_up(temp, 256) + 3 * align_up(static_cast<size_t>(ns) * 4, 256);
 }
@@ -177,7 +167,7 @@ int curve_sort(cudaStream_t stream, int64_t ns, const int32_t* idx, const double
   size_t temp = 0;
   cub::DeviceRadixSort::SortPairs(nullptr, temp, static_cast<const uint32_t*>(nullptr), static_cast<uint32_t*>(nullptr),
                                   static_cast<const int32_t*>(nullptr), static_cast<int32_t*>(nullptr),
-                                  static_cast<int>(ns), 0, 30);
+                                  static_cast<int>(ns), 0, kSphereCurveBits);
   const size_t arr = align_up(static_cast<size_t>(ns) * 4, 256);
   if (scratch_bytes < align_up(temp, 256) + 3 * arr)
     return set_error(LPM_ERR_STATE, "curve sort scratch too small");
@@ -190,7 +180,7 @@ int curve_sort(cudaStream_t stream, int64_t ns, const int32_t* idx, const double
                                                                                    vals_in);
   LPM_CUDA_TRY(cudaGetLastError());
   LPM_CUDA_TRY(cub::DeviceRadixSort::SortPairs(d_temp, temp, keys_in, keys_out, vals_in, sorted,
-                                               static_cast<int>(ns), 0, 30, stream));
+                                               static_cast<int>(ns), 0, kSphereCurveBits, stream));
   return LPM_OK;
 }
 
