@@ -14,7 +14,7 @@
 //    target at a source's position): the target forms (t_hi, t_lo) = rel2(t, o) with
 //    exactly the operations of the sources, and d = (t_hi - s_hi) + (t_lo - s_lo) keeps ~48
 //    bits; a self pair cancels bit for bit.
-// A compact group (R <= a/2 and R <= 64 x its smallest spacing h, i.e. a patch of a
+// A compact group (R <= a/2 and R <= 32 x its smallest spacing h, i.e. a patch of a
 // quasi-uniform point set) takes the far form for every target: the group record carries
 // R = 0, and its records use rel2_fast, the target's far-form operations, so a self pair
 // still cancels bit for bit.  For a target near such a group the roundings are an absolute
@@ -75,7 +75,9 @@ struct BveRel {
   static constexpr int kGroup = 128;
   static constexpr float kNearFactor = 3.0f;  // near: |t - o| < kNearFactor R
   static constexpr float kCompactRadius = 0.5f;  // compact: R <= kCompactRadius (unit sphere)
-  static constexpr float kCompactRatio = 64.0f;  // and R <= kCompactRatio h
+  // and R <= kCompactRatio h: refined meshes have R / h of 10-18 (median 12), sets without an even spacing
+  // 44 and more (their closest pairs are rarely consecutive, so h alone does not show them)
+  static constexpr float kCompactRatio = 32.0f;
 };
 
 // Offset of a hi/lo value from a float origin, rounded once: fl(p - o) to ~2^-24 relative
@@ -402,7 +404,7 @@ __device__ __forceinline__ SplitPoint split_point(double px, double py, double p
 // The frame of the thread's group of G sources within a tile of TILE (one CTA of TILE
 // threads, every thread one source): the origin o (the centroid in FP32: any point near it
 // does, and one without a low part saves the targets' offsets an operation), the radius R about o,
-// whether the group is compact (R <= a/2 and R <= 64 x the smallest distance h between
+// whether the group is compact (R <= a/2 and R <= 32 x the smallest distance h between
 // consecutive sources) and whether every |c_j| <= 2^-30 h^2 (c_j negligible in q), c_j =
 // |p|^2 - 1.  All of it in FP32 from the hi/lo positions (the offsets are exact to 2^-24): the FP64
 // pipe would bound this kernel.  R is widened by its rounding.

@@ -84,14 +84,15 @@ __host__ __device__ inline uint32_t hilbert_index2d(uint32_t x0, uint32_t x1) {
   return (spread16(X[0]) << 1) | spread16(X[1]);
 }
 
-// The curve index (kSphereCurveBits bits) of a point's direction: the six faces of the cube around
-// the sphere in turn, on each a 2-D Hilbert curve over 2^10 x 2^10 cells, laid so that one face's
+// The curve index of a point's direction, of `bits` bits (3 + 2 k): the six faces of the cube around
+// the sphere in turn, on each a 2-D Hilbert curve over 2^k x 2^k cells, laid so that one face's
 // curve ends at the cube's corner where the next one's starts.  The faces' gnomonic coordinates are
 // evened out by u (1.273 - 0.273 |u|), about (4 / pi) atan u.  Groups of 32 of 98,304 even sources have a
 // mean radius of 0.052 (95 % below 0.067) in this order, 0.076 (0.159) along the 3-D curve.
-constexpr int kSphereCurveBits = 23;
+constexpr int kSphereCurveBits = 23;      // three passes of a radix sort
+constexpr int kSphereCurveBitsFine = 27;  // four
 
-__host__ __device__ inline uint32_t sphere_curve_index(float x, float y, float z) {
+__host__ __device__ inline uint32_t sphere_curve_index(float x, float y, float z, int bits) {
   const float ax = x < 0.f ? -x : x, ay = y < 0.f ? -y : y, az = z < 0.f ? -z : z;
   uint32_t face;
   float m, u, v;  // the largest component, and the face's coordinates along and across its curve
@@ -118,7 +119,7 @@ __host__ __device__ inline uint32_t sphere_curve_index(float x, float y, float z
     const float q = (w * (1.273f - 0.273f * wa) + 1.f) * 32768.f;
     c[k] = q > 0.f ? (q < 65535.f ? static_cast<uint32_t>(q) : 65535u) : 0u;  // (NaN: 0)
   }
-  return (face << 20) | (hilbert_index2d(c[0], c[1]) >> 12);
+  return (face << (bits - 3)) | (hilbert_index2d(c[0], c[1]) >> (35 - bits));
 }
 
 }  // namespace lpm

@@ -323,7 +323,7 @@ struct lpm_bve_solver {
   double* psi = nullptr;  // psi_rel, psi_abs
 
   int sort_sources() {
-    return curve_sort(stream, ns, idx, x, y, z, 1.0 / radius, sort_scratch, sort_bytes, sorted);
+    return curve_sort(stream, ns, idx, x, y, z, 1.0 / radius, sort_scratch, sort_bytes, sorted, kSphereCurveBitsFine);
   }
 
   SumJob job(const double* px, const double* py, const double* pz, const double* pq, int kind,

@@ -3,8 +3,8 @@
 // The FP32C sweeps store every source relative to the origin of its group (32 to 128
 // consecutive sources), so groups must be spatially compact: sources are ordered by an index along a
 // Hilbert curve with a device radix sort (CUB).  On the sphere the curve runs over the faces of the
-// cube around it (sphere_curve_index), 23 bits, three passes of the sort; in the plane over a 2^16
-// grid on the bounding box.  The order only affects rounding (the FP32C sum is order-independent to
+// cube around it (sphere_curve_index), 23 bits and three passes of the sort, or 27 and four for the
+// order that a solver's step keeps for its four sums; in the plane over a 2^16 grid on the bounding box.  The order only affects rounding (the FP32C sum is order-independent to
 // its error bound); FP64 sums keep the reference's ascending order.
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_select.cuh>
@@ -17,12 +17,12 @@ namespace lpm {
 namespace {
 
 __global__ void curve_keys_kernel(int64_t ns, const int32_t* idx, const double* x, const double* y,
-                                   const double* z, double inv_a, uint32_t* keys, int32_t* vals) {
+                                   const double* z, double inv_a, int bits, uint32_t* keys, int32_t* vals) {
   const int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (k >= ns) return;
   const int32_t j = idx[k];
   keys[k] = sphere_curve_index(static_cast<float>(x[j] * inv_a), static_cast<float>(y[j] * inv_a),
-                               z ? static_cast<float>(z[j] * inv_a) : 0.f);
+                               z ? static_cast<float>(z[j] * inv_a) : 0.f, bits);
   vals[k] = j;
 }
 
@@ -36,7 +36,7 @@ __global__ void grouped_curve_keys_kernel(int64_t ns, const int32_t* idx, const 
   const int32_t g = grp[k];
   const double s = inv_a[g];
   keys[k] = (static_cast<uint64_t>(g) << kSphereCurveBits) |
-            sphere_curve_index(static_cast<float>(x[j] * s), static_cast<float>(y[j] * s), static_cast<float>(z[j] * s));
+            sphere_curve_index(static_cast<float>(x[j] * s), static_cast<float>(y[j] * s), static_cast<float>(z[j] * s), kSphereCurveBits);
   vals[k] = j;
 }
 
@@ -156,18 +156,18 @@ size_t curve_sort_bytes(int64_t ns) {
   size_t temp = 0;
   cub::DeviceRadixSort::SortPairs(nullptr, temp, static_cast<const uint32_t*>(nullptr), static_cast<uint32_t*>(nullptr),
                                   static_cast<const int32_t*>(nullptr), static_cast<int32_t*>(nullptr),
-                                  static_cast<int>(ns), 0, kSphereCurveBits);
+                                  static_cast<int>(ns), 0, kSphereCurveBitsFine);
   // keys in/out + values in
   return align_up(temp, 256) + 3 * align_up(static_cast<size_t>(ns) * 4, 256);
 }
 
 int curve_sort(cudaStream_t stream, int64_t ns, const int32_t* idx, const double* x, const double* y,
-                const double* z, double inv_a, void* scratch, size_t scratch_bytes, int32_t* sorted) {
+                const double* z, double inv_a, void* scratch, size_t scratch_bytes, int32_t* sorted, int bits) {
   if (ns <= 0) return LPM_OK;
   size_t temp = 0;
   cub::DeviceRadixSort::SortPairs(nullptr, temp, static_cast<const uint32_t*>(nullptr), static_cast<uint32_t*>(nullptr),
                                   static_cast<const int32_t*>(nullptr), static_cast<int32_t*>(nullptr),
-                                  static_cast<int>(ns), 0, kSphereCurveBits);
+                                  static_cast<int>(ns), 0, kSphereCurveBitsFine);
   const size_t arr = align_up(static_cast<size_t>(ns) * 4, 256);
   if (scratch_bytes < align_up(temp, 256) + 3 * arr)
     return set_error(LPM_ERR_STATE, "curve sort scratch too small");
@@ -176,11 +176,11 @@ int curve_sort(cudaStream_t stream, int64_t ns, const int32_t* idx, const double
   uint32_t* keys_in = reinterpret_cast<uint32_t*>(base + align_up(temp, 256));
   uint32_t* keys_out = reinterpret_cast<uint32_t*>(base + align_up(temp, 256) + arr);
   int32_t* vals_in = reinterpret_cast<int32_t*>(base + align_up(temp, 256) + 2 * arr);
-  curve_keys_kernel<<<static_cast<unsigned>(ceil_div(ns, 256)), 256, 0, stream>>>(ns, idx, x, y, z, inv_a, keys_in,
+  curve_keys_kernel<<<static_cast<unsigned>(ceil_div(ns, 256)), 256, 0, stream>>>(ns, idx, x, y, z, inv_a, bits, keys_in,
                                                                                    vals_in);
   LPM_CUDA_TRY(cudaGetLastError());
   LPM_CUDA_TRY(cub::DeviceRadixSort::SortPairs(d_temp, temp, keys_in, keys_out, vals_in, sorted,
-                                               static_cast<int>(ns), 0, kSphereCurveBits, stream));
+                                               static_cast<int>(ns), 0, bits, stream));
   return LPM_OK;
 }
 

@@ -1,6 +1,7 @@
 // sort.cuh -- Hilbert-curve ordering of source particles (device radix sort).
 #pragma once
 
+#include "hilbert.cuh"
 #include "lpm_common.cuh"
 
 namespace lpm {
@@ -8,10 +9,12 @@ namespace lpm {
 // Scratch bytes curve_sort needs for ns sources.
 size_t curve_sort_bytes(int64_t ns);
 
-// sorted[0..ns) = idx[0..ns) ordered by the Hilbert-curve index of (x, y, z) * inv_a.  z may be NULL
-// (planar particles).  Enqueued on `stream`; no allocation.
+// sorted[0..ns) = idx[0..ns) ordered by the Hilbert-curve index of the direction of (x, y, z), of
+// `bits` bits (kSphereCurveBits, or kSphereCurveBitsFine for an order that is kept: finer cells, one
+// more pass of the sort).  Enqueued on `stream`; no allocation.
 int curve_sort(cudaStream_t stream, int64_t ns, const int32_t* idx, const double* x, const double* y,
-                const double* z, double inv_a, void* scratch, size_t scratch_bytes, int32_t* sorted);
+                const double* z, double inv_a, void* scratch, size_t scratch_bytes, int32_t* sorted,
+                int bits = kSphereCurveBits);
 
 // Hilbert-curve order within groups (ensemble instances): entries are ordered by group first, then
 // by the Hilbert-curve index of (x, y, z) * inv_a[group]; idx/grp are the particle and group of each
