@@ -37,8 +37,16 @@ constexpr int kBveTile = 256;
 struct BveShape {
   int threads, tpt, minb;
   bool decoupled;
+  int tile;  // sources per sweep tile: 256, or 128 (a group) for small sets
 };
-constexpr BveShape kBveShapes[] = {{128, 4, 4, true}, {128, 4, 4, false}, {128, 6, 2, true}, {128, 8, 2, false}};
+// The last one is for small sets, whose few targets and sources leave most SMs idle at 512 targets by
+// 256 sources a CTA: icosahedral nest 3 (1,922 targets, 1,280 sources) has 20 such CTAs, and 80 of 256
+// targets by one group.
+constexpr BveShape kBveShapes[] = {{128, 4, 4, true, kBveTile},
+                                   {128, 4, 4, false, kBveTile},
+                                   {128, 6, 2, true, kBveTile},
+                                   {128, 8, 2, false, kBveTile},
+                                   {128, 2, 6, true, BveRel::kGroup}};
 constexpr int kBveShapeCount = sizeof(kBveShapes) / sizeof(kBveShapes[0]);
 constexpr int kPlaneThreads = 128, kPlaneTpt = 4, kPlaneTile = 256, kPlaneMinB = 4;
 // PSE sweeps (warp-decoupled pipeline): 256-source tiles in two stages; the divergence, whose
@@ -585,9 +593,11 @@ SumPlan plan_sum(int kind, int mode, int64_t ns, int64_t nt, int sm_count, int s
     pl.tiles_per_chunk = pl.n_tiles;
     pl.nsplit = cull_shares(tblocks, slots);
   } else {
-    const int64_t nsplit = choose_split(tblocks, pl.n_tiles, slots, 65535);
-    pl.tiles_per_chunk = ceil_div(pl.n_tiles, nsplit);
-    pl.nsplit = ceil_div(pl.n_tiles, pl.tiles_per_chunk);
+    const bool bve = kind == kSumBve || kind == kSumBveMesh;
+    const int64_t tiles = bve ? pl.n_tiles * (kBveTile / kBveShapes[shape].tile) : pl.n_tiles;
+    const int64_t nsplit = choose_split(tblocks, tiles, slots, 65535);
+    pl.tiles_per_chunk = ceil_div(tiles, nsplit);
+    pl.nsplit = ceil_div(tiles, pl.tiles_per_chunk);
   }
   pl.partial_bytes = static_cast<size_t>(pl.nsplit) * comps_of(kind) * nt * sizeof(double);
   if (kind == kSumSwePlane || kind == kSumSweSphere) {
@@ -1065,6 +1075,7 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
       a.status = job.status;
       a.wait = job.wait;
       const BveShape sh = kBveShapes[plan.shape];
+      a.n_tiles = plan.n_tiles * (kBveTile / sh.tile);
       const dim3 grid(static_cast<unsigned>(ceil_div(job.nt, sh.threads * sh.tpt)), static_cast<unsigned>(plan.nsplit));
       switch (plan.shape) {
         case 0:
@@ -1076,8 +1087,11 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
         case 2:
           bve_rel_sweep_kernel<128, 6, kBveTile, 2, true><<<grid, 128, 0, job.stream>>>(a, org);
           break;
-        default:
+        case 3:
           bve_rel_sweep_kernel<128, 8, kBveTile, 2, false><<<grid, 128, 0, job.stream>>>(a, org);
+          break;
+        default:
+          bve_rel_sweep_kernel<128, 2, BveRel::kGroup, 6, true><<<grid, 128, 0, job.stream>>>(a, org);
           break;
       }
       finish_bve_kernel<<<fin_grid, pb, 0, job.stream>>>(job.partial, plan.nsplit, job.nt, job.ib, job.x,
@@ -1418,15 +1432,16 @@ int autotune_bve_shape(const SumJob& job, int sm_count, int* shape) {
   cudaEvent_t e0, e1;
   LPM_CUDA_TRY(cudaEventCreate(&e0));
   LPM_CUDA_TRY(cudaEventCreate(&e1));
-  float best_ms = 3.4e38f;
-  int best = 0;
+  // The shapes in turn, several times over, and the best time of each: single runs scatter by a few
+  // percent, and the first ones find the clocks still rising.  Two rounds for a long sum, else four.
+  float ms[kBveShapeCount];
+  for (float& m : ms) m = 3.4e38f;
   int rc = LPM_OK;
-  for (int sh = 0; sh < kBveShapeCount && rc == LPM_OK; ++sh) {
-    const SumPlan p = plan_sum(j.kind, j.mode, j.ns, j.nt, sm_count, sh);
-    rc = launch_sum(j, p);  // warm-up (and sort) run
-    if (rc != LPM_OK) break;
-    float ms = 3.4e38f;
-    for (int again = 0; again < 3 && rc == LPM_OK; ++again) {  // the best of three: single runs scatter by a few percent
+  for (int round = 0, rounds = 2; round < rounds && rc == LPM_OK; ++round) {
+    for (int sh = 0; sh < kBveShapeCount && rc == LPM_OK; ++sh) {
+      // the small sets' shape only where the others' CTAs do not fill the SMs several times
+      if (kBveShapes[sh].tile < kBveTile && ceil_div(j.nt, 512) * ceil_div(j.ns, kBveTile) > 16 * sm_count) continue;
+      const SumPlan p = plan_sum(j.kind, j.mode, j.ns, j.nt, sm_count, sh);
       cudaEventRecord(e0, j.stream);
       rc = launch_sum(j, p);
       cudaEventRecord(e1, j.stream);
@@ -1437,15 +1452,11 @@ int autotune_bve_shape(const SumJob& job, int sm_count, int* shape) {
       }
       float one = 0.f;
       cudaEventElapsedTime(&one, e0, e1);
-      ms = std::min(ms, one);
-      if (one > 5.f) break;  // a long sum's single run is good enough
-    }
-    if (rc != LPM_OK) break;
-    if (ms < best_ms) {
-      best_ms = ms;
-      best = sh;
+      ms[sh] = std::min(ms[sh], one);
+      if (one < 5.f) rounds = 4;
     }
   }
+  const int best = static_cast<int>(std::min_element(ms, ms + kBveShapeCount) - ms);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (rc != LPM_OK) return rc;
