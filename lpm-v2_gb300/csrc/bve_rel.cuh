@@ -70,6 +70,13 @@ struct BveRel {
     float4 e1;  // e1, o.e1
     float4 e2;  // e2, o.e2
   };
+  // A target as floats.  The prep kernel splits the FP64 positions once per sum: every CTA of a target
+  // block needs them, and 20 FP64 instructions a target in each (2 lanes per clock and SM) took 3 % of
+  // a sweep at icosahedral nest 5.
+  struct __align__(16) Tgt {
+    float4 h;  // p_hi, -c_i (BveF32::load_target)
+    float4 l;  // p_lo, 0
+  };
   // sources per origin: 128 measured 4.4 % faster than 64 for the BVE sweep (half the per-group
   // work per source) at the same accuracy; the stream-function sweeps share the layout
   static constexpr int kGroup = 128;
@@ -146,6 +153,31 @@ __device__ __forceinline__ void bve_load_pairs(const BveF32::Params& prm, int64_
     pr[p].yl = make_float2(t0.yl, t1.yl);
     pr[p].zl = make_float2(t0.zl, t1.zl);
     pr[p].nc = make_float2(t0.nc, t1.nc);
+  }
+}
+
+__device__ __forceinline__ BveRel::Tgt bve_split_target(const BveF32::Params& prm, int64_t i) {
+  const BveF32::Tgt t = BveF32::load_target(prm, i);
+  return BveRel::Tgt{make_float4(t.xh, t.yh, t.zh, t.nc), make_float4(t.xl, t.yl, t.zl, 0.f)};
+}
+
+// The same from targets split before (tgt[0] is the first target of the block).
+template <int NP>
+__device__ __forceinline__ void bve_load_pairs(const BveRel::Tgt* __restrict__ tgt, int64_t count,
+                                               BveX2::Pair (&pr)[NP]) {
+#pragma unroll
+  for (int p = 0; p < NP; ++p) {
+    int64_t i0 = bve_target<2 * NP>(2 * p), i1 = bve_target<2 * NP>(2 * p + 1);
+    if (i0 >= count) i0 = count - 1;
+    if (i1 >= count) i1 = count - 1;
+    const BveRel::Tgt t0 = tgt[i0], t1 = tgt[i1];
+    pr[p].xh = make_float2(t0.h.x, t1.h.x);
+    pr[p].yh = make_float2(t0.h.y, t1.h.y);
+    pr[p].zh = make_float2(t0.h.z, t1.h.z);
+    pr[p].xl = make_float2(t0.l.x, t1.l.x);
+    pr[p].yl = make_float2(t0.l.y, t1.l.y);
+    pr[p].zl = make_float2(t0.l.z, t1.l.z);
+    pr[p].nc = make_float2(t0.h.w, t1.h.w);
   }
 }
 
@@ -331,7 +363,8 @@ __device__ __forceinline__ void bve_merge_pairs(const float2 (&ax)[NP], const fl
 
 template <int THREADS, int TPT, int TILE, int MINB, bool DECOUPLED>
 __global__ void __launch_bounds__(THREADS, MINB) bve_rel_sweep_kernel(SweepArgs<BveF32> a,
-                                                                      const BveRel::Group* __restrict__ org) {
+                                                                      const BveRel::Group* __restrict__ org,
+                                                                      const BveRel::Tgt* __restrict__ tgt) {
   static_assert(TPT % 2 == 0, "targets come in pairs");
   static_assert(TILE % BveRel::kGroup == 0, "whole origin groups per tile");
   constexpr int NP = TPT / 2;
@@ -346,7 +379,7 @@ __global__ void __launch_bounds__(THREADS, MINB) bve_rel_sweep_kernel(SweepArgs<
   float2 hx[NP], hy[NP], hz[NP], lx[NP], ly[NP], lz[NP];
   const int64_t first = static_cast<int64_t>(blockIdx.x) * (THREADS * TPT);
   const int64_t count = a.nt - first < THREADS * TPT ? a.nt - first : THREADS * TPT;
-  bve_load_pairs<NP>(a.p, a.ib + first, count, pr);
+  bve_load_pairs<NP>(tgt + first, count, pr);
 #pragma unroll
   for (int p = 0; p < NP; ++p) hx[p] = hy[p] = hz[p] = lx[p] = ly[p] = lz[p] = make_float2(0.f, 0.f);
 
@@ -649,13 +682,19 @@ __device__ __forceinline__ void bve_rel_prep_tile(const double* x, const double*
 }
 
 // Tile-relative records of the Hilbert-sorted source list `sorted` (ns entries, records
-// ns..npad-1 inert) and the group origins: one CTA of TILE threads per tile.
+// ns..npad-1 inert) and the groups (CTA t < n_tiles: tile t, TILE threads), then the nt targets from ib on.
 template <int TILE>
 __global__ void __launch_bounds__(TILE) bve_rel_prep_kernel(const double* x, const double* y, const double* z,
                                                             const double* zeta, const double* area,
-                                                            const int32_t* sorted, int64_t ns, double inv_a,
-                                                            double s_scale, BveRel::Rec* out, BveRel::Group* org) {
+                                                            const int32_t* sorted, int64_t ns, int64_t n_tiles,
+                                                            double inv_a, double s_scale, int64_t ib, int64_t nt,
+                                                            BveRel::Rec* out, BveRel::Group* org, BveRel::Tgt* tgt) {
   const int64_t t = blockIdx.x;
+  if (t >= n_tiles) {
+    const int64_t il = (t - n_tiles) * TILE + threadIdx.x;
+    if (il < nt) tgt[il] = bve_split_target(BveF32::Params{x, y, z, inv_a}, ib + il);
+    return;
+  }
   const int64_t k = t * TILE + threadIdx.x;
   const bool valid = k < ns;
   const int32_t j = valid ? sorted[k] : 0;

@@ -80,9 +80,8 @@ struct EnsArgs {
   int* head;
   const BveRel::Rec* src;
   const BveRel::Group* org;
-  const double *x, *y, *z;
-  const double* inv_a;  // per instance
-  double* partial;      // [slot][3][targets per item]
+  const BveRel::Tgt* tgt;
+  double* partial;  // [slot][3][targets per item]
   int* status;
 };
 
@@ -104,10 +103,9 @@ __global__ void __launch_bounds__(THREADS, MINB) ensemble_sweep_kernel(EnsArgs a
     __syncthreads();
     if (q >= a.n_items) break;
     const Item it = a.items[a.queue[q]];
-    const BveF32::Params prm{a.x, a.y, a.z, a.inv_a[it.inst]};
     BveX2::Pair pr[NP];
     float2 hx[NP], hy[NP], hz[NP], lx[NP], ly[NP], lz[NP];
-    bve_load_pairs<NP>(prm, it.t0, it.nt, pr);
+    bve_load_pairs<NP>(a.tgt + it.t0, it.nt, pr);
 #pragma unroll
     for (int p = 0; p < NP; ++p) hx[p] = hy[p] = hz[p] = lx[p] = ly[p] = lz[p] = make_float2(0.f, 0.f);
     int64_t tile = it.tile0;
@@ -139,14 +137,22 @@ __global__ void __launch_bounds__(THREADS, MINB) ensemble_sweep_kernel(EnsArgs a
 
 // Group-relative records of all instances: one CTA per (global) tile.  Tile t belongs to
 // instance tile_inst[t]; its sources are that instance's Hilbert-sorted sources
-// sorted[src_start[k] + (t - tile_off[k]) * kTile + lane], valid below ns_k.
+// sorted[src_start[k] + (t - tile_off[k]) * kTile + lane], valid below ns_k.  The CTAs after the
+// n_tiles tiles split the n particles into float targets.
 __global__ void __launch_bounds__(kTile) ensemble_prep_kernel(const int32_t* tile_inst, const int64_t* tile_off,
                                                               const int64_t* src_start, const int64_t* ns_k,
                                                               const int32_t* sorted, const double* x, const double* y,
                                                               const double* z, const double* zeta, const double* area,
-                                                              const double* radius, BveRel::Rec* out,
-                                                              BveRel::Group* org) {
+                                                              const double* radius, int64_t n_tiles, int64_t n,
+                                                              const int32_t* pinst, const double* inv_a,
+                                                              BveRel::Rec* out, BveRel::Group* org,
+                                                              BveRel::Tgt* tgt) {
   const int64_t t = blockIdx.x;
+  if (t >= n_tiles) {
+    const int64_t i = (t - n_tiles) * kTile + threadIdx.x;
+    if (i < n) tgt[i] = bve_split_target(BveF32::Params{x, y, z, inv_a[pinst[i]]}, i);
+    return;
+  }
   const int k = tile_inst[t];
   const int64_t local = (t - tile_off[k]) * kTile + threadIdx.x;
   const bool valid = local < ns_k[k];
@@ -275,6 +281,7 @@ struct lpm_ensemble {
   int64_t *d_tile_off = nullptr, *d_src_start = nullptr, *d_ns_k = nullptr;
   BveRel::Rec* rec = nullptr;
   BveRel::Group* org = nullptr;
+  BveRel::Tgt* tgt = nullptr;
   Item* items = nullptr;
   int* queue = nullptr;
   int n_items = 0;
@@ -338,11 +345,12 @@ struct lpm_ensemble {
     if (n_tiles > 0) {
       LPM_TRY(grouped_curve_sort(stream, ns_total, K, act_idx, act_grp, px, py, pz, inv_a, sort_scratch, sort_bytes,
                                   sorted));
-      ensemble_prep_kernel<<<static_cast<unsigned>(n_tiles), kTile, 0, stream>>>(
-          tile_inst, d_tile_off, d_src_start, d_ns_k, sorted, px, py, pz, pq, area, radius, rec, org);
     }
+    ensemble_prep_kernel<<<static_cast<unsigned>(n_tiles + ceil_div(n, kTile)), kTile, 0, stream>>>(
+        tile_inst, d_tile_off, d_src_start, d_ns_k, sorted, px, py, pz, pq, area, radius, n_tiles, n, pinst, inv_a, rec,
+        org, tgt);
     LPM_CUDA_TRY(cudaMemsetAsync(head, 0, sizeof(int), stream));
-    EnsArgs a{items, queue, n_items, head, rec, org, px, py, pz, inv_a, partial, status};
+    EnsArgs a{items, queue, n_items, head, rec, org, tgt, partial, status};
     if (shape == 0) {
       ensemble_sweep_kernel<128, 4, 4><<<grid, 128, 0, stream>>>(a);
     } else {
@@ -544,6 +552,7 @@ struct lpm_ensemble {
     LPM_TRY(arena.alloc(sort_bytes, &sort_scratch));
     LPM_TRY(dev_array(&rec, std::max<int64_t>(n_tiles * kTile, 1)));
     LPM_TRY(dev_array(&org, std::max<int64_t>(n_tiles * (kTile / BveRel::kGroup), 1)));
+    LPM_TRY(dev_array(&tgt, std::max<int64_t>(n, 1)));
     LPM_TRY(dev_array(&items, n_it));
     LPM_TRY(dev_array(&queue, n_it));
     LPM_TRY(dev_array(&blk_off, static_cast<size_t>(K) + 1));

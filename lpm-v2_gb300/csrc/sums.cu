@@ -552,7 +552,8 @@ SumPlan plan_sum(int kind, int mode, int64_t ns, int64_t nt, int sm_count, int s
     pl.tperm_offset = align_up(pl.src_bytes, 256);
     pl.src_bytes = pl.tperm_offset + 2 * align_up(static_cast<size_t>(nt) * sizeof(int32_t), 256);
   }
-  if (mode == LPM_MODE_FP32C && pse_lap_kind(kind)) {
+  if (mode == LPM_MODE_FP32C && (pse_lap_kind(kind) || kind == kSumBve || kind == kSumBveMesh)) {
+    static_assert(sizeof(PseLap::Tgt) == sizeof(BveRel::Tgt), "one size of a split target");
     pl.tgt_offset = align_up(pl.src_bytes, 256);
     pl.src_bytes = pl.tgt_offset + static_cast<size_t>(nt) * sizeof(PseLap::Tgt);
   }
@@ -1061,9 +1062,11 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
       BveRel::Rec* recs = static_cast<BveRel::Rec*>(job.src_buf);
       BveRel::Group* org = reinterpret_cast<BveRel::Group*>(
           static_cast<char*>(job.src_buf) + align_up(static_cast<size_t>(npad) * sizeof(BveRel::Rec), 256));
-      bve_rel_prep_kernel<kBveTile><<<static_cast<unsigned>(plan.n_tiles), kBveTile, 0, job.stream>>>(
-          job.x, job.y, job.z, job.s1, job.area, src_list, job.ns, inv_a, -1.0 / (2.0 * kPi * job.radius), recs,
-          org);
+      BveRel::Tgt* tgt = reinterpret_cast<BveRel::Tgt*>(static_cast<char*>(job.src_buf) + plan.tgt_offset);
+      const unsigned prep = static_cast<unsigned>(plan.n_tiles + ceil_div(job.nt, kBveTile));
+      bve_rel_prep_kernel<kBveTile><<<prep, kBveTile, 0, job.stream>>>(
+          job.x, job.y, job.z, job.s1, job.area, src_list, job.ns, plan.n_tiles, inv_a,
+          -1.0 / (2.0 * kPi * job.radius), job.ib, job.nt, recs, org, tgt);
       SweepArgs<BveF32> a;
       a.p = BveF32::Params{job.x, job.y, job.z, inv_a};
       a.src = reinterpret_cast<const BveF32::Rec*>(job.src_buf);
@@ -1079,19 +1082,19 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
       const dim3 grid(static_cast<unsigned>(ceil_div(job.nt, sh.threads * sh.tpt)), static_cast<unsigned>(plan.nsplit));
       switch (plan.shape) {
         case 0:
-          bve_rel_sweep_kernel<128, 4, kBveTile, 4, true><<<grid, 128, 0, job.stream>>>(a, org);
+          bve_rel_sweep_kernel<128, 4, kBveTile, 4, true><<<grid, 128, 0, job.stream>>>(a, org, tgt);
           break;
         case 1:
-          bve_rel_sweep_kernel<128, 4, kBveTile, 4, false><<<grid, 128, 0, job.stream>>>(a, org);
+          bve_rel_sweep_kernel<128, 4, kBveTile, 4, false><<<grid, 128, 0, job.stream>>>(a, org, tgt);
           break;
         case 2:
-          bve_rel_sweep_kernel<128, 6, kBveTile, 2, true><<<grid, 128, 0, job.stream>>>(a, org);
+          bve_rel_sweep_kernel<128, 6, kBveTile, 2, true><<<grid, 128, 0, job.stream>>>(a, org, tgt);
           break;
         case 3:
-          bve_rel_sweep_kernel<128, 8, kBveTile, 2, false><<<grid, 128, 0, job.stream>>>(a, org);
+          bve_rel_sweep_kernel<128, 8, kBveTile, 2, false><<<grid, 128, 0, job.stream>>>(a, org, tgt);
           break;
         default:
-          bve_rel_sweep_kernel<128, 2, BveRel::kGroup, 6, true><<<grid, 128, 0, job.stream>>>(a, org);
+          bve_rel_sweep_kernel<128, 2, BveRel::kGroup, 6, true><<<grid, 128, 0, job.stream>>>(a, org, tgt);
           break;
       }
       finish_bve_kernel<<<fin_grid, pb, 0, job.stream>>>(job.partial, plan.nsplit, job.nt, job.ib, job.x,

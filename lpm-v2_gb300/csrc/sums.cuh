@@ -25,7 +25,7 @@ struct SumPlan {
   // FP32C PSE sums: the targets' curve order (two lists of nt int32: [ib, ib + nt) and its
   // sorted permutation) at src_buf + tperm_offset; 0 when the sweep takes targets in order
   size_t tperm_offset = 0;
-  size_t tgt_offset = 0;  // FP32C Laplacians: the targets as floats (PseLap::Tgt) at src_buf + tgt_offset
+  size_t tgt_offset = 0;  // FP32C Laplacians and BVE: the targets as floats at src_buf + tgt_offset
 };
 
 enum SumKind : int {
