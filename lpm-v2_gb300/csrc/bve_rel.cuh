@@ -448,7 +448,8 @@ struct GroupFrame {
 };
 
 template <int TILE, int G>
-__device__ __forceinline__ GroupFrame sphere_group_frame(bool valid, const SplitPoint& sp, double cj) {
+__device__ __forceinline__ GroupFrame sphere_group_frame(bool valid, const SplitPoint& sp, double cj,
+                                                         float compact_radius = BveRel::kCompactRadius) {
   static_assert(G % 32 == 0 && TILE % G == 0, "whole warps per group");
   constexpr int NW = TILE / 32, WPG = G / 32;
   __shared__ float part[NW][4];
@@ -520,7 +521,7 @@ __device__ __forceinline__ GroupFrame sphere_group_frame(bool valid, const Split
     }
   }
   f.radius = sqrtf(rad) * 1.000001f;
-  f.compact = f.radius <= BveRel::kCompactRadius && f.radius <= BveRel::kCompactRatio * sqrtf(spc);
+  f.compact = f.radius <= compact_radius && f.radius <= BveRel::kCompactRatio * sqrtf(spc);
   // on the sphere: dropping every c_j moves q by <= 2^-30 h^2 relative to the smallest |d|^2
   f.on_sphere = cm <= 9.313225746154785e-10f * spc;
   return f;
@@ -612,6 +613,17 @@ __device__ __forceinline__ GroupBasis group_basis(const GroupFrame& f) {
   return b;
 }
 
+// A source's coordinates in its group's basis, s_j = a e1 + b e2 + c o for its offset (hi, lo): the
+// projections less their first-order coupling (2^-24 of them; the second order is 2^-48).
+__device__ __forceinline__ void basis_coords(const GroupBasis& b, const GroupFrame& f, const float (&hi)[3],
+                                             const float (&lo)[3], float& af, float& bf, float& cf) {
+  const float2 a0 = dot_pair(hi, lo, b.e1, 0.f), b0 = dot_pair(hi, lo, b.e2, 0.f), so = dot_pair(hi, lo, f.o, 0.f);
+  const float c0 = so.x * b.inv_o2;
+  af = a0.x + (a0.y - (a0.x * b.g11 + b0.x * b.g12 + c0 * b.k1));
+  bf = b0.x + (b0.y - (a0.x * b.g12 + b0.x * b.g22 + c0 * b.k2));
+  cf = (so.x + (so.y - (af * b.k1 + bf * b.k2))) * b.inv_o2;
+}
+
 // Records and groups of one tile of TILE sources (one CTA of TILE threads; every thread
 // one record).  `j` is the thread's particle (meaningful only if `valid`), `inv_a` and
 // `s_scale` the tile's sphere scale.  Every record is written as the offset of p_j from its
@@ -638,13 +650,8 @@ __device__ __forceinline__ void bve_rel_prep_tile(const double* x, const double*
     const float nc = __double2float_rn(-cj);
     float s, sl;
     split2(zeta[j] * area[j] * s_scale, s, sl);
-    // s_j = a e1 + b e2 + c o: the projections less their first-order coupling (2^-24 of them;
-    // the second order is 2^-48)
-    const float2 a0 = dot_pair(hi, lo, b.e1, 0.f), b0 = dot_pair(hi, lo, b.e2, 0.f), so = dot_pair(hi, lo, f.o, 0.f);
-    const float c0 = so.x * b.inv_o2;
-    const float af = a0.x + (a0.y - (a0.x * b.g11 + b0.x * b.g12 + c0 * b.k1));
-    const float bf = b0.x + (b0.y - (a0.x * b.g12 + b0.x * b.g22 + c0 * b.k2));
-    const float cf = (so.x + (so.y - (af * b.k1 + bf * b.k2))) * b.inv_o2;
+    float af, bf, cf;
+    basis_coords(b, f, hi, lo, af, bf, cf);
     // the strength times 1 + c, a and b, each rounded once
     auto times = [&](float v) {
       const float p = s * v;

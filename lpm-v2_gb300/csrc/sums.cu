@@ -55,6 +55,7 @@ constexpr int kPseThreads = 128, kPseTpt = 4, kPseTile = 256, kPseMinB = 4, kPse
 constexpr int kPseDivTile = 128, kPseDivStages = 4;
 constexpr int kLapMinB = 4;
 constexpr int kStreamThreads = 128, kStreamTpt = 4, kStreamTile = 256, kStreamMinB = 4;
+constexpr int kSphereStreamTpt = 6, kSphereStreamMinB = 3;
 constexpr int kBetaThreads = 128, kBetaTpt = 4, kBetaTile = 256, kBetaMinB = 4;
 constexpr int kSweMinB = 3;        // planar SWE velocity sweep: 128 x 4 targets, 3 CTAs per SM
 constexpr int kSweSphereMinB = 2;  // sphere SWE velocity sweep: 2 CTAs per SM (no spills; 10 % over 3)
@@ -353,9 +354,10 @@ int origin_group(int kind) {
   switch (kind) {
     case kSumBve:
     case kSumBveMesh:
-    case kSumSphereStream:
     case kSumSweSphere:
       return BveRel::kGroup;
+    case kSumSphereStream:
+      return StreamFn::kGroup;
     case kSumPseK8Geo:
     case kSumPseGaussChord:
     case kSumPseGrad:
@@ -390,6 +392,7 @@ size_t rec_bytes(int kind, int mode) {
     case kSumPlane:
       return sizeof(PlaneRel::Rec);
     case kSumSphereStream:
+      return sizeof(StreamFn::Rec);
     case kSumSweSphere:
       return sizeof(StreamRel::Rec);
     case kSumPlaneStream:
@@ -442,6 +445,7 @@ int targets_per_cta(int kind, int shape) {
     case kSumPlane:
       return kPlaneThreads * kPlaneTpt;
     case kSumSphereStream:
+      return kStreamThreads * kSphereStreamTpt;
     case kSumPlaneStream:
     case kSumSweSphere:
       return kStreamThreads * kStreamTpt;
@@ -542,7 +546,9 @@ SumPlan plan_sum(int kind, int mode, int64_t ns, int64_t nt, int sm_count, int s
                   "one origin layout size");
     pl.src_bytes = align_up(pl.src_bytes, 256) +
                    static_cast<size_t>(pl.n_tiles) * (tile / origin_group(kind)) *
-                       (kind == kSumBve || kind == kSumBveMesh ? sizeof(BveRel::Group) : sizeof(BveRel::Origin));
+                       (kind == kSumBve || kind == kSumBveMesh ? sizeof(BveRel::Group)
+                        : kind == kSumSphereStream             ? sizeof(StreamFn::Group)
+                                                               : sizeof(BveRel::Origin));
   }
   if (mode == LPM_MODE_FP32C && pse_culls_tiles(kind)) {
     // the tiles' balls follow the group origins
@@ -552,13 +558,13 @@ SumPlan plan_sum(int kind, int mode, int64_t ns, int64_t nt, int sm_count, int s
     pl.tperm_offset = align_up(pl.src_bytes, 256);
     pl.src_bytes = pl.tperm_offset + 2 * align_up(static_cast<size_t>(nt) * sizeof(int32_t), 256);
   }
-  if (mode == LPM_MODE_FP32C && (pse_lap_kind(kind) || kind == kSumBve || kind == kSumBveMesh)) {
+  if (mode == LPM_MODE_FP32C && (pse_lap_kind(kind) || kind == kSumBve || kind == kSumBveMesh || kind == kSumSphereStream)) {
     static_assert(sizeof(PseLap::Tgt) == sizeof(BveRel::Tgt), "one size of a split target");
     pl.tgt_offset = align_up(pl.src_bytes, 256);
     pl.src_bytes = pl.tgt_offset + static_cast<size_t>(nt) * sizeof(PseLap::Tgt);
   }
   if (mode == LPM_MODE_FP32C && kind == kSumSphereStream) {
-    // the sources' own zeta A (2 x nt) and the two totals follow the group origins
+    // the sources' own zeta A (2 x nt) and the two totals follow the targets
     pl.src_bytes = align_up(pl.src_bytes, 256) + align_up(2 * static_cast<size_t>(nt) * sizeof(double), 256) +
                    2 * sizeof(double);
   }
@@ -586,6 +592,7 @@ SumPlan plan_sum(int kind, int mode, int64_t ns, int64_t nt, int sm_count, int s
   const int minb = (kind == kSumBve || kind == kSumBveMesh)          ? kBveShapes[shape].minb
                    : kind == kSumSwePlane                            ? kSweMinB
                    : kind == kSumSweSphere                           ? kSweSphereMinB
+                   : kind == kSumSphereStream                        ? kSphereStreamMinB
                                                                      : 4;
   const int64_t slots = static_cast<int64_t>(sm_count > 0 ? sm_count : 152) * minb;
   if (mode == LPM_MODE_FP32C && pse_culls_tiles(kind)) {
@@ -1161,19 +1168,21 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
                            job.sort_bytes, job.sorted));
         src_list = job.sorted;
       }
-      // layout of src_buf: records, group origins, the sources' own zeta A (2 x nt), totals
+      // layout of src_buf: records, groups, split targets, the sources' own zeta A (2 x nt), totals
       char* base = static_cast<char*>(job.src_buf);
-      StreamRel::Rec* recs = reinterpret_cast<StreamRel::Rec*>(base);
-      const size_t org_off = align_up(static_cast<size_t>(npad) * sizeof(StreamRel::Rec), 256);
-      BveRel::Origin* org = reinterpret_cast<BveRel::Origin*>(base + org_off);
-      const size_t self_off = align_up(
-          org_off + static_cast<size_t>(plan.n_tiles) * (kStreamTile / BveRel::kGroup) * sizeof(BveRel::Origin), 256);
+      StreamFn::Rec* recs = reinterpret_cast<StreamFn::Rec*>(base);
+      StreamFn::Group* org = reinterpret_cast<StreamFn::Group*>(
+          base + align_up(static_cast<size_t>(npad) * sizeof(StreamFn::Rec), 256));
+      BveRel::Tgt* tgt = reinterpret_cast<BveRel::Tgt*>(base + plan.tgt_offset);
+      const size_t self_off = align_up(plan.tgt_offset + static_cast<size_t>(job.nt) * sizeof(BveRel::Tgt), 256);
       double* self_w = reinterpret_cast<double*>(base + self_off);
       double* tot =
           reinterpret_cast<double*>(base + self_off + align_up(2 * static_cast<size_t>(job.nt) * sizeof(double), 256));
       LPM_CUDA_TRY(cudaMemsetAsync(self_w, 0, 2 * static_cast<size_t>(job.nt) * sizeof(double), job.stream));
-      stream_rel_prep_kernel<kStreamTile><<<static_cast<unsigned>(plan.n_tiles), kStreamTile, 0, job.stream>>>(
-          job.x, job.y, job.z, job.s1, job.s2, job.area, src_list, job.ns, inv_a, job.ib, job.nt, recs, org, self_w);
+      const unsigned prep = static_cast<unsigned>(plan.n_tiles + ceil_div(job.nt, kStreamTile));
+      stream_prep_kernel<kStreamTile><<<prep, kStreamTile, 0, job.stream>>>(
+          job.x, job.y, job.z, job.s1, job.s2, job.area, src_list, job.ns, plan.n_tiles, inv_a, job.ib, job.nt, recs,
+          org, tgt, self_w);
       stream_totals_kernel<<<1, 1024, 0, job.stream>>>(job.s1, job.s2, job.area, job.src_idx, job.ns, tot);
       SweepArgs<BveF32> a;
       a.p = BveF32::Params{job.x, job.y, job.z, inv_a};
@@ -1184,10 +1193,10 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
       a.nt = job.nt;
       a.partial = job.partial;
       a.status = job.status;
-      const dim3 grid(static_cast<unsigned>(ceil_div(job.nt, kStreamThreads * kStreamTpt)),
+      const dim3 grid(static_cast<unsigned>(ceil_div(job.nt, kStreamThreads * kSphereStreamTpt)),
                       static_cast<unsigned>(plan.nsplit));
-      stream_rel_sweep_kernel<kStreamThreads, kStreamTpt, kStreamTile, kStreamMinB>
-          <<<grid, kStreamThreads, 0, job.stream>>>(a, recs, org);
+      stream_rel_sweep_kernel<kStreamThreads, kSphereStreamTpt, kStreamTile, kSphereStreamMinB>
+          <<<grid, kStreamThreads, 0, job.stream>>>(a, recs, org, tgt);
       // a^2 - x_i.x_j = (a^2 / 2) q_ij: the constant term is -ln(a^2 / 2) / (4 pi) per zeta A
       const double k_const = -std::log(0.5 * job.radius * job.radius) * kInv4Pi;
       finish_stream_kernel<<<fin_grid, pb, 0, job.stream>>>(job.partial, plan.nsplit, job.nt, 2, k_const, tot, self_w,
@@ -1270,8 +1279,7 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
           static_cast<char*>(job.src_buf) + align_up(static_cast<size_t>(npad) * sizeof(StreamRel::Rec), 256));
       const double k2 = 1.0 / (2.0 * kPi * job.radius * job.radius);
       stream_rel_prep_kernel<kStreamTile><<<static_cast<unsigned>(plan.n_tiles), kStreamTile, 0, job.stream>>>(
-          job.x, job.y, job.z, job.s1, job.s2, job.area, src_list, job.ns, inv_a, job.ib, job.nt, recs, org, nullptr,
-          -k2, k2);
+          job.x, job.y, job.z, job.s1, job.s2, job.area, src_list, job.ns, inv_a, recs, org, -k2, k2);
       SweepArgs<BveF32> a;
       a.p = BveF32::Params{job.x, job.y, job.z, inv_a};
       a.n_tiles = plan.n_tiles;
