@@ -605,7 +605,7 @@ __global__ void __launch_bounds__(TILE) stream_rel_prep_kernel(const double* x, 
 // |d|^2 (2), ln (ln_q2_shift: integer split, a table load per lane, 9 packed) and the
 // accumulation (1 FFMA2).  Near partials are flushed every 16 sources, far ones per group.
 template <int THREADS, int TPT, int TILE, int MINB>
-__global__ void __launch_bounds__(THREADS, MINB) plane_stream_rel_sweep_kernel(PlaneRelArgs a) {
+__global__ void __launch_bounds__(THREADS, MINB) plane_stream_rel_sweep_kernel(PlaneRelArgs<PlaneRel::Rec> a) {
   static_assert(TPT % 2 == 0, "targets come in pairs");
   constexpr int NP = TPT / 2;
   constexpr int G = PlaneRel::kGroup;
@@ -613,8 +613,7 @@ __global__ void __launch_bounds__(THREADS, MINB) plane_stream_rel_sweep_kernel(P
   constexpr int FLN = 16;
   static_assert(G % FLN == 0, "flush interval must divide the group");
   using Rec = PlaneRel::Rec;
-  __shared__ __align__(128) Rec stage[2][TILE];
-  __shared__ __align__(8) uint64_t bars[2];
+  __shared__ TilePipe<Rec, TILE, 2, PlaneRel::Origin, GPT> pipe;
   __shared__ __align__(8) float2 ln_tab[32];
 
   const int64_t chunk = blockIdx.y;
@@ -624,31 +623,16 @@ __global__ void __launch_bounds__(THREADS, MINB) plane_stream_rel_sweep_kernel(P
   float2 hs[NP], ls[NP], hk[NP], lk[NP];
   const int64_t first = static_cast<int64_t>(blockIdx.x) * (THREADS * TPT);
   const int64_t count = a.nt - first < THREADS * TPT ? a.nt - first : THREADS * TPT;
+  plane_load_pairs<NP>(a.tgt + first, count, pr);
 #pragma unroll
-  for (int p = 0; p < NP; ++p) {
-    int64_t i0 = (2 * p) * THREADS + threadIdx.x, i1 = (2 * p + 1) * THREADS + threadIdx.x;
-    if (i0 >= count) i0 = count - 1;  // duplicates of a valid target; results not stored
-    if (i1 >= count) i1 = count - 1;
-    float h0, l0, h1, l1;
-    split2(a.x[a.ib + first + i0], h0, l0);
-    split2(a.x[a.ib + first + i1], h1, l1);
-    pr[p].xh = make_float2(h0, h1);
-    pr[p].xl = make_float2(l0, l1);
-    split2(a.y[a.ib + first + i0], h0, l0);
-    split2(a.y[a.ib + first + i1], h1, l1);
-    pr[p].yh = make_float2(h0, h1);
-    pr[p].yl = make_float2(l0, l1);
-    hs[p] = ls[p] = hk[p] = lk[p] = make_float2(0.f, 0.f);
-  }
+  for (int p = 0; p < NP; ++p) hs[p] = ls[p] = hk[p] = lk[p] = make_float2(0.f, 0.f);
   constexpr float kTiny = 7.888609052210118e-31f;  // 2^-100: centring and near floor
   constexpr float kHuge = 1.2676506002282294e30f;  // 2^100
 
   ln_tab_load(ln_tab);
-  pipe_init(bars);
+  tile_pipe_init(pipe);
   uint32_t g = 0;
-  int64_t tile = ct.first;
-  staged_sweep<Rec, TILE>(a.src, ct.first, ct.count, stage[0], stage[1], bars, g, a.status, [&](const Rec* tl) {
-    const PlaneRel::Origin* og = a.org + tile * GPT;
+  auto body = [&](const Rec* tl, const PlaneRel::Origin* og) {
 #pragma unroll 1
     for (int g0 = 0; g0 < TILE; g0 += G) {
       const PlaneRel::Origin o = og[g0 / G];
@@ -731,15 +715,16 @@ __global__ void __launch_bounds__(THREADS, MINB) plane_stream_rel_sweep_kernel(P
         }
       }
     }
-    tile += ct.step;
-  }, ct.step);
+  };
+  warp_sweep_tiles(a.src, [ct](int64_t t) { return ct.first + t * ct.step; }, ct.count, pipe, g, a.status,
+                   default_wait(), a.org, body);
 
   constexpr double kLn2 = 0.69314718055994530942;
 #pragma unroll
   for (int p = 0; p < NP; ++p) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const int64_t il = first + (2 * p + h) * THREADS + threadIdx.x;
+      const int64_t il = first + bve_target<TPT>(2 * p + h);
       if (il < a.nt) {
         const double c = static_cast<double>(h ? hk[p].y : hk[p].x) + static_cast<double>(h ? lk[p].y : lk[p].x);
         a.partial[chunk * a.nt + il] =

@@ -57,7 +57,7 @@ constexpr int kLapMinB = 4;
 constexpr int kStreamThreads = 128, kStreamTpt = 4, kStreamTile = 256, kStreamMinB = 4;
 constexpr int kSphereStreamTpt = 6, kSphereStreamMinB = 3;
 constexpr int kBetaThreads = 128, kBetaTpt = 4, kBetaTile = 256, kBetaMinB = 4;
-constexpr int kSweMinB = 3;        // planar SWE velocity sweep: 128 x 4 targets, 3 CTAs per SM
+constexpr int kSweTpt = 4, kSweMinB = 4;  // planar SWE velocity sweep
 constexpr int kSweSphereMinB = 2;  // sphere SWE velocity sweep: 2 CTAs per SM (no spills; 10 % over 3)
 // FP64 sequential sweep shape
 // (64-source tiles for the PSE sums' cutoff; the sweeps without one run at the same rate at 128)
@@ -244,18 +244,18 @@ __global__ void finish_plane_kernel(const double* partial, int64_t nsplit, int64
   v[il] = sv;
 }
 
-// u, v and the double dot product ux ux + 2 uy vx + vy vy of the SWE velocity sweep's six
-// partials [chunk][6][nt] (SWEPlaneSolver.f90:530)
+// u, v and the double dot product ux ux + 2 uy vx + vy vy (SWEPlaneSolver.f90:530) of the SWE
+// velocity sweep's partials [chunk][4][nt]: u, v, -ux, -vx, with uy = vx and vy = -ux
 __global__ void swe_finish_kernel(const double* partial, int64_t nsplit, int64_t nt, double* u, double* v,
                                   double* ddot) {
   const int64_t il = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (il >= nt) return;
-  double s[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
   for (int64_t k = 0; k < nsplit; ++k)
-    for (int c = 0; c < 6; ++c) s[c] += partial[(k * 6 + c) * nt + il];
+    for (int c = 0; c < 4; ++c) s[c] += partial[(k * 4 + c) * nt + il];
   u[il] = s[0];
   v[il] = s[1];
-  ddot[il] = (s[2] * s[2] + (2.0 * s[3]) * s[4]) + s[5] * s[5];
+  ddot[il] = 2.0 * (s[2] * s[2] + s[3] * s[3]);
 }
 
 // The sphere SWE velocity from the seven partials [chunk][7][nt] (Dr, Dp, W):
@@ -402,7 +402,7 @@ size_t rec_bytes(int kind, int mode) {
     case kSumBetaStream:
       return sizeof(BetaStreamRel::Rec);
     case kSumSwePlane:
-      return sizeof(PlaneRel::Rec);
+      return sizeof(PlaneSwe::Rec);
     case kSumPseK8Geo:
     case kSumPseGaussChord:
     case kSumPseGrad:
@@ -429,7 +429,7 @@ int comps_of(int kind) {
     case kSumPseGrad:
       return 3;
     case kSumSwePlane:
-      return 6;
+      return 4;
     case kSumSweSphere:
       return 7;
     default:
@@ -444,6 +444,8 @@ int targets_per_cta(int kind, int shape) {
       return kBveShapes[shape].threads * kBveShapes[shape].tpt;
     case kSumPlane:
       return kPlaneThreads * kPlaneTpt;
+    case kSumSwePlane:
+      return kPlaneThreads * kSweTpt;
     case kSumSphereStream:
       return kStreamThreads * kSphereStreamTpt;
     case kSumPlaneStream:
@@ -558,7 +560,10 @@ SumPlan plan_sum(int kind, int mode, int64_t ns, int64_t nt, int sm_count, int s
     pl.tperm_offset = align_up(pl.src_bytes, 256);
     pl.src_bytes = pl.tperm_offset + 2 * align_up(static_cast<size_t>(nt) * sizeof(int32_t), 256);
   }
-  if (mode == LPM_MODE_FP32C && (pse_lap_kind(kind) || kind == kSumBve || kind == kSumBveMesh || kind == kSumSphereStream)) {
+  // the targets as floats, 32 bytes each (16 in the plane)
+  const bool split_targets = pse_lap_kind(kind) || kind == kSumBve || kind == kSumBveMesh || kind == kSumSphereStream ||
+                             kind == kSumPlane || kind == kSumPlaneStream || kind == kSumSwePlane;
+  if (mode == LPM_MODE_FP32C && split_targets) {
     static_assert(sizeof(PseLap::Tgt) == sizeof(BveRel::Tgt), "one size of a split target");
     pl.tgt_offset = align_up(pl.src_bytes, 256);
     pl.src_bytes = pl.tgt_offset + static_cast<size_t>(nt) * sizeof(PseLap::Tgt);
@@ -1118,17 +1123,17 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
       PlaneRel::Rec* recs = static_cast<PlaneRel::Rec*>(job.src_buf);
       PlaneRel::Origin* org = reinterpret_cast<PlaneRel::Origin*>(
           static_cast<char*>(job.src_buf) + align_up(static_cast<size_t>(npad) * sizeof(PlaneRel::Rec), 256));
-      plane_rel_prep_kernel<kPlaneTile><<<static_cast<unsigned>(plan.n_tiles), kPlaneTile, 0, job.stream>>>(
-          job.x, job.y, job.s1, job.area, src_list, job.ns, 1.0 / (2.0 * kPi), recs, org);
-      PlaneRelArgs a;
-      a.x = job.x;
-      a.y = job.y;
+      PlaneRel::Tgt* tgt = reinterpret_cast<PlaneRel::Tgt*>(static_cast<char*>(job.src_buf) + plan.tgt_offset);
+      const unsigned prep = static_cast<unsigned>(plan.n_tiles + ceil_div(job.nt, kPlaneTile));
+      plane_rel_prep_kernel<kPlaneTile><<<prep, kPlaneTile, 0, job.stream>>>(
+          job.x, job.y, job.s1, job.area, src_list, job.ns, plan.n_tiles, 1.0 / (2.0 * kPi), job.ib, job.nt, recs, org,
+          tgt);
+      PlaneRelArgs<PlaneRel::Rec> a;
       a.d2 = static_cast<float>(job.delta * job.delta) + 7.888609052210118e-31f;  // + 2^-100
       a.src = recs;
       a.org = org;
+      a.tgt = tgt;
       a.n_tiles = plan.n_tiles;
-      a.tiles_per_chunk = plan.tiles_per_chunk;
-      a.ib = job.ib;
       a.nt = job.nt;
       a.partial = job.partial;
       a.status = job.status;
@@ -1213,17 +1218,16 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
       PlaneRel::Rec* recs = static_cast<PlaneRel::Rec*>(job.src_buf);
       PlaneRel::Origin* org = reinterpret_cast<PlaneRel::Origin*>(
           static_cast<char*>(job.src_buf) + align_up(static_cast<size_t>(npad) * sizeof(PlaneRel::Rec), 256));
-      plane_rel_prep_kernel<kStreamTile><<<static_cast<unsigned>(plan.n_tiles), kStreamTile, 0, job.stream>>>(
-          job.x, job.y, job.s1, job.area, src_list, job.ns, kInv4Pi, recs, org);
-      PlaneRelArgs a;
-      a.x = job.x;
-      a.y = job.y;
+      PlaneRel::Tgt* tgt = reinterpret_cast<PlaneRel::Tgt*>(static_cast<char*>(job.src_buf) + plan.tgt_offset);
+      const unsigned prep = static_cast<unsigned>(plan.n_tiles + ceil_div(job.nt, kStreamTile));
+      plane_rel_prep_kernel<kStreamTile><<<prep, kStreamTile, 0, job.stream>>>(
+          job.x, job.y, job.s1, job.area, src_list, job.ns, plan.n_tiles, kInv4Pi, job.ib, job.nt, recs, org, tgt);
+      PlaneRelArgs<PlaneRel::Rec> a;
       a.d2 = 0.f;
       a.src = recs;
       a.org = org;
+      a.tgt = tgt;
       a.n_tiles = plan.n_tiles;
-      a.tiles_per_chunk = plan.tiles_per_chunk;
-      a.ib = job.ib;
       a.nt = job.nt;
       a.partial = job.partial;
       a.status = job.status;
@@ -1352,26 +1356,26 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
         src_list = job.sorted;
       }
       // velocity and velocity gradient (W = vort A / (2 pi), D = div A / (2 pi))
-      PlaneRel::Rec* recs = static_cast<PlaneRel::Rec*>(job.src_buf);
+      PlaneSwe::Rec* recs = static_cast<PlaneSwe::Rec*>(job.src_buf);
       PlaneRel::Origin* org = reinterpret_cast<PlaneRel::Origin*>(
-          static_cast<char*>(job.src_buf) + align_up(static_cast<size_t>(npad) * sizeof(PlaneRel::Rec), 256));
-      plane_rel_prep_kernel<kPlaneTile><<<static_cast<unsigned>(plan.n_tiles), kPlaneTile, 0, job.stream>>>(
-          job.x, job.y, job.s1, job.area, src_list, job.ns, 1.0 / (2.0 * kPi), recs, org, job.s2);
-      PlaneRelArgs a;
-      a.x = job.x;
-      a.y = job.y;
+          static_cast<char*>(job.src_buf) + align_up(static_cast<size_t>(npad) * sizeof(PlaneSwe::Rec), 256));
+      PlaneRel::Tgt* tgt = reinterpret_cast<PlaneRel::Tgt*>(static_cast<char*>(job.src_buf) + plan.tgt_offset);
+      const unsigned prep = static_cast<unsigned>(plan.n_tiles + ceil_div(job.nt, kPlaneTile));
+      plane_rel_prep_kernel<kPlaneTile><<<prep, kPlaneTile, 0, job.stream>>>(
+          job.x, job.y, job.s1, job.area, src_list, job.ns, plan.n_tiles, 1.0 / (2.0 * kPi), job.ib, job.nt, recs, org,
+          tgt, job.s2);
+      PlaneRelArgs<PlaneSwe::Rec> a;
       a.d2 = 0.f;
       a.src = recs;
       a.org = org;
+      a.tgt = tgt;
       a.n_tiles = plan.n_tiles;
-      a.tiles_per_chunk = plan.tiles_per_chunk;
-      a.ib = job.ib;
       a.nt = job.nt;
       a.partial = job.partial;
       a.status = job.status;
-      const dim3 grid(static_cast<unsigned>(ceil_div(job.nt, kPseThreads * kPseTpt)),
+      const dim3 grid(static_cast<unsigned>(ceil_div(job.nt, kPlaneThreads * kSweTpt)),
                       static_cast<unsigned>(plan.nsplit));
-      plane_swe_rel_sweep_kernel<kPseThreads, kPseTpt, kPlaneTile, kSweMinB><<<grid, kPseThreads, 0, job.stream>>>(a);
+      plane_swe_rel_sweep_kernel<kPlaneThreads, kSweTpt, kPlaneTile, kSweMinB><<<grid, kPlaneThreads, 0, job.stream>>>(a);
       swe_finish_kernel<<<fin_grid, pb, 0, job.stream>>>(job.partial, plan.nsplit, job.nt, job.out0, job.out1,
                                                          job.out2);
       // surface-height Laplacian: the planar K8 PSE sweep on sh = s3, same source order
