@@ -489,6 +489,39 @@ bool sum_uses_sorted_sources(int kind, int mode) {
 }
 
 namespace {
+// Split-K factor of a sweep with interleaved chunks (chunk c of s takes every s-th tile, so any s
+// serves): the s that minimises the modelled time of the fullest SM, in tiles of one CTA at full rate,
+//   mean chunk x CTAs in whole rounds + longest chunk x (rest / f(rest / per_sm) + per_sm / 10)
+//   + 0.2 x (256 x 512 / pairs of a tile) x CTAs,
+// with f(x) = 0.45 + 0.55 x the rate of a last round that fills x of the SM's places (2 of 4 CTAs ran
+// at 0.73 of 4's rate, 3 of 4 at 0.9), a tenth of a round for CTAs that take longer than their peers
+// (near groups), and a fifth of a 256-source tile of 512 targets per CTA.  More than one round is better
+// than one exactly full: BVE sums of 50,000, 100,000 and 150,000 points took 0.98, 2.62 and 5.32 ms at
+// 3.9 CTAs per SM (one round, as choose_split has it) and 0.89, 2.47 and 5.13 ms at 15 to 23.  At most
+// 64 CTAs per SM, which also bounds the partial sums.  Ties (0.5 %) go to the smaller split.
+int64_t choose_interleaved_split(int64_t blocks, int64_t tiles, int64_t sms, int64_t per_sm, int64_t tile_pairs) {
+  if (blocks < 1) blocks = 1;
+  int64_t lim = std::max<int64_t>(64 * sms / blocks, 1);
+  if (lim > tiles) lim = tiles;
+  int64_t best = 1;
+  double best_cost = 1e300;
+  const double cta = 0.2 * (256.0 * 512.0) / static_cast<double>(tile_pairs);
+  for (int64_t s = 1; s <= lim; ++s) {
+    const int64_t ctas = ceil_div(blocks * s, sms);
+    const int64_t whole = ctas / per_sm * per_sm, rest = ctas - whole;
+    const double longest = static_cast<double>(ceil_div(tiles, s));
+    const double mean = ctas <= per_sm ? longest : static_cast<double>(tiles) / static_cast<double>(s);
+    const double per = static_cast<double>(per_sm);
+    const double tail = rest > 0 ? static_cast<double>(rest) / (0.45 + 0.55 * static_cast<double>(rest) / per) : 0.0;
+    const double cost = mean * static_cast<double>(whole) + longest * (tail + 0.1 * per) + cta * static_cast<double>(ctas);
+    if (cost < best_cost * 0.995) {
+      best_cost = cost;
+      best = s;
+    }
+  }
+  return best;
+}
+
 // The FP32C PSE sums sweep only the tiles within reach of each CTA's targets, in balanced
 // shares (engine.cuh); their prep kernels write a ball per tile.
 bool pse_culls_tiles(int kind) {
@@ -608,9 +641,9 @@ SumPlan plan_sum(int kind, int mode, int64_t ns, int64_t nt, int sm_count, int s
   } else {
     const bool bve = kind == kSumBve || kind == kSumBveMesh;
     const int64_t tiles = bve ? pl.n_tiles * (kBveTile / kBveShapes[shape].tile) : pl.n_tiles;
-    const int64_t nsplit = choose_split(tblocks, tiles, slots, 65535);
-    pl.tiles_per_chunk = ceil_div(tiles, nsplit);
-    pl.nsplit = ceil_div(tiles, pl.tiles_per_chunk);
+    pl.nsplit = choose_interleaved_split(
+        tblocks, tiles, slots / minb, minb, (bve ? kBveShapes[shape].tile : tile) * targets_per_cta(kind, shape));
+    pl.tiles_per_chunk = ceil_div(tiles, pl.nsplit);
   }
   pl.partial_bytes = static_cast<size_t>(pl.nsplit) * comps_of(kind) * nt * sizeof(double);
   if (kind == kSumSwePlane || kind == kSumSweSphere) {
