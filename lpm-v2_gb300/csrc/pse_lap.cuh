@@ -173,11 +173,20 @@ __global__ void __launch_bounds__(THREADS, MINB) pse_lap_sweep_kernel(PseLapArgs
   tile_pipe_init(pipe);
   uint32_t g = 0;
   auto tile_body = [&](const Rec* tl, const Group* og) {
+    // a group's terms are summed on their own: a running sum of the tile's four groups had 1.1 to
+    // 1.3 times the error
     float2 acc[NP];
+    auto flush = [&]() {
 #pragma unroll
-    for (int p = 0; p < NP; ++p) acc[p] = make_float2(0.f, 0.f);
+      for (int p = 0; p < NP; ++p) {
+        comp_add(hs[p].x, ls[p].x, acc[p].x);
+        comp_add(hs[p].y, ls[p].y, acc[p].y);
+      }
+    };
 #pragma unroll 1
     for (int g0 = 0; g0 < TILE; g0 += G) {
+#pragma unroll
+      for (int p = 0; p < NP; ++p) acc[p] = make_float2(0.f, 0.f);
       const Group o = og[g0 / G];
       const Rec* gr = tl + g0;
       float2 tx[NP], ty[NP], tz[NP], nf[NP], nl[NP];
@@ -214,6 +223,7 @@ __global__ void __launch_bounds__(THREADS, MINB) pse_lap_sweep_kernel(PseLapArgs
         } else {
           lap_group<SPHERE, K8, ANG, false, 1, 2>(gr, a.q, tx, ty, tz, nf, nl, acc);
         }
+        flush();
         continue;
       }
       // wide group: d = (t_hi - s_hi) + (t_lo - s_lo)
@@ -240,11 +250,7 @@ __global__ void __launch_bounds__(THREADS, MINB) pse_lap_sweep_kernel(PseLapArgs
           acc[p] = __ffma2_rn(m, k, acc[p]);
         }
       }
-    }
-#pragma unroll
-    for (int p = 0; p < NP; ++p) {
-      comp_add(hs[p].x, ls[p].x, acc[p].x);
-      comp_add(hs[p].y, ls[p].y, acc[p].y);
+      flush();
     }
   };
   // this CTA's balanced share of the in-reach tiles of the whole source range (engine.cuh)
