@@ -204,7 +204,7 @@ __device__ __forceinline__ bool warp_near(const float2 (&tx)[NP], const float2 (
 }
 
 // One staged tile against NP target pairs: FP32 partials of D added into (ax, ay, az).  The far
-// loop is unrolled UNROLL times (4 measured 0.2 % faster than 2 for the 128 x 8 sweep).
+// loop is unrolled UNROLL times (4 is 1 to 2 % faster than 2 for the 128 x 6 sweep, 2 keeps the 128 x 4 one from spilling more).
 template <int NP, int TILE, int UNROLL = 4>
 __device__ __forceinline__ void bve_rel_tile(const BveRel::Rec* __restrict__ tl, const BveRel::Group* __restrict__ og,
                                              const BveX2::Pair (&pr)[NP], float2 (&ax)[NP], float2 (&ay)[NP],
@@ -361,7 +361,7 @@ __device__ __forceinline__ void bve_merge_pairs(const float2 (&ax)[NP], const fl
   }
 }
 
-template <int THREADS, int TPT, int TILE, int MINB, bool DECOUPLED>
+template <int THREADS, int TPT, int TILE, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB) bve_rel_sweep_kernel(SweepArgs<BveF32> a,
                                                                       const BveRel::Group* __restrict__ org,
                                                                       const BveRel::Tgt* __restrict__ tgt) {
@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(THREADS, MINB) bve_rel_sweep_kernel(SweepArgs<
   constexpr int NP = TPT / 2;
   constexpr int GPT = TILE / BveRel::kGroup;
   using Rec = BveRel::Rec;
-  __shared__ TilePipe<Rec, TILE, 2> pipe;  // (its full barriers serve the block-synchronous pipeline too)
+  __shared__ TilePipe<Rec, TILE, 2> pipe;
 
   const int64_t chunk = blockIdx.y;
   const ChunkTiles ct = chunk_tiles(a.n_tiles);
@@ -394,15 +394,9 @@ __global__ void __launch_bounds__(THREADS, MINB) bve_rel_sweep_kernel(SweepArgs<
     tile += ct.step;
     bve_merge_pairs<NP>(ax, ay, az, hx, hy, hz, lx, ly, lz);
   };
-  if constexpr (DECOUPLED) {
-    tile_pipe_init(pipe);
-    warp_sweep_tiles(src, [ct](int64_t k) { return ct.first + k * ct.step; }, ct.count, pipe, g, a.status, a.wait,
-                     static_cast<const Rec*>(nullptr), body);
-  } else {
-    pipe_init(pipe.full);
-    staged_sweep<Rec, TILE>(src, ct.first, ct.count, pipe.stage[0], pipe.stage[1], pipe.full, g, a.status, a.wait, body,
-                            ct.step);
-  }
+  tile_pipe_init(pipe);
+  warp_sweep_tiles(src, [ct](int64_t k) { return ct.first + k * ct.step; }, ct.count, pipe, g, a.status, a.wait,
+                   static_cast<const Rec*>(nullptr), body);
 
 #pragma unroll
   for (int p = 0; p < NP; ++p) {

@@ -30,23 +30,20 @@ constexpr double kPi = 3.1415926535897932384626433832795027975;
 
 // FP32C sweep shapes (threads per CTA, targets per thread, tile, min CTAs per SM)
 constexpr int kBveTile = 256;
-// Shapes of the sphere-BVE FP32C sweep the autotuner chooses from: threads per CTA,
-// targets per thread (in pairs), CTAs per SM, and whether its warps run decoupled (they lose less
-// to the near groups that some of them meet: icosahedral nest 5 7 % faster than the
-// block-synchronous pipeline, nest 6 2 %; at nest 7, with few near groups, 0.5 % slower).
+// Shapes of the sphere-BVE FP32C sweep the autotuner chooses from: threads per CTA, targets per thread
+// (in pairs), CTAs per SM.  All run warp-decoupled (their warps lose less to the near groups that some
+// of them meet).  128 x 6 at 3 CTAs per SM is the fastest from icosahedral nest 5 on, although it spills
+// 41 registers (accumulators, once per tile): 1.005, 11.77 and 177.7 ms an RK4 step at nests 5, 6 and 7,
+// where 128 x 4 at 4 took 1.041, 12.17 and 186.8.  128 x 6 and 128 x 8 at 2 CTAs per SM and block-synchronous
+// warps were never the fastest.
 struct BveShape {
   int threads, tpt, minb;
-  bool decoupled;
   int tile;  // sources per sweep tile: 256, or 128 (a group) for small sets
 };
 // The last one is for small sets, whose few targets and sources leave most SMs idle at 512 targets by
 // 256 sources a CTA: icosahedral nest 3 (1,922 targets, 1,280 sources) has 20 such CTAs, and 80 of 256
 // targets by one group.
-constexpr BveShape kBveShapes[] = {{128, 4, 4, true, kBveTile},
-                                   {128, 4, 4, false, kBveTile},
-                                   {128, 6, 2, true, kBveTile},
-                                   {128, 8, 2, false, kBveTile},
-                                   {128, 2, 6, true, BveRel::kGroup}};
+constexpr BveShape kBveShapes[] = {{128, 4, 4, kBveTile}, {128, 6, 3, kBveTile}, {128, 2, 6, BveRel::kGroup}};
 constexpr int kBveShapeCount = sizeof(kBveShapes) / sizeof(kBveShapes[0]);
 constexpr int kPlaneThreads = 128, kPlaneTpt = 4, kPlaneTile = 256, kPlaneMinB = 4;
 // PSE sweeps (warp-decoupled pipeline): 256-source tiles in two stages; the divergence, whose
@@ -563,8 +560,6 @@ size_t sort_scratch_bytes(int kind, int64_t ns, int64_t nt) {
   if (kind == kSumPseGaussChord) return std::max({curve_sort_bytes(m), curve_sort2d_bytes(m), select_in_order_bytes(m)});
   return std::max(curve_sort_bytes(m), pse_sorts_targets(kind) ? select_in_order_bytes(m) : size_t{0});
 }
-
-int bve_shape_count() { return kBveShapeCount; }
 
 SumPlan plan_sum(int kind, int mode, int64_t ns, int64_t nt, int sm_count, int shape) {
   if (shape < 0 || shape >= kBveShapeCount) shape = 0;
@@ -1127,19 +1122,13 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
       const dim3 grid(static_cast<unsigned>(ceil_div(job.nt, sh.threads * sh.tpt)), static_cast<unsigned>(plan.nsplit));
       switch (plan.shape) {
         case 0:
-          bve_rel_sweep_kernel<128, 4, kBveTile, 4, true><<<grid, 128, 0, job.stream>>>(a, org, tgt);
+          bve_rel_sweep_kernel<128, 4, kBveTile, 4><<<grid, 128, 0, job.stream>>>(a, org, tgt);
           break;
         case 1:
-          bve_rel_sweep_kernel<128, 4, kBveTile, 4, false><<<grid, 128, 0, job.stream>>>(a, org, tgt);
-          break;
-        case 2:
-          bve_rel_sweep_kernel<128, 6, kBveTile, 2, true><<<grid, 128, 0, job.stream>>>(a, org, tgt);
-          break;
-        case 3:
-          bve_rel_sweep_kernel<128, 8, kBveTile, 2, false><<<grid, 128, 0, job.stream>>>(a, org, tgt);
+          bve_rel_sweep_kernel<128, 6, kBveTile, 3><<<grid, 128, 0, job.stream>>>(a, org, tgt);
           break;
         default:
-          bve_rel_sweep_kernel<128, 2, BveRel::kGroup, 6, true><<<grid, 128, 0, job.stream>>>(a, org, tgt);
+          bve_rel_sweep_kernel<128, 2, BveRel::kGroup, 6><<<grid, 128, 0, job.stream>>>(a, org, tgt);
           break;
       }
       finish_bve_kernel<<<fin_grid, pb, 0, job.stream>>>(job.partial, plan.nsplit, job.nt, job.ib, job.x,

@@ -15,7 +15,7 @@ struct SumPlan {
   int64_t nsplit = 1;        // split-K chunks (gridDim.y)
   size_t src_bytes = 0;      // bytes of the padded source-record array
   size_t partial_bytes = 0;  // bytes of the FP64 partial sums
-  int shape = 0;             // sweep shape (sphere BVE FP32C; see bve_shape_count)
+  int shape = 0;             // sweep shape (sphere BVE FP32C)
   int fp64_threads = 128;    // FP64 sequential sweep CTA size (32, 64 or 128: the best-balanced)
   int64_t sm_count = 152;    // SMs the FP64 sweeps are laid out for
   // a second sweep of the same job (the planar SWE surface-height Laplacian): its tiles and
@@ -102,9 +102,6 @@ int64_t choose_split(int64_t blocks, int64_t tiles, int64_t slots, int64_t max_s
 // Decides tiles, split-K and (for the sphere BVE FP32C sweep) the CTA shape of a job on a
 // device with sm_count SMs.
 SumPlan plan_sum(int kind, int mode, int64_t ns, int64_t nt, int sm_count, int shape = 0);
-
-// Number of sweep shapes of the sphere BVE FP32C sum.
-int bve_shape_count();
 
 // Autotuner: the shape of the sphere BVE FP32C sweep for a problem size, chosen once per
 // size class by timing every shape on the job (its targets limited to a bounded subset) and
