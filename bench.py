@@ -59,11 +59,11 @@ L2_FLUSH_BYTES = 256 << 20
 # DRAM bytes (ncu dram__bytes_read.sum + dram__bytes_write.sum) of one full-size icos nest 8
 # sweep launch, from a single-pass ncu capture of this benchmark's own step (ncu cannot run
 # inside the timed region, so this is a recorded constant, not a figure of this run)
-SWEEP_TRAFFIC_ICOS8 = 264_474_880 + 126_703_360
-# Pipe utilisation of the same sweep kernel (ncu --set full of bve_rel_sweep_kernel<128,4,256,4>,
+SWEEP_TRAFFIC_ICOS8 = 357_470_000 + 131_950_000
+# Pipe utilisation of the same sweep kernel (ncu of bve_rel_sweep_kernel<128,6,256,3>,
 # the autotuner's shape, on this workload at icos nest 7, one launch): the pipe-level counterpart
 # of the flop-contract fraction; recorded constants, not figures of this run
-SWEEP_PIPES_ICOS7 = {"fma_pipe_active": 0.6801, "xu_pipe_active": 0.6448, "issue_active": 0.5366}
+SWEEP_PIPES_ICOS7 = {"fma_pipe_active": 0.5786, "xu_pipe_active": 0.7248, "issue_active": 0.4589}
 # FP32 CUDA-core nominal peak: 152 SMs x 128 lanes x 2 flops per FMA, per MHz of SM clock
 FP32_NOMINAL_TFLOPS_PER_MHZ = 152 * 128 * 2 / 1e6
 # FP64: 2 DFMA per clock per SM (4 flops), per MHz
@@ -399,7 +399,7 @@ def run_ours(args):
                          "traffic": SWEEP_TRAFFIC_ICOS8 if args.nest == 8 else None,
                          "traffic_unit": "bytes per sweep launch: ncu dram__bytes_read.sum + dram__bytes_write.sum "
                                          "of one full-size launch (a recorded capture, not measured in this run)",
-                         "pipes": dict(SWEEP_PIPES_ICOS7, source="ncu --set full of the same sweep kernel on this "
+                         "pipes": dict(SWEEP_PIPES_ICOS7, source="ncu of the same sweep kernel on this "
                                        "workload at icos nest 7 (sm__pipe_fma_cycles_active, "
                                        "sm__pipe_xu_cycles_active, smsp__issue_active; recorded, not this run)"),
                          "kernel": "bve_rel_sweep_kernel (+ its prep and finish kernels) per velocity sum",

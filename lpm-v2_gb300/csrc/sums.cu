@@ -344,9 +344,9 @@ int tile_of(int kind, int mode) {
   }
 }
 
-// Sources per group origin of a group-relative FP32C layout: 128 for the sphere BVE sweep and
-// the sweeps that share its layout, 64 for the PSE sweeps (their cutoff's granularity) and
-// the planar and beta-plane ones.
+// Sources per group origin of a group-relative FP32C layout: 128 for the velocity sums and the planar
+// stream function (half the per-group work of 64), 64 for the sphere stream functions (the log1p form wants
+// small groups) and the beta plane, less for the PSE sums (their cutoff's granularity).
 int origin_group(int kind) {
   switch (kind) {
     case kSumBve:
