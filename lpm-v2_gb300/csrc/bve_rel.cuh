@@ -607,6 +607,12 @@ __device__ __forceinline__ GroupBasis group_basis(const GroupFrame& f) {
   return b;
 }
 
+// The radius of the near test: the group's, and at least sqrt(|k|) / 2.  C = ct + k and the coordinates c (about
+// 2k) are rounded at the size of k = (1 - |o|^2) / 2, which is R^2 / 4 for a patch of the sphere but up to 2^-24 for a
+// tight cluster, whose origin is off the sphere by its own rounding (and more for points off the sphere); at
+// |t| >= 1.5 sqrt(|k|) h is no smaller than |k|, so those roundings stay a few ulps of it.
+__device__ __forceinline__ float near_radius(float r, const GroupBasis& b) { return fmaxf(r, 0.5f * sqrtf(fabsf(b.k))); }
+
 // A source's coordinates in its group's basis, s_j = a e1 + b e2 + c o for its offset (hi, lo): the
 // projections less their first-order coupling (2^-24 of them; the second order is 2^-48).
 __device__ __forceinline__ void basis_coords(const GroupBasis& b, const GroupFrame& f, const float (&hi)[3],
@@ -672,7 +678,7 @@ __device__ __forceinline__ void bve_rel_prep_tile(const double* x, const double*
     // in d for all of them.  Measured at icosahedral nests 5, 6, 7 against FP64 (relative L2 of the
     // velocity): 1.86e-7, 8.60e-8, 4.95e-8 from 3 R on, 1.73e-7, 7.95e-8, 4.65e-8 from 1.5 R on, and
     // 3, 3 and 1 % faster.
-    g.o.hi.w = f.compact ? -0.5f * f.radius : f.radius;
+    g.o.hi.w = f.compact ? -near_radius(0.5f * f.radius, b) : near_radius(f.radius, b);
     if (b.singular) g.o.hi.w = 1e15f;             // near every target
     g.o.lo.x = b.k;
     g.o.lo.y = 1.f - b.k;  // |o|^2 + k

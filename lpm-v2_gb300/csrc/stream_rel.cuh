@@ -530,7 +530,8 @@ __global__ void __launch_bounds__(TILE) stream_prep_kernel(const double* x, cons
   if (threadIdx.x % G == 0) {
     StreamFn::Group g;
     g.o = group_origin(f);
-    g.o.hi.w = f.compact ? -f.radius : f.radius;
+    const float rn = near_radius(f.radius, b);
+    g.o.hi.w = f.compact ? -rn : rn;
     if (b.singular) g.o.hi.w = 1e15f;  // near every target
     if (k >= ns) g.o.hi.w = 3.0e38f;   // no sources
     g.o.lo = make_float4(b.k, 1.f - b.k, 1.00001f * sqrtf(fmaxf(mx[wid][0], mx[wid + 1][0])),
