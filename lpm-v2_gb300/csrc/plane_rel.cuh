@@ -98,7 +98,8 @@ __global__ void __launch_bounds__(THREADS, MINB) plane_rel_sweep_kernel(PlaneRel
   constexpr int G = PlaneRel::kGroup;
   constexpr int GPT = TILE / G;
   using Rec = PlaneRel::Rec;
-  __shared__ TilePipe<Rec, TILE, 2, PlaneRel::Origin, GPT> pipe;
+  __shared__ __align__(128) Rec stage[2][TILE];
+  __shared__ __align__(8) uint64_t bars[2];
 
   const int64_t chunk = blockIdx.y;
   const ChunkTiles ct = chunk_tiles(a.n_tiles);
@@ -112,7 +113,7 @@ __global__ void __launch_bounds__(THREADS, MINB) plane_rel_sweep_kernel(PlaneRel
   for (int p = 0; p < NP; ++p) hu[p] = hv[p] = lu[p] = lv[p] = make_float2(0.f, 0.f);
   const float2 d2 = make_float2(a.d2, a.d2);
 
-  tile_pipe_init(pipe);
+  pipe_init(bars);
   uint32_t g = 0;
   auto body = [&](const Rec* tl, const PlaneRel::Origin* og) {
     float2 au[NP], av[NP];
@@ -192,8 +193,11 @@ __global__ void __launch_bounds__(THREADS, MINB) plane_rel_sweep_kernel(PlaneRel
       comp_add(hv[p].y, lv[p].y, av[p].y);
     }
   };
-  warp_sweep_tiles(a.src, [ct](int64_t t) { return ct.first + t * ct.step; }, ct.count, pipe, g, a.status,
-                   default_wait(), a.org, body);
+  int64_t tile = ct.first;
+  staged_sweep<Rec, TILE>(a.src, ct.first, ct.count, stage[0], stage[1], bars, g, a.status, [&](const Rec* tl) {
+    body(tl, a.org + tile * GPT);
+    tile += ct.step;
+  }, ct.step);
 
 #pragma unroll
   for (int p = 0; p < NP; ++p) {

@@ -614,7 +614,8 @@ __global__ void __launch_bounds__(THREADS, MINB) plane_stream_rel_sweep_kernel(P
   constexpr int FLN = 16;
   static_assert(G % FLN == 0, "flush interval must divide the group");
   using Rec = PlaneRel::Rec;
-  __shared__ TilePipe<Rec, TILE, 2, PlaneRel::Origin, GPT> pipe;
+  __shared__ __align__(128) Rec stage[2][TILE];
+  __shared__ __align__(8) uint64_t bars[2];
   __shared__ __align__(8) float2 ln_tab[32];
 
   const int64_t chunk = blockIdx.y;
@@ -631,7 +632,7 @@ __global__ void __launch_bounds__(THREADS, MINB) plane_stream_rel_sweep_kernel(P
   constexpr float kHuge = 1.2676506002282294e30f;  // 2^100
 
   ln_tab_load(ln_tab);
-  tile_pipe_init(pipe);
+  pipe_init(bars);
   uint32_t g = 0;
   auto body = [&](const Rec* tl, const PlaneRel::Origin* og) {
 #pragma unroll 1
@@ -717,8 +718,11 @@ __global__ void __launch_bounds__(THREADS, MINB) plane_stream_rel_sweep_kernel(P
       }
     }
   };
-  warp_sweep_tiles(a.src, [ct](int64_t t) { return ct.first + t * ct.step; }, ct.count, pipe, g, a.status,
-                   default_wait(), a.org, body);
+  int64_t tile = ct.first;
+  staged_sweep<Rec, TILE>(a.src, ct.first, ct.count, stage[0], stage[1], bars, g, a.status, [&](const Rec* tl) {
+    body(tl, a.org + tile * GPT);
+    tile += ct.step;
+  }, ct.step);
 
   constexpr double kLn2 = 0.69314718055994530942;
 #pragma unroll

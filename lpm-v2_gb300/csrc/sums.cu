@@ -495,10 +495,10 @@ namespace {
 // (near groups), and a fifth of a 256-source tile of 512 targets per CTA.  More than one round is better
 // than one exactly full: BVE sums of 50,000, 100,000 and 150,000 points took 0.98, 2.62 and 5.32 ms at
 // 3.9 CTAs per SM (one round, as choose_split has it) and 0.89, 2.47 and 5.13 ms at 15 to 23.  At most
-// 64 CTAs per SM, which also bounds the partial sums.  Ties (0.5 %) go to the smaller split.
+// 256 CTAs per SM, which bounds the partial sums (64 was 1.3 % slower for the plane at quad nest 8).  Ties (0.5 %) go to the smaller split.
 int64_t choose_interleaved_split(int64_t blocks, int64_t tiles, int64_t sms, int64_t per_sm, int64_t tile_pairs) {
   if (blocks < 1) blocks = 1;
-  int64_t lim = std::max<int64_t>(64 * sms / blocks, 1);
+  int64_t lim = std::max<int64_t>(256 * sms / blocks, 1);
   if (lim > tiles) lim = tiles;
   int64_t best = 1;
   double best_cost = 1e300;
