@@ -334,7 +334,7 @@ def run_ours(args):
         fp64 = {"value": r64, "unit": UNIT, "fp32c_over_fp64": value / r64,
                 "contract_tflops": FLOPS_PER_INTERACTION * r64 / 1e3,
                 "frac_of_nominal_fp64_peak": FLOPS_PER_INTERACTION * r64 / 1e3 / (FP64_NOMINAL_TFLOPS_PER_MHZ * mhz),
-                "kernel": "seq_fp64_kernel<BveF64<0>> (one target per thread, sources in ascending order, "
+                "kernel": "seq_i64_kernel<BveI64<0>> (four lanes per target, sources in ascending order, "
                           "bit-identical to the oracle)",
                 "sample": f"targets {b64}..{b64 + m64 - 1} against all {ns} sources ({inter64:.3e} interactions), "
                           "one host C-ABI call, wall clock, copies included",
