@@ -323,9 +323,11 @@ __global__ void __launch_bounds__(TILE) pse_lap_prep_kernel(const double* x, con
 #pragma unroll
     for (int c = 0; c < 3; ++c) rel2(sp.h[c], sp.l[c], fr.o[c], hi[c], lo[c]);
     const float ar = __double2float_rn(area[j]);
-    float fs, fe;  // f_j - f_g = fs + fe
-    two_sum(fh, -fg, fs, fe);
-    fe += fl;
+    // f_j - f_g = fs + fe, fs rounded from all of it: the low part of f_j is the whole of F_j where f_j and f_g
+    // round to the same float (every group of a field with a large mean, and a group's first source)
+    float d, de, fs, fe;
+    two_sum(fh, -fg, d, de);
+    two_sum(d, de + fl, fs, fe);
     const float af = ar * fs, al = fmaf(ar, fs, -af) + ar * fe;
     r.a = make_float4(-hi[0], -hi[0], -hi[1], -hi[1]);
     r.b = make_float4(-hi[2], -hi[2], ar, ar);
