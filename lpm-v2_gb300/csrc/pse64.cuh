@@ -6,15 +6,20 @@
 //  - chord distances: q = |d|^2 / eps^2;
 //  - great-circle distances: q = theta^2 (a / eps)^2, with theta^2 = 4 asin^2(c / 2) a polynomial
 //    in the squared chord c^2 of the unit directions (Chebyshev interpolation of the function,
-//    within 2^-57 of it; for c up to 0.45, 1.14 and, with the supplement beyond 90 degrees, 2);
-//  - the constants' divisions (eps, 3, pi) are folded into k0..k3;
+//    within 2^-57 of it; for c up to 0.45, 1.14 and, with the supplement beyond 90 degrees, 2).
+//    c^2 comes from the positions: |d|^2 / r^2 for particles as far from the centre as each other to their
+//    rounding, (|d|^2 - (r - r')^2) / (r r') for others;
+//  - pi and the powers of eps divide the sum once at the end;
 //  - E by table and polynomial (P. T. P. Tang, Table-driven implementation of the exponential
 //    function, ACM TOMS 15, 1989): with s = 256 q / ln 2 and i = round(s),
 //    E = 2^-(i / 256) 2^-((s - i) / 256), a table of 256 powers and a polynomial of degree 4
 //    (remainder 4e-17).
-// That is about 32 FP64 instructions a pair for K8 of the great-circle distance, where the
+// That is about 33 FP64 instructions a pair for K8 of the great-circle distance, where the
 // reference's expressions take about 150.  The results agree with the reference's to its own rounding
-// (1e-15 of the largest; its exp and atan2 are not CUDA's either).  A lane's sum is in the reference's
+// (1e-15 of the largest; its exp and atan2 are not CUDA's either): root mean square error against the sums in
+// extended precision, as a share of the reference expressions' own, at cubed nest 5: K8 0.58, gradient 0.60,
+// divergence 0.87; 0.57, 0.66 and 0.98 for particles 1e-7 off the sphere (pairs of rounded unit directions
+// and kernel polynomials in s, with rounded coefficients, gave 1.4 to 3 times the reference's error).  A lane's sum is in the reference's
 // ascending order; small target sets have up to 8 lanes per target, each summing its part of every
 // tile, and add the parts at the end.
 //
@@ -29,14 +34,14 @@
 //    warp work on different sources, and take about as many each.  At cubed nest 6 a warp takes
 //    1.02 x the mean number of pairs in reach of a target; tile by tile it would take 1.31 x, whole
 //    tiles 1.9 x.  Two pairs, because a warp alone waits about 80 clocks for each FP64 result.
-// A pair with a particle that has no direction (at the origin of a sphere) or no finite position
-// takes the reference's expressions as they stand (Op::Plain), as do all pairs of a reach beyond
-// the polynomials' range.
+// A pair with a particle that has no direction (at the origin of a sphere) or no finite position, or
+// whose particles differ by more than a quarter in their distance from the centre, takes the reference's
+// expressions as they stand (Op::Plain), as do all pairs of a reach beyond the polynomials' range.
 //
 // Bound by the FP64 pipe (2 lanes per clock per SM): 73-77 % busy at cubed nest 6, the rest being
 // the last warps of an SM.  Host calls on GB300, ms, before (the reference's expressions over whole
 // tiles) and after: cubed nest 4 K8 7.1 -> 0.38, gradient 7.5 -> 0.43, double dot 13.5 -> 0.48; nest 6
-// K8 37 -> 4.4, Gaussian 12.7 -> 1.8, gradient 40 -> 5.3, divergence 49 -> 6.3, double dot 67 -> 6.8,
+// K8 37 -> 4.55, Gaussian 12.7 -> 1.65, gradient 40 -> 5.2, divergence 49 -> 6.3, double dot 67 -> 6.8,
 // interpolation 37 -> 4.6; quad nest 6 K8 7.3 -> 1.2, gradient 8.4 -> 1.3, second partials 11.5 -> 1.5.
 #pragma once
 
@@ -86,8 +91,8 @@ struct Pse64Src {
 };
 
 struct Pse64Args {
-  double c;               // s = 256 q / ln 2 per squared distance (chord) or squared angle
-  double k0, k1, k2, k3;  // the kernel as a polynomial in s, with the constants that divide it
+  double c;               // q per squared distance (chord) or squared angle
+  double scale, unscale;  // what divides the kernel's polynomial (pi, powers of eps), and its inverse
   double reach;           // of the cutoff, in the test space
   int unit;               // 1: the test space is unit directions
   int all_plain;          // 1: every pair in the reference's expressions
@@ -101,23 +106,41 @@ struct Pse64Args {
   int* status;
 };
 
+constexpr double kPse64PerQ = 369.32993046757463228;  // 256 / ln 2
+
 // The point of particle i in the test space.  A point at the origin of a sphere has no direction
 // (and atan2(0, 0) puts it at distance 0 from everything); it becomes NaN, which every test reads
 // as "in reach".
-__device__ __forceinline__ double3 cut_point(const double* x, const double* y, const double* z, int64_t i, int unit) {
-  double3 q = make_double3(x[i], y[i], z ? z[i] : 0.0);
+struct CutPoint {
+  double3 raw, q;  // the position, and the point in the test space
+  double r;        // |raw| (test space of unit directions)
+};
+
+__device__ __forceinline__ CutPoint cut_point(const double* x, const double* y, const double* z, int64_t i, int unit) {
+  CutPoint p;
+  p.raw = make_double3(x[i], y[i], z ? z[i] : 0.0);
+  p.q = p.raw;
+  p.r = 1.0;
   if (unit) {
-    const double nq = sqrt(q.x * q.x + q.y * q.y + q.z * q.z);
-    const double inv = nq > 0.0 ? 1.0 / nq : __longlong_as_double(0x7ff8000000000000LL);
-    q = make_double3(q.x * inv, q.y * inv, q.z * inv);
+    // (explicit operations: the targets' and the sources' |p| have to round alike)
+    p.r = sqrt(fma(p.raw.x, p.raw.x, fma(p.raw.y, p.raw.y, __dmul_rn(p.raw.z, p.raw.z))));
+    const double inv = p.r > 0.0 ? 1.0 / p.r : __longlong_as_double(0x7ff8000000000000LL);
+    p.q = make_double3(p.raw.x * inv, p.raw.y * inv, p.raw.z * inv);
   }
-  return q;
+  return p;
 }
 
-// Whether a test point is NaN or infinite in some component.
-__device__ __forceinline__ bool odd_point(const double3& q) {
-  const double v = (q.x - q.x) + (q.y - q.y) + (q.z - q.z);
-  return !(v == 0.0);
+// Whether a point's pairs take the reference's expressions: NaN or infinite in some component of the
+// test space, or (unit directions) at a distance whose square would leave the exponent's range.
+__device__ __forceinline__ bool odd_point(const CutPoint& p) {
+  const double v = (p.q.x - p.q.x) + (p.q.y - p.q.y) + (p.q.z - p.q.z);
+  return !(v == 0.0) || !(p.r >= 0x1p-450 && p.r <= 0x1p450);
+}
+
+// Whether two particles' distances from the sphere's centre are the same to their rounding (within 4
+// units in the last place); a particle that is odd has one that is no other's.
+__device__ __forceinline__ bool same_radius(long long a, double b) {
+  return static_cast<unsigned long long>(__double_as_longlong(b)) - static_cast<unsigned long long>(a) + 4ull <= 8ull;
 }
 
 // ------------------------------------------------------------------ a pair's kernel value
@@ -143,45 +166,73 @@ __device__ __forceinline__ double angle2(double v) {
   return t * t;
 }
 
-template <bool POLY>
-__device__ __forceinline__ double pse64_kernel_value(const Pse64Args& a, double s, const double* powers) {
+// The kernel (without what divides its polynomial) at q = c v.  The polynomial is in q, where its
+// coefficients are exact: in s, their roundings were common to all pairs of a sum, whose moments cancel.
+template <class Op>
+__device__ __forceinline__ double pse64_kernel_value(double v, double c, const double* powers) {
   const double big = 6755399441055744.0;  // 1.5 x 2^52: the sum's low word is round(s)
-  const double t = s + big;
+  const double q = __dmul_rn(v, c);
+  const double t = fma(q, kPse64PerQ, big);
   const int i = __double2loint(t);
-  const double f = s - (t - big);
+  const double f = fma(q, kPse64PerQ, __dsub_rn(big, t));
   double p = 0x1.3b2ab6fba4e77p-39;  // (-ln 2 / 256)^n / n!
   p = fma(p, f, -0x1.c6b08d704a0c0p-29);
   p = fma(p, f, 0x1.ebfbdff82c58fp-19);
   p = fma(p, f, -0x1.62e42fefa39efp-9);
   p = fma(p, f, 1.0);
-  const double e = powers[i & 255] * p;
+  const double e = __dmul_rn(powers[i & 255], p);
   const double scaled = __hiloint2double(__double2hiint(e) - ((i >> 8) << 20), __double2loint(e));
-  const double w = POLY ? scaled * fma(fma(fma(a.k3, s, a.k2), s, a.k1), s, a.k0) : scaled * a.k0;
-  // s >= 1020 x 256 (q >= 707, where the kernel is below 1e-300) leaves the exponent's range
-  return __double2hiint(s) >= 0x410fe000 ? 0.0 : w;
+  const double w = Op::kPoly ? __dmul_rn(scaled, Op::poly(q)) : scaled;
+  // at q >= 707 (0x40861800 00000000, where the kernel is below 1e-300) i leaves the exponent's range
+  return __double2hiint(q) >= 0x40861800 ? 0.0 : w;
 }
 
 // ------------------------------------------------------------------ operators
-// An operator's record holds the test point (x, y, z), the fields that its pairs need, the
-// particle's index and whether it is odd (odd_point).  add() adds the pair's terms, with w the kernel
-// value over the operator's powers of eps; the accumulators are Plain's, in its units.
+// An operator's record holds the position (x, y, z), the fields that its pairs need, the particle's
+// index and whether it is odd (odd_point); with great-circle distances also |p| and its inverse (r NaN
+// if odd).  add() adds the pair's terms, with d the difference of the positions and w the kernel value.
+// The accumulators are Plain's, in units of Pse64Args::scale.
 struct Pse64Op {
   static constexpr bool kPoly = true;   // false: a plain Gaussian
   static constexpr bool kUnit = false;  // true: great-circle distances
 };
+// The kernels over pi as polynomials in q = r^2 (times e^-q).
+struct Pse64K8 {  // bivariateLaplacianKernel8
+  __device__ static __forceinline__ double poly(double q) {
+    return fma(fma(fma(-2.0 / 3.0, q, 10.0), q, -40.0), q, 40.0);
+  }
+};
+struct Pse64K1 {  // bivariateFirstDerivativeKernel8
+  __device__ static __forceinline__ double poly(double q) {
+    return fma(fma(fma(1.0 / 3.0, q, -5.0), q, 20.0), q, -20.0);
+  }
+};
+struct Pse64Delta8 {  // bivariateDeltaKernel8
+  __device__ static __forceinline__ double poly(double q) {
+    return fma(fma(fma(-1.0 / 6.0, q, 2.0), q, -6.0), q, 4.0);
+  }
+};
+
+template <bool UNIT>
+struct __align__(16) Pse64ScalarRec {
+  double x, y, z, f, area;
+  int32_t idx, odd;
+};
+template <>
+struct __align__(16) Pse64ScalarRec<true> {
+  double x, y, z, f, area, r, inv;
+  int32_t idx, odd;
+};
 
 template <int KIND>
-struct PseLap64 : Pse64Op {
+struct PseLap64 : Pse64Op, Pse64K8 {
   using Plain = PseF64<KIND>;
   using Params = PseF64Params;
   using Acc = typename Plain::Acc;
   static constexpr int kDim = KIND == kPseK8Chord ? 2 : 3;
   static constexpr bool kPoly = KIND != kPseGaussChord;
   static constexpr bool kUnit = KIND == kPseK8Geodesic;
-  struct __align__(16) Rec {
-    double x, y, z, f, area;
-    int32_t idx, odd;
-  };
+  using Rec = Pse64ScalarRec<kUnit>;
   struct Tgt {
     double f;
   };
@@ -199,39 +250,38 @@ struct PseLap64 : Pse64Op {
 };
 
 template <bool SPHERE>
-struct PseInterp64 : Pse64Op {
+struct PseInterp64 : Pse64Op, Pse64Delta8 {
   static constexpr bool kUnit = SPHERE;
   using Plain = PseInterpF64<SPHERE>;
   using Params = PseExtF64Params;
   using Acc = typename Plain::Acc;
   static constexpr int kDim = 3;
-  struct __align__(16) Rec {
-    double x, y, z, fa;
-    int32_t idx, odd;
-    double pad;
-  };
+  using Rec = Pse64ScalarRec<SPHERE>;  // f: the product f A
   struct Tgt {};
   __device__ static void fill(Rec& r, const Pse64Src& s, int64_t j) {
-    r.fa = __dmul_rn(s.s1[j], s.area[j]);
-    r.pad = 0.0;
+    r.f = __dmul_rn(s.s1[j], s.area[j]);
+    r.area = 0.0;
   }
   __device__ static Tgt load(const Params&, int64_t) { return Tgt{}; }
   __device__ static __forceinline__ void add(const Tgt&, const Rec& r, double, double, double, double w, Acc& a) {
-    a.s = fma(r.fa, w, a.s);
+    a.s = fma(r.f, w, a.s);
   }
   __device__ static Rec64 plain_record(const Pse64Src& s, int64_t j) { return PseLap64<0>::plain_record(s, j); }
 };
 
-struct PsePlaneGrad64 : Pse64Op {
+struct PsePlaneGrad64 : Pse64Op, Pse64K1 {
   using Plain = PsePlaneGradF64;
   using Params = PseExtF64Params;
   using Acc = Plain::Acc;
   static constexpr int kDim = 2;
-  using Rec = PseLap64<0>::Rec;
+  using Rec = Pse64ScalarRec<false>;
   struct Tgt {
     double f;
   };
-  __device__ static void fill(Rec& r, const Pse64Src& s, int64_t j) { PseLap64<0>::fill(r, s, j); }
+  __device__ static void fill(Rec& r, const Pse64Src& s, int64_t j) {
+    r.f = s.s1[j];
+    r.area = s.area[j];
+  }
   __device__ static Tgt load(const Params& p, int64_t i) { return Tgt{p.s1[i]}; }
   __device__ static __forceinline__ void add(const Tgt& t, const Rec& r, double dx, double dy, double, double w,
                                              Acc& a) {
@@ -243,7 +293,7 @@ struct PsePlaneGrad64 : Pse64Op {
 };
 
 template <class Base>  // PsePlaneSecondF64 or PsePlaneDdotF64
-struct PlaneD464 : Pse64Op {
+struct PlaneD464 : Pse64Op, Pse64K1 {
   using Plain = Base;
   using Params = PseExtF64Params;
   using Acc = typename Base::Acc;
@@ -277,44 +327,39 @@ struct PlaneD464 : Pse64Op {
   }
 };
 
-// The sphere's first-derivative operators use the raw differences x_i - x_j beside the angle.
-struct PseVecRec64 {
-  double x, y, z, rx, ry, rz, a, b, c, area;
+// The sphere's first-derivative operators.
+struct __align__(16) PseVecRec64 {
+  double x, y, z, a, b, c, area, r, inv;
   int32_t idx, odd;
 };
 
 template <class Base>
-struct PseSphereVec64 : Pse64Op {
+struct PseSphereVec64 : Pse64Op, Pse64K1 {
   static constexpr bool kUnit = true;
   using Plain = Base;
   using Acc = typename Base::Acc;
   static constexpr int kDim = 3;
-  struct __align__(16) Rec : PseVecRec64 {
-    double pad;
-  };
+  using Rec = PseVecRec64;
   __device__ static void fill(Rec& r, const Pse64Src& s, int64_t j) {
-    r.rx = s.x[j];
-    r.ry = s.y[j];
-    r.rz = s.z[j];
     r.a = s.s1[j];
     r.b = s.s2 ? s.s2[j] : 0.0;
     r.c = s.s3 ? s.s3[j] : 0.0;
     r.area = s.area[j];
-    r.pad = 0.0;
   }
 };
 
 struct PseGrad64 : PseSphereVec64<PseGradF64> {
   using Params = PseVecF64Params;
   struct Tgt {
-    double x, y, z, f;
+    double f;
   };
-  __device__ static Tgt load(const Params& p, int64_t i) { return Tgt{p.x[i], p.y[i], p.z[i], p.f[i]}; }
-  __device__ static __forceinline__ void add(const Tgt& t, const Rec& r, double, double, double, double w, Acc& a) {
+  __device__ static Tgt load(const Params& p, int64_t i) { return Tgt{p.f[i]}; }
+  __device__ static __forceinline__ void add(const Tgt& t, const Rec& r, double dx, double dy, double dz, double w,
+                                             Acc& a) {
     const double g = (r.a + t.f) * r.area * w;
-    a.g0 = fma(g, t.x - r.rx, a.g0);
-    a.g1 = fma(g, t.y - r.ry, a.g1);
-    a.g2 = fma(g, t.z - r.rz, a.g2);
+    a.g0 = fma(g, dx, a.g0);
+    a.g1 = fma(g, dy, a.g1);
+    a.g2 = fma(g, dz, a.g2);
   }
   __device__ static Rec64 plain_record(const Pse64Src& s, int64_t j) { return PseLap64<0>::plain_record(s, j); }
 };
@@ -328,11 +373,12 @@ struct PseDiv64 : PseSphereVec64<PseDivF64> {
     return Tgt{p.x[i], p.y[i], p.z[i], p.vx[i], p.vy[i], p.vz[i]};
   }
   // (P d) . V = d . V - (x . d) (x . V)
-  __device__ static __forceinline__ void add(const Tgt& t, const Rec& r, double, double, double, double w, Acc& a) {
-    const double dx = t.x - r.rx, dy = t.y - r.ry, dz = t.z - r.rz;
+  __device__ static __forceinline__ void add(const Tgt& t, const Rec& r, double dx, double dy, double dz, double w,
+                                             Acc& a) {
     const double vx = r.a + t.vx, vy = r.b + t.vy, vz = r.c + t.vz;
-    const double dv = fma(dx, vx, fma(dy, vy, dz * vz));
-    const double xd = fma(t.x, dx, fma(t.y, dy, t.z * dz)), xv = fma(t.x, vx, fma(t.y, vy, t.z * vz));
+    const double dv = fma(dx, vx, fma(dy, vy, __dmul_rn(dz, vz)));
+    const double xd = fma(t.x, dx, fma(t.y, dy, __dmul_rn(t.z, dz))),
+                 xv = fma(t.x, vx, fma(t.y, vy, __dmul_rn(t.z, vz)));
     a.d = fma(fma(-xd, xv, dv) * r.area, w, a.d);
   }
   __device__ static RecVec64 plain_record(const Pse64Src& s, int64_t j) {
@@ -343,14 +389,13 @@ struct PseDiv64 : PseSphereVec64<PseDivF64> {
 struct PseSphereDdot64 : PseSphereVec64<PseSphereDdotF64> {
   using Params = PseExtF64Params;
   struct Tgt {
-    double x, y, z, u, v;
+    double u, v;
   };
-  __device__ static Tgt load(const Params& p, int64_t i) {
-    return Tgt{p.x[i], p.y[i], p.z[i], p.s1[i], p.s2[i]};
-  }
-  __device__ static __forceinline__ void add(const Tgt& t, const Rec& r, double, double, double, double w, Acc& a) {
+  __device__ static Tgt load(const Params& p, int64_t i) { return Tgt{p.s1[i], p.s2[i]}; }
+  __device__ static __forceinline__ void add(const Tgt& t, const Rec& r, double dx, double dy, double dz, double w,
+                                             Acc& a) {
     const double g = r.area * w;
-    const double gx = g * (t.x - r.rx), gy = g * (t.y - r.ry), gz = g * (t.z - r.rz);
+    const double gx = g * dx, gy = g * dy, gz = g * dz;
     const double su = r.a + t.u, sv = r.b + t.v, sw = r.c + t.v;  // w_j with v_i, as the reference
     a.ux = fma(su, gx, a.ux);
     a.uy = fma(su, gy, a.uy);
@@ -389,8 +434,10 @@ __global__ void __launch_bounds__(kPse64Tile) pse64_prep_kernel(Pse64Src s, cons
   const int64_t k = static_cast<int64_t>(blockIdx.x) * kPse64Tile + tid;
   const bool valid = k < ns;
   const int32_t j = valid ? idx[k] : 0;
-  const double3 q = valid ? cut_point(s.x, s.y, s.z, j, unit) : make_double3(0.0, 0.0, 0.0);
-  const bool odd = odd_point(q);
+  CutPoint p{};
+  if (valid) p = cut_point(s.x, s.y, s.z, j, unit);
+  const double3 q = p.q;
+  const bool odd = valid && odd_point(p);
   red[0][tid] = odd ? 0.0 : q.x;
   red[1][tid] = odd ? 0.0 : q.y;
   red[2][tid] = odd ? 0.0 : q.z;
@@ -421,9 +468,13 @@ __global__ void __launch_bounds__(kPse64Tile) pse64_prep_kernel(Pse64Src s, cons
   typename Op::Rec r{};
   if (valid) {
     Op::fill(r, s, j);
-    r.x = q.x;
-    r.y = q.y;
-    r.z = q.z;
+    r.x = p.raw.x;
+    r.y = p.raw.y;
+    r.z = p.raw.z;
+    if constexpr (Op::kUnit) {
+      r.r = odd ? __longlong_as_double(0x7ff8000000000000LL) : p.r;
+      r.inv = 1.0 / p.r;
+    }
     r.idx = j;
     r.odd = odd ? 1 : 0;
   }
@@ -462,8 +513,11 @@ __global__ void __launch_bounds__(32) pse64_sweep_kernel(typename Op::Params p, 
   const int64_t kk = valid ? k : a.nt - 1;
   const int64_t i = a.tperm ? static_cast<int64_t>(a.tperm[kk]) : a.ib + kk;
   const typename Op::Tgt t = Op::load(p, i);
-  const double3 tp = cut_point(a.x, a.y, a.z, i, a.unit);
-  const bool odd = a.all_plain || odd_point(tp);
+  const CutPoint cp = cut_point(a.x, a.y, a.z, i, a.unit);
+  const double3 tp = cp.q;
+  const bool odd = a.all_plain || odd_point(cp);
+  const long long rbits = odd ? static_cast<long long>(1ull << 63) : __double_as_longlong(cp.r);
+  const double inv = 1.0 / cp.r, inv2 = __dmul_rn(inv, inv);
   for (int e = lane; e < 256; e += 32) powers[e] = a.powers[e];
   tile_pipe_init(pp);  // (synchronises)
   // the ball around the warp's targets (NaN or infinite: in reach of everything)
@@ -474,6 +528,50 @@ __global__ void __launch_bounds__(32) pse64_sweep_kernel(typename Op::Params p, 
   const double wr = sqrt(far) * (1.0 + 1e-9) + 1e-9 * (fabs(wx) + fabs(wy) + fabs(wz)) + a.reach;
 
   Acc acc{};
+  // A pair's kernel value and terms.  `same`: both particles are as far from the sphere's centre.  The
+  // squared chord comes from the positions, whose differences are exact to 2^-53: rounding the unit
+  // directions moved every target by up to 2^-53, which the derivative kernels amplify by 1 / eps.
+  auto offset = [&](const Rec& n) {
+    return make_double3(__dsub_rn(cp.raw.x, n.x), __dsub_rn(cp.raw.y, n.y),
+                        Op::kDim == 3 ? __dsub_rn(cp.raw.z, n.z) : 0.0);
+  };
+  auto squared = [&](const Rec& n, const double3& d, bool same) {
+    double v = Op::kDim == 3 ? fma(d.x, d.x, fma(d.y, d.y, __dmul_rn(d.z, d.z))) : fma(d.x, d.x, __dmul_rn(d.y, d.y));
+    if constexpr (Op::kUnit) {
+      if (same) {
+        v = __dmul_rn(v, inv2);
+      } else {  // |p - p'|^2 = (r - r')^2 + r r' chord^2
+        const double dr = __dsub_rn(cp.r, n.r);
+        v = __dmul_rn(fma(-dr, dr, v), __dmul_rn(inv, n.inv));
+      }
+    }
+    return v;
+  };
+  auto regular = [&](const Rec& n) {
+    if constexpr (Op::kUnit) return same_radius(rbits, n.r);
+    return !odd && !n.odd;
+  };
+  // any pair
+  auto one = [&](const Rec& n) {
+    bool plain = odd || n.odd;
+    if constexpr (Op::kUnit) plain |= !(fabs(cp.r - n.r) <= 0.25 * cp.r);  // (the difference above cancels)
+    if (plain) {
+      constexpr int NA = static_cast<int>(sizeof(Acc) / sizeof(double));
+      const Acc d = pse64_plain<Op>(p, a.src, i, n.idx, odd ? acc : Acc{});
+      if (odd) {
+        acc = d;  // an odd target's sum is all in Plain's units
+      } else {
+        double* av = reinterpret_cast<double*>(&acc);
+        const double* dv = reinterpret_cast<const double*>(&d);
+#pragma unroll
+        for (int c = 0; c < NA; ++c) av[c] = fma(dv[c], a.unscale, av[c]);
+      }
+      return;
+    }
+    const double3 d = offset(n);
+    const double w = pse64_kernel_value<Op>(angle2<ANG>(squared(n, d, regular(n))), a.c, powers);
+    Op::add(t, n, d.x, d.y, d.z, w, acc);
+  };
   int held = 0;  // entries of mine and tile_of that this lane holds
   // Evaluates the held sources in ascending order.
   auto evaluate = [&]() {
@@ -501,20 +599,17 @@ __global__ void __launch_bounds__(32) pse64_sweep_kernel(typename Op::Params p, 
       at1 = next();
       r0 = *(at0 ? at0 : src);  // on their way while this pair of pairs is evaluated
       r1 = *(at1 ? at1 : src);
-      if (odd || n0.odd || n1.odd) {
-        acc = pse64_plain<Op>(p, a.src, i, n0.idx, acc);
-        if (two) acc = pse64_plain<Op>(p, a.src, i, n1.idx, acc);
+      if (!(regular(n0) && regular(n1))) {
+        one(n0);
+        if (two) one(n1);
         continue;
       }
-      const double x0 = tp.x - n0.x, y0 = tp.y - n0.y, z0 = Op::kDim == 3 ? tp.z - n0.z : 0.0;
-      const double x1 = tp.x - n1.x, y1 = tp.y - n1.y, z1 = Op::kDim == 3 ? tp.z - n1.z : 0.0;
-      const double q0 = Op::kDim == 3 ? fma(x0, x0, fma(y0, y0, z0 * z0)) : fma(x0, x0, y0 * y0);
-      const double q1 = Op::kDim == 3 ? fma(x1, x1, fma(y1, y1, z1 * z1)) : fma(x1, x1, y1 * y1);
-      const double w0 = pse64_kernel_value<Op::kPoly>(a, angle2<ANG>(q0) * a.c, powers);
-      const double w1 = pse64_kernel_value<Op::kPoly>(a, angle2<ANG>(q1) * a.c, powers);
-      Op::add(t, n0, x0, y0, z0, w0, acc);
+      const double3 d0 = offset(n0), d1 = offset(n1);
+      const double w0 = pse64_kernel_value<Op>(angle2<ANG>(squared(n0, d0, true)), a.c, powers);
+      const double w1 = pse64_kernel_value<Op>(angle2<ANG>(squared(n1, d1, true)), a.c, powers);
+      Op::add(t, n0, d0.x, d0.y, d0.z, w0, acc);
       Acc more = acc;
-      Op::add(t, n1, x1, y1, z1, w1, more);
+      Op::add(t, n1, d1.x, d1.y, d1.z, w1, more);
       if (two) acc = more;
     }
     held = 0;
@@ -578,13 +673,13 @@ __global__ void __launch_bounds__(32) pse64_sweep_kernel(typename Op::Params p, 
     __syncwarp();
   }
   evaluate();
-  if constexpr (S > 1) {  // the parts' sums
-    constexpr int NA = static_cast<int>(sizeof(Acc) / sizeof(double));
-    double* av = reinterpret_cast<double*>(&acc);
+  constexpr int NA = static_cast<int>(sizeof(Acc) / sizeof(double));
+  double* av = reinterpret_cast<double*>(&acc);
 #pragma unroll
-    for (int c = 0; c < NA; ++c)
+  for (int c = 0; c < NA; ++c) {
 #pragma unroll
-      for (int o = 1; o < S; o <<= 1) av[c] += __shfl_xor_sync(0xffffffffu, av[c], o);
+    for (int o = 1; o < S; o <<= 1) av[c] += __shfl_xor_sync(0xffffffffu, av[c], o);  // the parts' sums
+    if (!odd) av[c] = __dmul_rn(av[c], a.scale);
   }
   if (valid && lane % S == 0) Op::Plain::store(p, i, i - a.ib, acc);
 }

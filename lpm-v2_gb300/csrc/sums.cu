@@ -375,12 +375,13 @@ size_t rec_bytes(int kind, int mode) {
   if (mode == LPM_MODE_FP64) {
     if (kind == kSumBve || kind == kSumBveMesh) return sizeof(BveI64<0>::Rec);
     if (kind == kSumPlane) return sizeof(PlaneI64::Rec);
-    if (kind == kSumPseGrad || kind == kSumPseDiv || kind == kSumPseSphereDdot) return sizeof(PseGrad64::Rec);
+    if (kind == kSumPseGrad || kind == kSumPseDiv || kind == kSumPseSphereDdot) return sizeof(PseVecRec64);
+    if (kind == kSumPseK8Geo || kind == kSumPseInterpSphere) return sizeof(Pse64ScalarRec<true>);
     if (kind == kSumPsePlaneSecond || kind == kSumPsePlaneDdot) return sizeof(PlaneD464<PsePlaneSecondF64>::Rec);
     if (kind == kSumSwePlane || kind == kSumSweSphere) return sizeof(RecVec64);
     if (kind == kSumSphereStream || kind == kSumPlaneStream || kind == kSumBetaPlane || kind == kSumBetaStream)
       return sizeof(RecStream64);
-    return sizeof(PseLap64<kPseK8Geodesic>::Rec);  // the scalar PSE sums
+    return sizeof(Pse64ScalarRec<false>);  // the other scalar PSE sums
   }
   switch (kind) {
     case kSumBve:
@@ -850,12 +851,6 @@ int launch_pse_lap(const SumJob& job, const SumPlan& plan, int64_t npad) {
 }  // namespace
 
 namespace {
-// The PSE kernels over pi as polynomials in q = r^2 (times e^-q).
-constexpr double kK8[4] = {40.0, -40.0, 10.0, -2.0 / 3.0};      // bivariateLaplacianKernel8
-constexpr double kK1[4] = {-20.0, 20.0, -5.0, 1.0 / 3.0};       // bivariateFirstDerivativeKernel8
-constexpr double kDelta8[4] = {4.0, -6.0, 2.0, -1.0 / 6.0};     // bivariateDeltaKernel8
-constexpr double kGauss[4] = {4.0, 0.0, 0.0, 0.0};
-
 template <class Op, int S>
 void launch_pse64_sweep(const SumJob& job, int ang, const typename Op::Params& p, const Pse64Args& a,
                         const typename Op::Rec* recs) {
@@ -876,8 +871,7 @@ void launch_pse64_sweep(const SumJob& job, int ang, const typename Op::Params& p
 // An FP64 PSE sum (pse64.cuh): the targets' curve order, prep and sweep.  `over` divides the kernel
 // (the operator's powers of eps).
 template <class Op>
-int launch_pse64(const SumJob& job, const SumPlan& plan, const typename Op::Params& p, const double (&poly)[4],
-                 double over) {
+int launch_pse64(const SumJob& job, const SumPlan& plan, const typename Op::Params& p, double over) {
   using Rec = typename Op::Rec;
   const int64_t npad = plan.n_tiles * kPse64Tile;
   char* base = static_cast<char*>(job.src_buf);
@@ -893,13 +887,10 @@ int launch_pse64(const SumJob& job, const SumPlan& plan, const typename Op::Para
   Pse64Args a;
   int unit = 0;
   fp64_cutoff(job.kind, &unit);
-  const double per_s = std::log(2.0) / 256.0;  // q of one unit of s
   const double scale = unit ? job.radius / job.eps : 1.0 / job.eps;
-  a.c = scale * scale / per_s;
-  a.k0 = poly[0] / kPi / over;
-  a.k1 = poly[1] * per_s / kPi / over;
-  a.k2 = poly[2] * per_s * per_s / kPi / over;
-  a.k3 = poly[3] * per_s * per_s * per_s / kPi / over;
+  a.c = scale * scale;
+  a.unscale = kPi * over * (Op::kPoly ? 1.0 : 0.25);  // (the Gaussian's 4)
+  a.scale = 1.0 / a.unscale;
   a.reach = kPse64Reach * job.eps / (unit ? job.radius : 1.0);
   a.unit = unit;
   a.all_plain = unit && a.reach > kAngWideMax;
@@ -988,9 +979,9 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
       case kSumPseK8Chord: {
         const double eps2 = job.eps * job.eps;
         PseF64Params p{job.x, job.y, job.z, job.s1, job.eps, eps2, 1.0 / eps2, job.radius, job.out0};
-        if (job.kind == kSumPseK8Geo) return launch_pse64<PseLap64<kPseK8Geodesic>>(job, plan, p, kK8, eps2);
-        if (job.kind == kSumPseGaussChord) return launch_pse64<PseLap64<kPseGaussChord>>(job, plan, p, kGauss, eps2);
-        return launch_pse64<PseLap64<kPseK8Chord>>(job, plan, p, kK8, eps2);
+        if (job.kind == kSumPseK8Geo) return launch_pse64<PseLap64<kPseK8Geodesic>>(job, plan, p, eps2);
+        if (job.kind == kSumPseGaussChord) return launch_pse64<PseLap64<kPseGaussChord>>(job, plan, p, eps2);
+        return launch_pse64<PseLap64<kPseK8Chord>>(job, plan, p, eps2);
       }
       case kSumPseGrad:
       case kSumPseDiv: {
@@ -999,10 +990,10 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
                           job.eps * eps2, job.radius, 0.0, job.out0, job.out1, job.out2};
         if (job.kind == kSumPseGrad) {
           p.scale = 1.0 / eps2;  // MultiplyFieldByScalar(scalarGrad, 1/eps**2)
-          return launch_pse64<PseGrad64>(job, plan, p, kK1, eps2);
+          return launch_pse64<PseGrad64>(job, plan, p, eps2);
         }
         p.scale = 1.0 / job.eps;  // MultiplyFieldByScalar(divergence, 1/eps)
-        return launch_pse64<PseDiv64>(job, plan, p, kK1, job.eps * eps2);
+        return launch_pse64<PseDiv64>(job, plan, p, job.eps * eps2);
       }
       case kSumSphereStream:
       case kSumPlaneStream: {
@@ -1031,17 +1022,17 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
                           job.radius, job.radius2, 0.0, 1.0 / job.eps, job.out0, job.out1, job.out2, job.out3};
         switch (job.kind) {
           case kSumPsePlaneGrad:
-            return launch_pse64<PsePlaneGrad64>(job, plan, p, kK1, eps3);
+            return launch_pse64<PsePlaneGrad64>(job, plan, p, eps3);
           case kSumPseInterpPlane:
-            return launch_pse64<PseInterp64<false>>(job, plan, p, kDelta8, eps2);
+            return launch_pse64<PseInterp64<false>>(job, plan, p, eps2);
           case kSumPseInterpSphere:
-            return launch_pse64<PseInterp64<true>>(job, plan, p, kDelta8, eps2);
+            return launch_pse64<PseInterp64<true>>(job, plan, p, eps2);
           case kSumPsePlaneSecond:
-            return launch_pse64<PlaneD464<PsePlaneSecondF64>>(job, plan, p, kK1, eps3);
+            return launch_pse64<PlaneD464<PsePlaneSecondF64>>(job, plan, p, eps3);
           case kSumPsePlaneDdot:
-            return launch_pse64<PlaneD464<PsePlaneDdotF64>>(job, plan, p, kK1, eps3);
+            return launch_pse64<PlaneD464<PsePlaneDdotF64>>(job, plan, p, eps3);
           default:
-            return launch_pse64<PseSphereDdot64>(job, plan, p, kK1, eps3);
+            return launch_pse64<PseSphereDdot64>(job, plan, p, eps3);
         }
       }
       case kSumSwePlane:
