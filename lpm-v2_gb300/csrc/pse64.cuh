@@ -19,9 +19,10 @@
 // (1e-15 of the largest; its exp and atan2 are not CUDA's either): root mean square error against the sums in
 // extended precision, as a share of the reference expressions' own, at cubed nest 5: K8 0.58, gradient 0.60,
 // divergence 0.87; 0.57, 0.66 and 0.98 for particles 1e-7 off the sphere (pairs of rounded unit directions
-// and kernel polynomials in s, with rounded coefficients, gave 1.4 to 3 times the reference's error).  A lane's sum is in the reference's
-// ascending order; small target sets have up to 8 lanes per target, each summing its part of every
-// tile, and add the parts at the end.
+// and kernel polynomials in s, with rounded coefficients, gave 1.4 to 3 times the reference's error).  A lane's sum is in the
+// reference's ascending order; a target has 2 to 8 lanes, each summing its part of every tile, and adds the
+// parts at the end.  How many follows from the sources alone, so that a target's bits do not depend on
+// which other targets a call has.
 //
 // At r >= 7 each kernel (its polynomial times e^-49) is below 1e-14 of its peak, and the sum
 // leaves those pairs out:
@@ -520,12 +521,14 @@ __global__ void __launch_bounds__(32) pse64_sweep_kernel(typename Op::Params p, 
   const double inv = 1.0 / cp.r, inv2 = __dmul_rn(inv, inv);
   for (int e = lane; e < 256; e += 32) powers[e] = a.powers[e];
   tile_pipe_init(pp);  // (synchronises)
-  // the ball around the warp's targets (NaN or infinite: in reach of everything)
+  // The ball around the warp's targets (NaN or infinite: in reach of everything).  The lanes' own tests let
+  // a source pass at up to 1.00003 reach + 4e-6 of its tile's radius; no tile with such a source is left
+  // out, so that a target's sum does not depend on the warp it is in.
   const double wx = warp_sum(tp.x) / 32.0, wy = warp_sum(tp.y) / 32.0, wz = warp_sum(tp.z) / 32.0;
   double far = (tp.x - wx) * (tp.x - wx) + (tp.y - wy) * (tp.y - wy) + (tp.z - wz) * (tp.z - wz);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) far = fmax(far, __shfl_xor_sync(0xffffffffu, far, o));
-  const double wr = sqrt(far) * (1.0 + 1e-9) + 1e-9 * (fabs(wx) + fabs(wy) + fabs(wz)) + a.reach;
+  const double wr = sqrt(far) * (1.0 + 1e-9) + 1e-9 * (fabs(wx) + fabs(wy) + fabs(wz)) + a.reach * 1.00004;
 
   Acc acc{};
   // A pair's kernel value and terms.  `same`: both particles are as far from the sphere's centre.  The
@@ -623,7 +626,7 @@ __global__ void __launch_bounds__(32) pse64_sweep_kernel(typename Op::Params p, 
     bool in = tl < a.n_tiles;
     if (in) {
       const TileBall b = a.bounds[tl];
-      const double dx = wx - b.x, dy = wy - b.y, dz = wz - b.z, lim = wr + b.r;
+      const double dx = wx - b.x, dy = wy - b.y, dz = wz - b.z, lim = wr + b.r * 1.00001;
       in = !(dx * dx + dy * dy + dz * dz > lim * lim);
     }
     const unsigned m = __ballot_sync(0xffffffffu, in);

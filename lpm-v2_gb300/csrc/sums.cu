@@ -920,15 +920,20 @@ int launch_pse64(const SumJob& job, const SumPlan& plan, const typename Op::Para
   }, &a.tperm));
   pse64_prep_kernel<Op><<<static_cast<unsigned>(plan.n_tiles), kPse64Tile, 0, job.stream>>>(
       a.src, job.src_idx, job.ns, unit, recs, side, bounds, powers);
-  // Lanes per target: the fewest that put three warps on every scheduler, at most 8.  Measured at 1,
-  // 2, 4 and 8 lanes (K8, host call, ms): cubed nest 3 1.17, 0.63, 0.36, 0.25; nest 5 1.55, 1.24,
-  // 1.43, 1.26; nest 6 5.21, 4.44, 4.46, 4.60; nest 7 21.7, 21.6, 22.4, 23.7; quad nest 4 0.43, 0.36,
-  // 0.29, 0.27; nest 6 1.07, 1.20, 1.19, 1.25.  One warp can use a quarter of an SM's FP64 pipe.
-  int lanes = 1;
-  while (lanes < 8 && job.nt * lanes < 3 * plan.sm_count * 4 * 32) lanes *= 2;
-  if (lanes == 1) {
-    launch_pse64_sweep<Op, 1>(job, ang, p, a, recs);
-  } else if (lanes == 2) {
+  // Lanes per target, 2 to 8: the fewest that put three warps on every scheduler when the targets are the
+  // sources and as many particles again.  Measured at 1, 2, 4 and 8 lanes (K8, host call, ms): cubed nest 3
+  // 1.17, 0.63, 0.36, 0.25; nest 5 1.55, 1.24, 1.43, 1.26; nest 6 5.21, 4.44, 4.46, 4.60; nest 7 21.7, 21.6,
+  // 22.4, 23.7; quad nest 4 0.43, 0.36, 0.29, 0.27; nest 6 1.07, 1.20, 1.19, 1.25.  One warp can use a
+  // quarter of an SM's FP64 pipe.
+  // The rule counts sources, not targets, because the lanes' parts are what a target's sum is added up in:
+  // a rank's block of targets, or a batch of query points, gets the same bits as the whole set.  Counting
+  // targets was faster for the smallest blocks only (cubed nest 6, 1/4, 1/8 and 1/32 of the targets: 1.52,
+  // 0.97 and 0.52 ms against 1.54, 1.24 and 1.24).  One lane for the largest sets would be 3 to 6 % faster
+  // where the reach is short (quad nest 7 at eps 0.05 2.59 ms against 2.75) and 2 % slower for K8 at cubed
+  // nest 7, and its small blocks half as fast.
+  int lanes = 2;
+  while (lanes < 8 && 2 * job.ns * lanes < 3 * plan.sm_count * 4 * 32) lanes *= 2;
+  if (lanes == 2) {
     launch_pse64_sweep<Op, 2>(job, ang, p, a, recs);
   } else if (lanes == 4) {
     launch_pse64_sweep<Op, 4>(job, ang, p, a, recs);
