@@ -517,7 +517,8 @@ __device__ __forceinline__ GroupFrame sphere_group_frame(bool valid, const Split
   f.radius = sqrtf(rad) * 1.000001f;
   f.compact = f.radius <= compact_radius && f.radius <= BveRel::kCompactRatio * sqrtf(spc);
   // on the sphere: dropping every c_j moves q by <= 2^-30 h^2 relative to the smallest |d|^2
-  f.on_sphere = cm <= 9.313225746154785e-10f * spc;
+  // (a group of one source has no distance to compare with)
+  f.on_sphere = spc < 3.0e38f && cm <= 9.313225746154785e-10f * spc;
   return f;
 }
 
