@@ -10,7 +10,8 @@
 // pairs are counted as done.
 //
 // Layout: sources and targets in curve order.  A group of kGroup sources has an origin o near its
-// centroid; positions (unit directions for the great circle, x / a for the chord, x in the plane)
+// centroid (in the plane with a low part: far from the coordinates' origin a float alone would make every
+// group wide, and at a shift of 1e8 a sum at quad nest 7 took 3.9 ms instead of 0.5); positions (unit directions for the great circle, x / a for the chord, x in the plane)
 // are held relative to it.  A pair needs only the exponent's base-2 argument y = -r^2 log2 e:
 //   v = |t - s|^2 from the offsets (3 + 3 packed FP32x2 operations; 2 + 2 in the plane),
 //   y = v (q0 + q1 v + ...)     for the great circle, theta^2 = 4 asin^2(sqrt(v) / 2) as a polynomial
@@ -32,6 +33,7 @@
 
 #include "bve_rel.cuh"
 #include "ops.cuh"
+#include "plane_rel.cuh"
 #include "pse_rel.cuh"
 
 namespace lpm {
@@ -49,7 +51,7 @@ struct PseLap {
   };
   struct __align__(16) Group {
     float4 o;  // origin, R
-    float4 f;  // the field's group constant, 1 for a wide group
+    float4 f;  // the field's group constant, 1 for a wide group, the origin's low part (plane)
   };
   struct __align__(16) Tgt {
     float4 h;  // position, field: high parts
@@ -194,8 +196,8 @@ __global__ void __launch_bounds__(THREADS, MINB) pse_lap_sweep_kernel(PseLapArgs
       bool in[NP], near = false;
 #pragma unroll
       for (int p = 0; p < NP; ++p) {
-        tx[p] = rel1x2(xh[p], xl[p], o.o.x);
-        ty[p] = rel1x2(yh[p], yl[p], o.o.y);
+        tx[p] = SPHERE ? rel1x2(xh[p], xl[p], o.o.x) : rel1x2(xh[p], xl[p], o.o.x, o.f.z);
+        ty[p] = SPHERE ? rel1x2(yh[p], yl[p], o.o.y) : rel1x2(yh[p], yl[p], o.o.y, o.f.w);
         tz[p] = SPHERE ? rel1x2(zh[p], zl[p], o.o.z) : make_float2(0.f, 0.f);
         float2 n2 = __ffma2_rn(ty[p], ty[p], __fmul2_rn(tx[p], tx[p]));
         if (SPHERE) n2 = __ffma2_rn(tz[p], tz[p], n2);
@@ -230,9 +232,14 @@ __global__ void __launch_bounds__(THREADS, MINB) pse_lap_sweep_kernel(PseLapArgs
       float2 ux[NP], uy[NP], uz[NP];
 #pragma unroll
       for (int p = 0; p < NP; ++p) {
-        rel2x2(xh[p], xl[p], o.o.x, tx[p], ux[p]);
-        rel2x2(yh[p], yl[p], o.o.y, ty[p], uy[p]);
-        if (SPHERE) rel2x2(zh[p], zl[p], o.o.z, tz[p], uz[p]);
+        if (SPHERE) {
+          rel2x2(xh[p], xl[p], o.o.x, tx[p], ux[p]);
+          rel2x2(yh[p], yl[p], o.o.y, ty[p], uy[p]);
+          rel2x2(zh[p], zl[p], o.o.z, tz[p], uz[p]);
+        } else {
+          rel2x2(xh[p], xl[p], o.o.x, o.f.z, tx[p], ux[p]);
+          rel2x2(yh[p], yl[p], o.o.y, o.f.w, ty[p], uy[p]);
+        }
       }
       for (int j = 0; j < G; ++j) {
         const float4 ra = gr[j].a, rb = gr[j].b, rc = gr[j].c, rd = gr[j].d;
@@ -272,6 +279,46 @@ __global__ void __launch_bounds__(THREADS, MINB) pse_lap_sweep_kernel(PseLapArgs
           static_cast<double>(h ? hs[p].y : hs[p].x) + static_cast<double>(h ? ls[p].y : ls[p].x);
     }
   }
+}
+
+// The frame of a warp's group of 32 planar sources: the centroid with its low part (planar sets lie
+// anywhere, and a float origin is off by half the float spacing there), and the radius about it.  The mean
+// is taken of the offsets from the first source.
+struct PlaneFrame {
+  float o[2], ol[2];
+  float radius;
+};
+
+__device__ __forceinline__ PlaneFrame plane_group_frame(bool valid, const SplitPoint& sp) {
+  PlaneFrame f;
+  float d[2], n = valid ? 1.f : 0.f;
+  double first[2];
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    const float h0 = __shfl_sync(0xffffffffu, sp.h[c], 0), l0 = __shfl_sync(0xffffffffu, sp.l[c], 0);
+    first[c] = static_cast<double>(h0) + static_cast<double>(l0);
+    d[c] = valid ? __fadd_rn(__fadd_rn(sp.h[c], -h0), __fadd_rn(sp.l[c], -l0)) : 0.f;
+  }
+  float m[2] = {d[0], d[1]};
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    m[0] += __shfl_xor_sync(0xffffffffu, m[0], o);
+    m[1] += __shfl_xor_sync(0xffffffffu, m[1], o);
+    n += __shfl_xor_sync(0xffffffffu, n, o);
+  }
+  const float inv = n > 0.f ? 1.f / n : 0.f;
+  float r = 0.f;
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    split2(first[c] + static_cast<double>(m[c] * inv), f.o[c], f.ol[c]);
+    const float e = valid ? __fadd_rn(__fadd_rn(sp.h[c], -f.o[c]), __fadd_rn(sp.l[c], -f.ol[c])) : 0.f;
+    r += e * e;
+  }
+  if (!(r == r)) r = __int_as_float(0x7f800000);  // a NaN source: an infinite radius
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) r = fmaxf(r, __shfl_xor_sync(0xffffffffu, r, o));
+  f.radius = sqrtf(r) * 1.000001f;
+  return f;
 }
 
 // Records, groups and balls of the sorted sources (CTA t < n_tiles: tile t, TILE threads, every thread
@@ -315,13 +362,27 @@ __global__ void __launch_bounds__(TILE) pse_lap_prep_kernel(const double* x, con
     sp = position(j);
     split2(f[j], fh, fl);
   }
-  const GroupFrame fr = sphere_group_frame<TILE, G>(valid, sp, 0.0);
+  float og[3] = {0.f, 0.f, 0.f}, ogl[2] = {0.f, 0.f}, radius;  // the group's origin and radius
+  if constexpr (SPHERE) {
+    const GroupFrame fr = sphere_group_frame<TILE, G>(valid, sp, 0.0);
+    for (int c = 0; c < 3; ++c) og[c] = fr.o[c];
+    radius = fr.radius;
+  } else {
+    const PlaneFrame fr = plane_group_frame(valid, sp);
+    for (int c = 0; c < 2; ++c) og[c] = fr.o[c], ogl[c] = fr.ol[c];
+    radius = fr.radius;
+  }
   const float fg = __shfl_sync(0xffffffffu, fh, 0);  // the first source's field
   PseLap::Rec r;
   if (valid) {
-    float hi[3], lo[3];
+    float hi[3] = {0.f, 0.f, 0.f}, lo[3] = {0.f, 0.f, 0.f};
+    if constexpr (SPHERE) {
 #pragma unroll
-    for (int c = 0; c < 3; ++c) rel2(sp.h[c], sp.l[c], fr.o[c], hi[c], lo[c]);
+      for (int c = 0; c < 3; ++c) rel2(sp.h[c], sp.l[c], og[c], hi[c], lo[c]);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 2; ++c) rel2(sp.h[c], sp.l[c], og[c], ogl[c], hi[c], lo[c]);
+    }
     const float ar = __double2float_rn(area[j]);
     // f_j - f_g = fs + fe, fs rounded from all of it: the low part of f_j is the whole of F_j where f_j and f_g
     // round to the same float (every group of a field with a large mean, and a group's first source)
@@ -340,8 +401,8 @@ __global__ void __launch_bounds__(TILE) pse_lap_prep_kernel(const double* x, con
   __shared__ float4 ball[GPT];  // the groups' balls for the tile's ball (w < 0: empty group)
   if (threadIdx.x % G == 0) {
     PseLap::Group o;
-    o.o = make_float4(fr.o[0], fr.o[1], fr.o[2], fr.radius);
-    o.f = make_float4(fg, fr.radius > PseLap::kWide * c_cut ? 1.f : 0.f, 0.f, 0.f);
+    o.o = make_float4(og[0], og[1], og[2], radius);
+    o.f = make_float4(fg, radius > PseLap::kWide * c_cut ? 1.f : 0.f, ogl[0], ogl[1]);
     grp[t * GPT + threadIdx.x / G] = o;
     ball[threadIdx.x / G] = valid ? o.o : make_float4(0.f, 0.f, 0.f, -1.f);
   }
