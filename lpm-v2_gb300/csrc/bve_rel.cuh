@@ -15,9 +15,8 @@
 //    exactly the operations of the sources, and d = (t_hi - s_hi) + (t_lo - s_lo) keeps ~48
 //    bits; a self pair cancels bit for bit.
 // A compact group (R <= a/2 and R <= 32 x its smallest spacing h, i.e. a patch of a
-// quasi-uniform point set) takes the far form for every target: the group record carries
-// R = 0, and its records use rel2_fast, the target's far-form operations, so a self pair
-// still cancels bit for bit.  For a target near such a group the roundings are an absolute
+// quasi-uniform point set) takes one-subtraction differences for every target: its records use
+// rel2_fast, the target's far-form operations, so a self pair still cancels bit for bit.  For a target near such a group the roundings are an absolute
 // 2^-24 R inside the near-field sum sum_j S_j / |d_j|^2, which grows only like ln(1/h) on a
 // quasi-uniform set, so the velocity error scales with R, not R/h (1.0e-7 relative at
 // icosahedral nest 8).  Groups that fail the test (clustered or sparse points) keep the
@@ -29,7 +28,7 @@
 // fma(dz,dz, fma(dy,dy, fma(dx,dx, -c_i))), one operation less per pair.
 // Then  q = |d|^2 - c_i - c_j,  w = S_j / q,  D += w d  with c = |p|^2 - 1 and
 // S_j = -zeta_j A_j / (2 pi a) as in BveF32; u = D x p_i in FP64.
-// A group whose warp is far (every target at |t - o| >= 3R, 1.5R if it is compact) takes the
+// A group whose warp is far (every target at |t - o| >= 3R, 1.5R or 1.25R if it is compact) takes the
 // expanded form in a basis (o, e1, e2) of the group, e1 and e2 about orthonormal to o: with the
 // source p_j = (1 + c) o + a e1 + b e2 and h = q/2 = 1 - p_i.p_j,
 //   h = C - c gamma - a alpha - b beta,   alpha = p_i.e1, beta = p_i.e2, gamma = p_i.o, C = 1 - gamma,
@@ -85,6 +84,9 @@ struct BveRel {
   // and R <= kCompactRatio h: refined meshes have R / h of 10-18 (median 12), sets without an even spacing
   // 44 and more (their closest pairs are rarely consecutive, so h alone does not show them)
   static constexpr float kCompactRatio = 32.0f;
+  // the far form of a compact group starts at kCompactFar R, of a small one (R <= kCompactSmall; from
+  // icosahedral nest 6 on) at kCompactFarSmall R
+  static constexpr float kCompactFar = 1.5f, kCompactFarSmall = 1.25f, kCompactSmall = 0.2f;
 };
 
 // Offset of a hi/lo value from a float origin, rounded once: fl(p - o) to ~2^-24 relative
@@ -673,13 +675,15 @@ __device__ __forceinline__ void bve_rel_prep_tile(const double* x, const double*
   if (threadIdx.x % BveRel::kGroup == 0) {
     BveRel::Group g;
     g.o = group_origin(f);
-    // The sign marks a compact group, whose far form starts at 1.5 R: there |h| >= R^2 / 8 and the
-    // expanded form's roundings are at most about 20 x 2^-24 of it, at the nearest of the group's
-    // sources alone, while the difference form near a compact group carries an absolute 2^-24 R
-    // in d for all of them.  Measured at icosahedral nests 5, 6, 7 against FP64 (relative L2 of the
-    // velocity): 1.86e-7, 8.60e-8, 4.95e-8 from 3 R on, 1.73e-7, 7.95e-8, 4.65e-8 from 1.5 R on, and
-    // 3, 3 and 1 % faster.
-    g.o.hi.w = f.compact ? -near_radius(0.5f * f.radius, b) : near_radius(f.radius, b);
+    // The sign marks a compact group, whose far form starts at kCompactFar R, or kCompactFarSmall R if it is
+    // small: there |h| >= R^2 / 8 (R^2 / 32), and the expanded form's roundings are at most about 20 (60) x 2^-24
+    // of it, at the nearest of the group's sources alone, while the difference form near a compact group
+    // carries an absolute 2^-24 R in d for all of them.  Relative L2 error of the velocity against FP64 over
+    // all targets, two fields, with the far form from 3 R, 1.5 R and 1.25 R on: icosahedral nest 6 12.0e-8, 11.1e-8,
+    // 10.9e-8; nest 7 6.26e-8, 5.86e-8, 5.77e-8; nest 8 3.69e-8, 3.51e-8, 3.46e-8; at nest 4, whose groups
+    // are not small, 17.3e-8 and 17.5e-8.  1.5 R is 3 % faster than 3 R at nests 5 and 6, 1.25 R no faster.
+    const float from = f.radius <= BveRel::kCompactSmall ? BveRel::kCompactFarSmall : BveRel::kCompactFar;
+    g.o.hi.w = f.compact ? -near_radius(from / BveRel::kNearFactor * f.radius, b) : near_radius(f.radius, b);
     if (b.singular) g.o.hi.w = 1e15f;             // near every target
     g.o.lo.x = b.k;
     g.o.lo.y = 1.f - b.k;  // |o|^2 + k
