@@ -49,7 +49,7 @@ struct BetaRelArgs {
   const double *x, *y;
   const BetaRel::Rec* src;
   const BetaRel::Origin* org;
-  int64_t n_tiles, tiles_per_chunk, ib, nt;
+  int64_t n_tiles, ib, nt;
   double* partial;  // [chunk][2][nt]
   int* status;
 };
@@ -331,7 +331,7 @@ struct BetaStreamRelArgs {
   const double *x, *y;
   const BetaStreamRel::Rec* src;
   const BetaStreamRel::Origin* org;
-  int64_t n_tiles, tiles_per_chunk, ib, nt;
+  int64_t n_tiles, ib, nt;
   double* partial;  // [chunk][2][nt]
   int* status;
 };

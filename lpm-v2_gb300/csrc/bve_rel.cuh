@@ -22,7 +22,7 @@
 // icosahedral nest 8).  Groups that fail the test (clustered or sparse points) keep the
 // near/far choice, whose error bound holds for any point distribution.
 // Particle order along the mesh or the curve keeps a warp's targets close together, so a
-// warp meets few near groups (at icosahedral nest 8 about one group in a thousand).
+// warp meets few near groups (at icosahedral nest 8 three in a thousand).
 // A group whose sources all lie on the sphere to within |c_j| <= 2^-30 h^2 (h its smallest
 // spacing; always the case once positions are renormalised) drops c_j: q is then
 // fma(dz,dz, fma(dy,dy, fma(dx,dx, -c_i))), one operation less per pair.
@@ -129,8 +129,9 @@ __device__ __forceinline__ void rel2x2(float2 ph, float2 pl, float oh, float2& r
 }
 
 // The place in its CTA's block of a thread's m-th target of TPT: a warp holds 32 TPT consecutive
-// targets, which are close together in a mesh's order, so that it meets fewer near groups (38.6 %
-// of the groups at icosahedral nest 5 where 32-runs spread over the block met 45 %).
+// targets, which are close together in a mesh's order, so that it meets fewer near groups (by count, for
+// 6 targets a thread, 17 % of the groups at icosahedral nest 5 and 4.8 % at nest 6, where 32-runs spread over the block
+// would meet 24 % and 6.9 %).
 template <int TPT>
 __device__ __forceinline__ int bve_target(int m) {
   return static_cast<int>(threadIdx.x >> 5) * (32 * TPT) + m * 32 + static_cast<int>(threadIdx.x & 31u);
@@ -538,7 +539,8 @@ __device__ __forceinline__ void group_offsets(const GroupFrame& f, const SplitPo
   }
 }
 
-// The group record: centroid, radius (0 for a compact group: never near), on-sphere flag.
+// The group record: origin, radius (0 for a compact group; the sweeps that have a near form for compact
+// groups put its near radius there, negative), on-sphere flag.
 __device__ __forceinline__ BveRel::Origin group_origin(const GroupFrame& f) {
   BveRel::Origin o;
   o.hi = make_float4(f.o[0], f.o[1], f.o[2], f.compact ? 0.f : f.radius);

@@ -386,7 +386,7 @@ struct SweepArgs {
   typename Op::Params p;
   const typename Op::Rec* src;  // padded to n_tiles * TILE records
   int64_t n_tiles;
-  int64_t tiles_per_chunk;
+  int64_t tiles_per_chunk = 0;  // of a sweep over consecutive chunks (bve_x2.cuh)
   int64_t ib;         // first target (0-based particle index)
   int64_t nt;         // number of targets
   double* partial;    // [gridDim.y][Op::NC][nt]

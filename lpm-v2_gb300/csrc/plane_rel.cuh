@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(THREADS, MINB) plane_rel_sweep_kernel(PlaneRel
       }
       // the group's terms are summed on their own and then added to the tile's: a running
       // FP32 sum of a whole tile's terms (both signs, e.g. the two lobes of a dipole) rounds
-      // at the size of the tile's partial sum 256 times, a group sum only 64 times
+      // at the size of the tile's partial sum 256 times, a group sum only 128 times
       float2 gu[NP], gv[NP];
 #pragma unroll
       for (int p = 0; p < NP; ++p) gu[p] = gv[p] = make_float2(0.f, 0.f);

@@ -65,7 +65,7 @@ struct PseRelArgs {
   float half_a2;  // a^2 / 2 (divergence: P d = d - (a^2 |d|^2 / 2) p_i)
   const PseRel::Rec* src;
   const BveRel::Origin* org;  // hi.w: near radius (0 for a compact group), lo.w: group radius
-  int64_t n_tiles, tiles_per_chunk, ib, nt;
+  int64_t n_tiles, ib, nt;
   // targets in curve order: position k of the sweep is particle tperm[k] (nullptr: ib + k);
   // partial sums are stored at the particle's own place, (tperm[k] - ib)
   const int32_t* tperm;
@@ -96,17 +96,16 @@ __device__ __forceinline__ void pse_position(const double* x, const double* y, c
 
 template <int ANG>
 __device__ __forceinline__ float2 pse_r2(float2 v, float2 ks2) {
+  static_assert(ANG != kPseAngleChord, "the chord's sums are pse_lap.cuh's");
   if (ANG == kPseAngleSeries) {
     float2 sr = __ffma2_rn(v, make_float2(3.1746032e-4f, 3.1746032e-4f), make_float2(1.7857143e-3f, 1.7857143e-3f));
     sr = __ffma2_rn(sr, v, make_float2(1.1111111e-2f, 1.1111111e-2f));
     sr = __ffma2_rn(sr, v, make_float2(8.3333336e-2f, 8.3333336e-2f));
     sr = __ffma2_rn(sr, v, make_float2(1.0f, 1.0f));
     return __fmul2_rn(__fmul2_rn(v, ks2), sr);
-  } else if (ANG == kPseAngleAsin) {
+  } else {
     const float h0 = asinf(fminf(0.5f * sqrtf(v.x), 1.0f)), h1 = asinf(fminf(0.5f * sqrtf(v.y), 1.0f));
     return __fmul2_rn(make_float2(4.0f * h0 * h0, 4.0f * h1 * h1), ks2);
-  } else {
-    return __fmul2_rn(v, ks2);
   }
 }
 

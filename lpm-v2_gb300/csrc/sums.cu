@@ -496,7 +496,13 @@ namespace {
 // (near groups), and a fifth of a 256-source tile of 512 targets per CTA.  More than one round is better
 // than one exactly full: BVE sums of 50,000, 100,000 and 150,000 points took 0.98, 2.62 and 5.32 ms at
 // 3.9 CTAs per SM (one round, as choose_split has it) and 0.89, 2.47 and 5.13 ms at 15 to 23.  At most
-// 256 CTAs per SM, which bounds the partial sums (64 was 1.3 % slower for the plane at quad nest 8).  Ties (0.5 %) go to the smaller split.
+// 256 CTAs per SM (64 was 1.3 % slower for the plane at quad nest 8), which bounds the partial sums: 256 x SMs x a CTA's targets x
+// components doubles, on 152 SMs at most 0.72 GB for the BVE, 0.48 for the sphere stream functions, 0.32 for
+// the plane, 0.64 and 1.1 for the SWE integrals of plane and sphere (330 MB at icosahedral nest 8, 91 MB at
+// 100,003 points).  The finish kernel's reads of them are not in the model: calls for 1 to 1,500 targets of nest 8 took
+// what they took with a few hundred chunks (0.97 to 1.00 of it).  The constants are from the BVE; the beta plane gained
+// as much (quad nests 6 and 7 0.99 -> 0.75 and 5.37 -> 4.80 ms, whole sets), the sphere SWE less (5,000 targets of
+// nest 7 3.14 -> 2.75 ms).  Ties (0.5 %) go to the smaller split.
 int64_t choose_interleaved_split(int64_t blocks, int64_t tiles, int64_t sms, int64_t per_sm, int64_t tile_pairs) {
   if (blocks < 1) blocks = 1;
   int64_t lim = std::max<int64_t>(256 * sms / blocks, 1);
@@ -617,11 +623,10 @@ SumPlan plan_sum(int kind, int mode, int64_t ns, int64_t nt, int sm_count, int s
     pl.sm_count = sms;
     pl.fp64_threads = fp64_block_threads(nt, sms);
     pl.nsplit = 1;
-    pl.tiles_per_chunk = pl.n_tiles;
     pl.partial_bytes = 0;
     return pl;
   }
-  // Split the source range so that the last wave of CTAs is nearly full.
+  // Split the source tiles among the CTAs of a target block.
   const int64_t tblocks = ceil_div(nt, targets_per_cta(kind, shape));
   const int minb = (kind == kSumBve || kind == kSumBveMesh)          ? kBveShapes[shape].minb
                    : kind == kSumSwePlane                            ? kSweMinB
@@ -632,21 +637,18 @@ SumPlan plan_sum(int kind, int mode, int64_t ns, int64_t nt, int sm_count, int s
   if (mode == LPM_MODE_FP32C && pse_culls_tiles(kind)) {
     // every CTA scans the whole source range for its in-reach tiles and takes one of nsplit
     // equal shares of them
-    pl.tiles_per_chunk = pl.n_tiles;
     pl.nsplit = cull_shares(tblocks, slots);
   } else {
     const bool bve = kind == kSumBve || kind == kSumBveMesh;
     const int64_t tiles = bve ? pl.n_tiles * (kBveTile / kBveShapes[shape].tile) : pl.n_tiles;
     pl.nsplit = choose_interleaved_split(
         tblocks, tiles, slots / minb, minb, (bve ? kBveShapes[shape].tile : tile) * targets_per_cta(kind, shape));
-    pl.tiles_per_chunk = ceil_div(tiles, pl.nsplit);
   }
   pl.partial_bytes = static_cast<size_t>(pl.nsplit) * comps_of(kind) * nt * sizeof(double);
   if (kind == kSumSwePlane || kind == kSumSweSphere) {
     // the surface-height Laplacian: the K8 PSE sweep (planar or geodesic), after the velocity sweep
     const SumPlan pp = plan_sum(kind == kSumSwePlane ? kSumPseK8Chord : kSumPseK8Geo, mode, ns, nt, sm_count, 0);
     pl.aux_n_tiles = pp.n_tiles;
-    pl.aux_tiles_per_chunk = pp.tiles_per_chunk;
     pl.aux_nsplit = pp.nsplit;
     pl.aux_tgt_offset = pp.tgt_offset;
     pl.aux_src_offset = align_up(pl.src_bytes, 256);
@@ -741,7 +743,6 @@ int launch_pse_rel(const SumJob& job, const SumPlan& plan, int64_t npad) {
       reinterpret_cast<const char*>(a.org) +
       align_up(static_cast<size_t>(plan.n_tiles) * (tile / PseRel::kGroup) * sizeof(BveRel::Origin), 256));
   a.n_tiles = plan.n_tiles;
-  a.tiles_per_chunk = plan.tiles_per_chunk;
   a.ib = job.ib;
   a.nt = job.nt;
   a.partial = job.partial;
@@ -1107,7 +1108,6 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
       a.p = BveF32::Params{job.x, job.y, job.z, inv_a};
       a.src = reinterpret_cast<const BveF32::Rec*>(job.src_buf);
       a.n_tiles = plan.n_tiles;
-      a.tiles_per_chunk = plan.tiles_per_chunk;
       a.ib = job.ib;
       a.nt = job.nt;
       a.partial = job.partial;
@@ -1211,7 +1211,6 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
       a.p = BveF32::Params{job.x, job.y, job.z, inv_a};
       a.src = nullptr;
       a.n_tiles = plan.n_tiles;
-      a.tiles_per_chunk = plan.tiles_per_chunk;
       a.ib = job.ib;
       a.nt = job.nt;
       a.partial = job.partial;
@@ -1275,7 +1274,6 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
       a.src = recs;
       a.org = org;
       a.n_tiles = plan.n_tiles;
-      a.tiles_per_chunk = plan.tiles_per_chunk;
       a.ib = job.ib;
       a.nt = job.nt;
       a.partial = job.partial;
@@ -1305,7 +1303,6 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
       SweepArgs<BveF32> a;
       a.p = BveF32::Params{job.x, job.y, job.z, inv_a};
       a.n_tiles = plan.n_tiles;
-      a.tiles_per_chunk = plan.tiles_per_chunk;
       a.ib = job.ib;
       a.nt = job.nt;
       a.partial = job.partial;
@@ -1327,7 +1324,6 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
       jp.src_buf = static_cast<char*>(job.src_buf) + plan.aux_src_offset;
       SumPlan pp;
       pp.n_tiles = plan.aux_n_tiles;
-      pp.tiles_per_chunk = plan.aux_tiles_per_chunk;
       pp.nsplit = plan.aux_nsplit;
       pp.tgt_offset = plan.aux_tgt_offset;
       LPM_TRY(launch_pse_lap(jp, pp, plan.aux_n_tiles * kPseTile));
@@ -1353,7 +1349,6 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
       a.src = recs;
       a.org = org;
       a.n_tiles = plan.n_tiles;
-      a.tiles_per_chunk = plan.tiles_per_chunk;
       a.ib = job.ib;
       a.nt = job.nt;
       a.partial = job.partial;
@@ -1405,7 +1400,6 @@ int launch_sum(const SumJob& job, const SumPlan& plan) {
       jp.src_buf = static_cast<char*>(job.src_buf) + plan.aux_src_offset;
       SumPlan pp;
       pp.n_tiles = plan.aux_n_tiles;
-      pp.tiles_per_chunk = plan.aux_tiles_per_chunk;
       pp.nsplit = plan.aux_nsplit;
       pp.tgt_offset = plan.aux_tgt_offset;
       LPM_TRY(launch_pse_lap(jp, pp, plan.aux_n_tiles * kPseTile));

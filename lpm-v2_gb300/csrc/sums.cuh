@@ -11,7 +11,6 @@ namespace lpm {
 // partial sums (FP32C only).
 struct SumPlan {
   int64_t n_tiles = 0;       // source tiles (ns padded to a tile multiple)
-  int64_t tiles_per_chunk = 0;
   int64_t nsplit = 1;        // split-K chunks (gridDim.y)
   size_t src_bytes = 0;      // bytes of the padded source-record array
   size_t partial_bytes = 0;  // bytes of the FP64 partial sums
@@ -20,7 +19,7 @@ struct SumPlan {
   int64_t sm_count = 152;    // SMs the FP64 sweeps are laid out for
   // a second sweep of the same job (the planar SWE surface-height Laplacian): its tiles and
   // split, its source records at src_buf + aux_src_offset; it reuses the partials
-  int64_t aux_n_tiles = 0, aux_tiles_per_chunk = 0, aux_nsplit = 0;
+  int64_t aux_n_tiles = 0, aux_nsplit = 0;
   size_t aux_src_offset = 0, aux_tgt_offset = 0;
   // FP32C PSE sums: the targets' curve order (two lists of nt int32: [ib, ib + nt) and its
   // sorted permutation) at src_buf + tperm_offset; 0 when the sweep takes targets in order
