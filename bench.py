@@ -16,8 +16,9 @@ Metric: Ginteractions/s (interactions = N_targets * N_sources - self pairs per s
   e2e   : the same steps through the C ABI with the state copied from pinned host memory
           before and back after every step (lpm_bve_set_state / lpm_bve_timestep /
           lpm_bve_get_state), timed with CUDA events on the same stream
-  roofline: the velocity-sum kernels against the measured FP32 FMA peak (24 flops/pair),
-          with the sweep's recorded ncu pipe utilisation beside the contract fraction
+  roofline: the velocity-sum kernels against the measured FP32 FMA peak, by the 12 flops a pair that
+          they execute (the reference's expressions have 24: contract_tflops), with the sweep's
+          recorded ncu pipe utilisation
   accuracy: the FP32C velocity at the final state against the oracle (FP64) on a target block
   fp64_gpu: the plain FP64 GPU kernel (parity mode) on the same state, on a block of targets
           that fills every SM, and the FP32C/FP64 ratio
@@ -54,20 +55,26 @@ UNIT = "Ginteractions/s"
 # the PSE operators that have an FP64 form only (their FP32C form would be ill-conditioned):
 # --workload sum runs them in FP64 whatever --mode says
 FP64_ONLY_SUMS = ("pse_plane_grad", "pse_plane_second", "pse_plane_ddot", "pse_sphere_ddot", "pse_interp")
-FLOPS_PER_INTERACTION = 24  # dot 5, a^2-dot 1, x4pi a 1, zeta A/den 2, cross 9, accumulate 6
+FLOPS_PER_INTERACTION = 24  # the reference's: dot 5, a^2-dot 1, x4pi a 1, zeta A/den 2, cross 9, accumulate 6
+# what the FP32C sweep executes for a pair of a far group (csrc/bve_rel.cuh): six FMAs, and one reciprocal
+EXECUTED_FLOPS_PER_INTERACTION = 12
+# FP64 instructions a pair of the FP64 sweep (its products and divisions run on the integer pipes): ncu
+# sm__inst_executed_pipe_fp64 x 32 lanes over the pairs, recorded at icos nest 4 (13,183,344 for 3.93e7 pairs)
+FP64_INSTRUCTIONS_PER_INTERACTION = 10.7
 L2_FLUSH_BYTES = 256 << 20
 # DRAM bytes (ncu dram__bytes_read.sum + dram__bytes_write.sum) of one full-size icos nest 8
 # sweep launch, from a single-pass ncu capture of this benchmark's own step (ncu cannot run
 # inside the timed region, so this is a recorded constant, not a figure of this run)
-SWEEP_TRAFFIC_ICOS8 = 357_470_000 + 131_950_000
+SWEEP_TRAFFIC_ICOS8 = 567_180_000 + 307_200_000
+SWEEP_TRAFFIC_GRID = "2561 x 7 CTAs of 128 threads"
 # Pipe utilisation of the same sweep kernel (ncu of bve_rel_sweep_kernel<128,6,256,3>,
 # the autotuner's shape, on this workload at icos nest 7, one launch): the pipe-level counterpart
-# of the flop-contract fraction; recorded constants, not figures of this run
-SWEEP_PIPES_ICOS7 = {"fma_pipe_active": 0.5786, "xu_pipe_active": 0.7248, "issue_active": 0.4589}
+# of the executed-flops fraction; recorded constants, not figures of this run
+SWEEP_PIPES_ICOS7 = {"fma_pipe_active": 0.5781, "xu_pipe_active": 0.7308, "issue_active": 0.4590}
 # FP32 CUDA-core nominal peak: 152 SMs x 128 lanes x 2 flops per FMA, per MHz of SM clock
 FP32_NOMINAL_TFLOPS_PER_MHZ = 152 * 128 * 2 / 1e6
-# FP64: 2 DFMA per clock per SM (4 flops), per MHz
-FP64_NOMINAL_TFLOPS_PER_MHZ = 152 * 4 / 1e6
+# FP64: 2 instructions per clock per SM (lanes), in Ginstructions/s per MHz
+FP64_NOMINAL_GINST_PER_MHZ = 152 * 2 / 1e3
 # FP64 parity-mode rate at the headline size: the FP64 sweep on a block of targets that gives
 # every SM two 128-thread CTAs (the per-target cost is the same for every target)
 FP64_BLOCK_TARGETS = 152 * 2 * 128
@@ -302,7 +309,7 @@ def run_ours(args):
     # velocity-sum kernels: events around each sum inside the graph
     sums = 4 * args.steps
     sum_ms = (k_ms1 - k_ms0) / sums
-    achieved_tflops = FLOPS_PER_INTERACTION * per_sum / (sum_ms * 1e-3) / 1e12
+    achieved_tflops = EXECUTED_FLOPS_PER_INTERACTION * per_sum / (sum_ms * 1e-3) / 1e12
 
     # ---------------- accuracy of the FP32C velocity at the final state against the oracle
     # (the reference loop restated in C, FP64) on a seeded block of targets
@@ -333,7 +340,7 @@ def run_ours(args):
         mhz = clocks.get("sm_mhz") or 2070.0
         fp64 = {"value": r64, "unit": UNIT, "fp32c_over_fp64": value / r64,
                 "contract_tflops": FLOPS_PER_INTERACTION * r64 / 1e3,
-                "frac_of_nominal_fp64_peak": FLOPS_PER_INTERACTION * r64 / 1e3 / (FP64_NOMINAL_TFLOPS_PER_MHZ * mhz),
+                "frac_of_nominal_fp64_peak": FP64_INSTRUCTIONS_PER_INTERACTION * r64 / (FP64_NOMINAL_GINST_PER_MHZ * mhz),
                 "kernel": "seq_i64_kernel<BveI64<0>> (four lanes per target, sources in ascending order, "
                           "bit-identical to the oracle)",
                 "sample": f"targets {b64}..{b64 + m64 - 1} against all {ns} sources ({inter64:.3e} interactions), "
@@ -398,12 +405,15 @@ def run_ours(args):
                                                                                             or 2070.0)),
                          "traffic": SWEEP_TRAFFIC_ICOS8 if args.nest == 8 else None,
                          "traffic_unit": "bytes per sweep launch: ncu dram__bytes_read.sum + dram__bytes_write.sum "
-                                         "of one full-size launch (a recorded capture, not measured in this run)",
+                                         "of one full-size launch (a recorded capture, not measured in this run), "
+                                         "grid " + SWEEP_TRAFFIC_GRID,
                          "pipes": dict(SWEEP_PIPES_ICOS7, source="ncu of the same sweep kernel on this "
                                        "workload at icos nest 7 (sm__pipe_fma_cycles_active, "
                                        "sm__pipe_xu_cycles_active, smsp__issue_active; recorded, not this run)"),
                          "kernel": "bve_rel_sweep_kernel (+ its prep and finish kernels) per velocity sum",
-                         "ms_per_launch": sum_ms, "flops_per_interaction": FLOPS_PER_INTERACTION,
+                         "ms_per_launch": sum_ms, "flops_per_interaction": EXECUTED_FLOPS_PER_INTERACTION,
+                         "contract_flops_per_interaction": FLOPS_PER_INTERACTION,
+                         "contract_tflops": achieved_tflops * FLOPS_PER_INTERACTION / EXECUTED_FLOPS_PER_INTERACTION,
                          "peak_source": "measured in-process FFMA loop (lpm_measure_fp32_peak); "
                                         "frac_of_nominal: 152 SMs x 128 lanes x 2 flops x the median SM clock"},
             "fp64_gpu": fp64,

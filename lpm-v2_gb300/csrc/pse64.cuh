@@ -39,7 +39,8 @@
 // whose particles differ by more than a quarter in their distance from the centre, takes the reference's
 // expressions as they stand (Op::Plain), as do all pairs of a reach beyond the polynomials' range.
 //
-// Bound by the FP64 pipe (2 lanes per clock per SM): 73-77 % busy at cubed nest 6, the rest being
+// Bound by the FP64 pipe (2 lanes per clock per SM): 74 % busy for K8 and 70 % for the
+// gradient at cubed nest 6, the rest being
 // the last warps of an SM.  Host calls on GB300, ms, before (the reference's expressions over whole
 // tiles) and after: cubed nest 4 K8 7.1 -> 0.38, gradient 7.5 -> 0.43, double dot 13.5 -> 0.48; nest 6
 // K8 37 -> 4.55, Gaussian 12.7 -> 1.65, gradient 40 -> 5.2, divergence 49 -> 6.3, double dot 67 -> 6.8,

@@ -256,9 +256,10 @@ __global__ void prep_plane_i64_kernel(const double* x, const double* y, const do
 // sequential loop.  More lanes give a small target set more warps, for S ceil(NA / S) additions
 // per pair instead of NA (i64_lanes picks S).
 //
-// Bound by the FP64 pipe and the integer pipes together (BVE at icos nest 6, S = 4: the FP64
-// pipe, with 10 instructions a pair where the plain loop has 31, is about 78 % busy, the ALU and
-// IMAD pipes 60 %); a small set by the latency of a pair's chain.  Host calls on GB300,
+// Bound by the FP64 pipe and the integer pipes together (BVE at icos nest 6, S = 4: 10.7 FP64
+// instructions a pair, where the plain loop has 31, are 83 % of the pipe at 49 Ginteractions/s; counters at nest
+// 4, 27 Ginteractions/s: FP64 47 %, ALU 36 % busy; plane at quad nest 6: FP64 78 %, ALU 33 %); a small set by
+// the latency of a pair's chain.  Host calls on GB300,
 // Ginteractions/s, against the same loop in FP64 instructions only: BVE icos nest 3, 4, 5, 6
 // 3.9, 13.1, 15.6, 15.7 -> 6.5, 27.4, 43.7, 49.1; plane quad nest 4, 5, 6 6.8, 21.0, 27.7 ->
 // 10.0, 34.2, 53.6.  Two sources per lane in flight (the same rates) and the final products on
