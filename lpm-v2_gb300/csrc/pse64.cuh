@@ -139,10 +139,11 @@ __device__ __forceinline__ bool odd_point(const CutPoint& p) {
   return !(v == 0.0) || !(p.r >= 0x1p-450 && p.r <= 0x1p450);
 }
 
-// Whether two particles' distances from the sphere's centre are the same to their rounding (within 4
-// units in the last place); a particle that is odd has one that is no other's.
+// Whether two particles' distances from the sphere's centre are the same to their rounding (within 8
+// units in the last place: turned, scaled and renormalised meshes differ by up to 6, and a pair that is not the same
+// takes its warp through the general path); a particle that is odd has one that is no other's.
 __device__ __forceinline__ bool same_radius(long long a, double b) {
-  return static_cast<unsigned long long>(__double_as_longlong(b)) - static_cast<unsigned long long>(a) + 4ull <= 8ull;
+  return static_cast<unsigned long long>(__double_as_longlong(b)) - static_cast<unsigned long long>(a) + 8ull <= 16ull;
 }
 
 // ------------------------------------------------------------------ a pair's kernel value
