@@ -19,7 +19,16 @@
  *  - mode selects the arithmetic:
  *      LPM_MODE_FP64  : FP64, the reference expression association with no fused
  *                       multiply-add, sources swept in ascending index order: results are
- *                       bit-identical to the Fortran loop built without FMA contraction.
+ *                       bit-identical to the Fortran loop built without FMA contraction
+ *                       (velocity sums, SWE velocities and double dot product) or within
+ *                       1e-12 of the largest value where a transcendental function enters.
+ *                       The PSE sums are FP64 throughout but in expressions of their own:
+ *                       within 1e-12 of the largest value, with a root mean square error no
+ *                       larger than the reference expressions'.  They leave out pairs
+ *                       beyond r = distance / eps = 7 (each below 1e-14 of the kernel's
+ *                       peak) when there are more than 256 sources, and add a target's pairs
+ *                       in a fixed order that depends on the sources alone: a block of
+ *                       targets gets the same bits as the whole set.
  *      LPM_MODE_FP32C : pair arithmetic in FP32 with hi/lo positions, chord-form
  *                       denominators, per-tile compensated (TwoSum) accumulation and an
  *                       FP64 cross-tile reduction (velocity relative error <= 1e-6).
@@ -122,8 +131,7 @@ int lpm_pse_sphere_divergence(int64_t n, const double* x, const double* y, const
                               double radius, int64_t i_begin, int64_t i_end, double* div,
                               int mode);
 
-/* The remaining PSE operators have only LPM_MODE_FP64 (the reference's association, like the
- * other FP64 sums); LPM_MODE_FP32C returns LPM_ERR_ARG.  The shallow-water integrals have
+/* The remaining PSE operators have only LPM_MODE_FP64; LPM_MODE_FP32C returns LPM_ERR_ARG.  The shallow-water integrals have
  * both modes. */
 
 /* Replaces PSEPlaneGradientAtParticles (src/PSEDirectSum.f90:180-217): (gx, gy) =
@@ -362,7 +370,9 @@ int lpm_bve_velocity_noalloc(int64_t n, const double* x, const double* y, const 
 /* ------------------------------------------------------------------ workspace and test hooks */
 
 /* Frees the device workspace the host-buffer calls keep between calls (it grows to the
- * largest sum seen and is otherwise held until the process exits).  Synchronous; the next
+ * largest sum seen and is otherwise held until the process exits; the partial sums of an
+ * LPM_MODE_FP32C sum take up to 0.3 to 1.1 GB of it on 152 SMs, 330 MB for the sphere velocity of
+ * 2 million particles).  Synchronous; the next
  * host-buffer call allocates again.  No counterpart in the reference, which has no device
  * memory; the analogue of releasing a cached allocator's free blocks. */
 int lpm_release_workspace(void);
@@ -376,9 +386,8 @@ int lpm_release_workspace(void);
  * released or kept consistent, so the next call succeeds.
  *
  * lpm_debug_inject_wait_timeout(skip_tile, budget_ns): the next host-buffer LPM_MODE_FP32C
- * sphere-BVE sum (lpm_bve_velocity, lpm_bve_set_velocity_from_vorticity; block-synchronous
- * tile pipeline) or sphere PSE sum (lpm_pse_sphere_laplacian, _gradient, _divergence;
- * warp-decoupled pipeline) does not issue the copy of source tile `skip_tile` and bounds its
+ * sphere-BVE sum (lpm_bve_velocity, lpm_bve_set_velocity_from_vorticity) or sphere PSE sum
+ * (lpm_pse_sphere_laplacian, _gradient, _divergence) does not issue the copy of source tile `skip_tile` and bounds its
  * waits by budget_ns (0 < budget_ns <= 1e9) instead of 1 s.  The waits for that tile run out, the call returns LPM_ERR_TIMEOUT with the
  * caller's outputs untouched, and the context stays usable.  Nothing faults: no copy is in
  * flight for the skipped tile.  One-shot. */
