@@ -19,8 +19,8 @@
 //   y = q0 v                    for chords (the factor is in the target's and record's scale),
 //   E = 2^y (2 MUFU, which run at twice the reciprocal's rate), K8 = E (p0 + p1 y + p2 y^2 + p3 y^3),
 //   (f_j - f_i) A_j = A_j F_j - A_j F_i with F the field less a group constant: one FMA forms it from
-//   floats (two more operations with their low parts near the group, where the difference is smaller than
-//   F), and one accumulates its product with K.
+//   floats, and one accumulates its product with K (near the group, where the difference is smaller than F:
+//   F_j - F_i from float pairs in three operations, times A_j K).
 // The kernel is smooth at r = 0, so that no pair needs more than the offsets' 2^-24: a group that is
 // small against eps (R <= 2 eps) takes one form for every target, self pairs included (f_j - f_i =
 // 0).  A wider group (particles far apart against eps, or a set far from its coordinates' origin)
@@ -46,7 +46,7 @@ struct PseLap {
   struct __align__(16) Rec {
     float4 a;  // -sx, -sx, -sy, -sy
     float4 b;  // -sz, -sz, A, A
-    float4 c;  // A F, A F, and the low part of the product, twice
+    float4 c;  // A F, A F, and F as a float pair
     float4 d;  // the offset's low parts -sx, -sy, -sz (wide groups), 0
   };
   struct __align__(16) Group {
@@ -98,8 +98,10 @@ __device__ __forceinline__ float2 lap_kernel(float2 y) {
   return __fmul2_rn(e, p);
 }
 
-// Target pairs [P0, P1) of a warp against one group.  CLOSE: A_j (F_j - F_i) with the low parts of A_j F_j
-// and F_i, for targets so near the group that the difference is smaller than its terms.
+// Target pairs [P0, P1) of a warp against one group.  CLOSE: F_j - F_i from the float pairs, for targets
+// so near the group that the difference is smaller than its terms; both pairs come from the same operations, so
+// a particle's own pair is exactly zero (K is largest there, and a residue of 2^-48 f would be all that a set
+// without neighbours in reach has).
 template <bool SPHERE, bool K8, int ANG, bool CLOSE, int P0, int P1, int NP>
 __device__ __forceinline__ void lap_group(const PseLap::Rec* __restrict__ gr, const float (&q)[7],
                                           const float2 (&tx)[NP], const float2 (&ty)[NP], const float2 (&tz)[NP],
@@ -116,9 +118,12 @@ __device__ __forceinline__ void lap_group(const PseLap::Rec* __restrict__ gr, co
         v = __ffma2_rn(dz, dz, v);
       }
       const float2 k = lap_kernel<K8>(lap_exponent<ANG>(v, q));
-      float2 m = __ffma2_rn(hi2(rb), nf[p], lo2(rc));
-      if (CLOSE) m = __fadd2_rn(__ffma2_rn(hi2(rb), nl[p], hi2(rc)), m);
-      acc[p] = __ffma2_rn(m, k, acc[p]);
+      if (CLOSE) {
+        const float2 m = __fadd2_rn(__fadd2_rn(make_float2(rc.z, rc.z), nf[p]), __fadd2_rn(make_float2(rc.w, rc.w), nl[p]));
+        acc[p] = __ffma2_rn(m, __fmul2_rn(hi2(rb), k), acc[p]);
+      } else {
+        acc[p] = __ffma2_rn(__ffma2_rn(hi2(rb), nf[p], lo2(rc)), k, acc[p]);
+      }
     }
   }
 }
@@ -203,16 +208,18 @@ __global__ void __launch_bounds__(THREADS, MINB) pse_lap_sweep_kernel(PseLapArgs
         if (SPHERE) n2 = __ffma2_rn(tz[p], tz[p], n2);
         // each target pair's 64 targets on their own: consecutive in curve order
         in[p] = __any_sync(0xffffffffu, !(n2.x >= reach * reach) | !(n2.y >= reach * reach));
-        near |= !(n2.x >= close * close) | !(n2.y >= close * close);
-        // -F_i = (f of the group) - f_i as a float, and what that leaves
+        near |= !(n2.x > close * close) | !(n2.y > close * close);  // (a group of radius 0: its own particle)
+        // -F_i = (f of the group) - f_i as a float pair, with the operations of the records
         const float2 fg = make_float2(o.f.x, o.f.x), mf = make_float2(-fh[p].x, -fh[p].y),
                      ml = make_float2(-fl[p].x, -fl[p].y);
         const float2 s = __fadd2_rn(fg, mf);
-        nf[p] = __fadd2_rn(s, ml);
-        const float2 b = __fadd2_rn(s, make_float2(-fg.x, -fg.y));  // TwoSum of fg and mf, then of ml
+        const float2 b = __fadd2_rn(s, make_float2(-fg.x, -fg.y));  // TwoSum of fg and mf
         const float2 e = __fadd2_rn(__fadd2_rn(fg, __fadd2_rn(b, make_float2(-s.x, -s.y))),
                                     __fadd2_rn(mf, make_float2(-b.x, -b.y)));
-        nl[p] = __fadd2_rn(__fadd2_rn(__fadd2_rn(s, make_float2(-nf[p].x, -nf[p].y)), ml), e);
+        const float2 r = __fadd2_rn(e, ml);  // |r| <= |s| or s = 0
+        nf[p] = __fadd2_rn(s, r);
+        const float2 d = __fadd2_rn(nf[p], make_float2(-s.x, -s.y));
+        nl[p] = __fadd2_rn(r, make_float2(-d.x, -d.y));
       }
       if (!in[0] && !in[1]) continue;  // every pair has r^2 > 49
       if (o.f.y == 0.f) {
@@ -253,8 +260,8 @@ __global__ void __launch_bounds__(THREADS, MINB) pse_lap_sweep_kernel(PseLapArgs
             v = __ffma2_rn(dz, dz, v);
           }
           const float2 k = lap_kernel<K8>(lap_exponent<ANG>(v, a.q));
-          const float2 m = __fadd2_rn(__ffma2_rn(hi2(rb), nl[p], hi2(rc)), __ffma2_rn(hi2(rb), nf[p], lo2(rc)));
-          acc[p] = __ffma2_rn(m, k, acc[p]);
+          const float2 m = __fadd2_rn(__fadd2_rn(make_float2(rc.z, rc.z), nf[p]), __fadd2_rn(make_float2(rc.w, rc.w), nl[p]));
+          acc[p] = __ffma2_rn(m, __fmul2_rn(hi2(rb), k), acc[p]);
         }
       }
       flush();
@@ -389,10 +396,10 @@ __global__ void __launch_bounds__(TILE) pse_lap_prep_kernel(const double* x, con
     float d, de, fs, fe;
     two_sum(fh, -fg, d, de);
     two_sum(d, de + fl, fs, fe);
-    const float af = ar * fs, al = fmaf(ar, fs, -af) + ar * fe;
+    const float af = ar * fs;
     r.a = make_float4(-hi[0], -hi[0], -hi[1], -hi[1]);
     r.b = make_float4(-hi[2], -hi[2], ar, ar);
-    r.c = make_float4(af, af, al, al);
+    r.c = make_float4(af, af, fs, fe);
     r.d = make_float4(-lo[0], -lo[1], -lo[2], 0.f);
   } else {
     r.a = r.b = r.c = r.d = make_float4(0.f, 0.f, 0.f, 0.f);  // zero area: no contribution

@@ -257,23 +257,20 @@ def test_log1p_form_of_far_groups():
 # ------------------------------------------------------------------ Laplacians
 @pytest.mark.parametrize("mean", [0.0, 1.0, 1e6])
 def test_field_difference_of_the_laplacians_pair(mean):
-    """A_j (f_j - f_i) as A F_j - A F_i with F the field less the group's constant, low parts included."""
+    """F_j - F_i from float pairs of the field less the group's constant; a particle's own pair is zero."""
     rng = np.random.default_rng(3)
-    f, a = mean + rng.normal(size=33), rng.uniform(0.5, 1.5, 32)
+    f = mean + rng.normal(size=64)
     fh, fl = _split2(f)
-    ar, fg = a.astype(F), fh[0]
-    s, e = _two_sum(fh[:32], np.full(32, -fg))
-    e = e + fl[:32]
-    fs = s + e  # renormalised before it is rounded
-    fe = (s - fs) + e
-    af = ar * fs
-    al = _fma(ar, fs, -af) + ar * fe
-    s, b = _two_sum(np.array([fg]), -fh[32:])
-    nf = s - fl[32:]
-    nl = ((s - nf) - fl[32:]) + b
-    m = _fma(ar, np.full(32, nl[0]), al) + _fma(ar, np.full(32, nf[0]), af)
-    exact = a * (f[:32] - f[32])
-    assert np.abs(m - exact).max() <= 2.0**-22 * np.abs(exact).max() + 2.0**-46 * abs(mean)
+    s, e = _two_sum(fh, np.full(64, -fh[0]))  # the records'
+    fs, fe = _two_sum(s, e + fl)
+    s, e = _two_sum(np.full(64, fh[0]), -fh)  # the targets'
+    r = e - fl
+    nf = s + r
+    nl = r - (nf - s)
+    m = (fs + nf[:, None]) + (fe + nl[:, None])
+    assert np.all(np.diag(m) == 0.0)
+    exact = f - f[:, None]
+    assert np.abs(m - exact).max() <= 2.0**-23 * np.abs(exact).max() + 2.0**-47 * abs(mean)
 
 
 def test_laplacian_kernel_in_the_exponents_unit():
