@@ -79,7 +79,9 @@ struct PseRelComps {
   static constexpr int value = OP == kPseOpGrad ? 3 : 1;
 };
 
-// Position of particle i as the operator uses it.
+// Position of particle i as the operator uses it.  A particle at the sphere's centre has no direction; it
+// stays there, a unit from every other (its pairs are then nothing for any eps below 0.1 a), instead of
+// making its own sum, and as a source its group's, NaN.
 template <int ANG>
 __device__ __forceinline__ void pse_position(const double* x, const double* y, const double* z, int64_t i,
                                              double inv_a, double& px, double& py, double& pz) {
@@ -87,7 +89,8 @@ __device__ __forceinline__ void pse_position(const double* x, const double* y, c
   py = y[i] * inv_a;
   pz = z[i] * inv_a;
   if (ANG != kPseAngleChord) {
-    const double s = 1.0 / sqrt(fma(px, px, fma(py, py, pz * pz)));
+    const double n2 = fma(px, px, fma(py, py, pz * pz));
+    const double s = n2 > 0.0 ? 1.0 / sqrt(n2) : 1.0;
     px *= s;
     py *= s;
     pz *= s;
