@@ -84,3 +84,18 @@ def test_shells_against_the_oracle(lg, oracle_mod):
         ref = oracle_mod.pse_laplacian(*p, f[0], area, active, 0.05, 1.0, kernel=0, ib=ib, ie=ie)
         got = lg.pse_sphere_laplacian_at_particles(*p, f[0], area, active, 0.05, 1.0, i_begin=ib + 1, i_end=ie, mode="fp64")
         assert np.abs(got[s] - ref).max() <= 1e-12 * np.abs(ref).max()
+
+
+# 8, 4, 4 and 2 lanes per target on 152 SMs
+@pytest.mark.parametrize("ns", [7295, 7296, 14591, 14592])
+def test_every_lane_count(lg, oracle_mod, ns):
+    rng = np.random.default_rng(ns)
+    p = rng.normal(size=(3, 15000))
+    p /= np.linalg.norm(p, axis=0)
+    f, area = rng.normal(size=15000), rng.uniform(0.5, 1.5, 15000) / 15000
+    active = (rng.permutation(15000) < ns).astype(np.int32)
+    for kernel in (0, 1):
+        ref = oracle_mod.pse_laplacian(*p, f, area, active, 0.05, 1.0, kernel=kernel, ib=700, ie=1200)
+        got = lg.pse_sphere_laplacian_at_particles(*p, f, area, active, 0.05, 1.0, kernel=kernel, i_begin=701, i_end=1200,
+                                                   mode="fp64")
+        assert np.abs(got[700:1200] - ref).max() <= 1e-12 * np.abs(ref).max()
