@@ -16,10 +16,10 @@
 //    bits; a self pair cancels bit for bit.
 // A compact group (R <= a/2 and R <= 32 x its smallest spacing h, i.e. a patch of a
 // quasi-uniform point set) takes one-subtraction differences for every target: its records use
-// rel2_fast, the target's far-form operations, so a self pair still cancels bit for bit.  For a target near such a group the roundings are an absolute
-// 2^-24 R inside the near-field sum sum_j S_j / |d_j|^2, which grows only like ln(1/h) on a
-// quasi-uniform set, so the velocity error scales with R, not R/h (1.0e-7 relative at
-// icosahedral nest 8).  Groups that fail the test (clustered or sparse points) keep the
+// rel2_fast, the target's far-form operations, so a self pair still cancels bit for bit.
+// For a target near such a group the roundings are an absolute 2^-24 R inside the near-field sum
+// sum_j S_j / |d_j|^2, which grows only like ln(1/h) on a quasi-uniform set, so the velocity error
+// scales with R, not R/h (1.0e-7 relative at icosahedral nest 8).  Groups that fail the test (clustered or sparse points) keep the
 // near/far choice, whose error bound holds for any point distribution.
 // Particle order along the mesh or the curve keeps a warp's targets close together, so a
 // warp meets few near groups (at icosahedral nest 8 three in a thousand).
@@ -39,8 +39,8 @@
 // B_j/2 - t.s_j and four sums) took 8, 2 and 4.  Any basis does: the records solve for (a, b, c) in
 // the rounded one, alpha = t.e1 + o.e1 carries the group constant o.e1 (about 2^-25), and gamma =
 // |o|^2 + k - ct, C = ct + k with ct = (|t|^2 - c_i)/2 and k = (1 - |o|^2)/2, so no term loses
-// digits: C and the products are at most a few h at the 3R boundary, and q stays within a few ulps.  A compact group with a target of the warp near it keeps d = t_hi - s_hi
-// (10-11 operations; it contains the self pairs), any other near group the two-float form (17).
+// digits: C and the products are at most a few h at the 3R boundary, and q stays within a few ulps.
+// A compact group with a target of the warp near it keeps d = t_hi - s_hi (10-11 operations; it contains the self pairs), any other near group the two-float form (17).
 // Forming the targets' offsets, projections and the near test cost about 25 per pair and group.
 // Targets keep their original order (only sources are sorted), so no scatter is needed.
 #pragma once

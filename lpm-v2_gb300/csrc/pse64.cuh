@@ -14,14 +14,14 @@
 //    function, ACM TOMS 15, 1989): with s = 256 q / ln 2 and i = round(s),
 //    E = 2^-(i / 256) 2^-((s - i) / 256), a table of 256 powers and a polynomial of degree 4
 //    (remainder 4e-17).
-// That is about 33 FP64 instructions a pair for K8 of the great-circle distance, where the
+// That is about 32 FP64 instructions a pair for K8 of the great-circle distance, where the
 // reference's expressions take about 150.  The results agree with the reference's to its own rounding
 // (1e-15 of the largest; its exp and atan2 are not CUDA's either): root mean square error against the sums in
 // extended precision, as a share of the reference expressions' own, at cubed nest 5: K8 0.58, gradient 0.60,
 // divergence 0.87; 0.57, 0.66 and 0.98 for particles 1e-7 off the sphere (pairs of rounded unit directions
-// and kernel polynomials in s, with rounded coefficients, gave 1.4 to 3 times the reference's error).  A lane's sum is in the
-// reference's ascending order; a target has 2 to 8 lanes, each summing its part of every tile, and adds the
-// parts at the end.  How many follows from the sources alone, so that a target's bits do not depend on
+// and kernel polynomials in s, with rounded coefficients, gave 1.4 to 3 times the reference's error).
+// A lane's sum is in the reference's ascending order; a target has 2 to 8 lanes, each summing its part of
+// every tile, and adds the parts at the end.  How many follows from the sources alone, so that a target's bits do not depend on
 // which other targets a call has.
 //
 // At r >= 7 each kernel (its polynomial times e^-49) is below 1e-14 of its peak, and the sum
@@ -39,11 +39,10 @@
 // whose particles differ by more than a quarter in their distance from the centre, takes the reference's
 // expressions as they stand (Op::Plain), as do all pairs of a reach beyond the polynomials' range.
 //
-// Bound by the FP64 pipe (2 lanes per clock per SM): 74 % busy for K8 and 70 % for the
-// gradient at cubed nest 6, the rest being
-// the last warps of an SM.  Host calls on GB300, ms, before (the reference's expressions over whole
+// Bound by the FP64 pipe (2 lanes per clock per SM): 74 % busy for K8 and 71 % for the
+// gradient at cubed nest 6, the rest being the last warps of an SM.  Host calls on GB300, ms, before (the reference's expressions over whole
 // tiles) and after: cubed nest 4 K8 7.1 -> 0.38, gradient 7.5 -> 0.43, double dot 13.5 -> 0.48; nest 6
-// K8 37 -> 4.55, Gaussian 12.7 -> 1.65, gradient 40 -> 5.2, divergence 49 -> 6.3, double dot 67 -> 6.8,
+// K8 37 -> 4.40, Gaussian 12.7 -> 1.64, gradient 40 -> 5.1, divergence 49 -> 6.3, double dot 67 -> 6.8,
 // interpolation 37 -> 4.6; quad nest 6 K8 7.3 -> 1.2, gradient 8.4 -> 1.3, second partials 11.5 -> 1.5.
 #pragma once
 
@@ -65,11 +64,14 @@ constexpr int64_t kPse64AllPairs = 4 * kPse64Tile;
 enum { kAngNone = 0, kAngNear = 1, kAngFar = 2, kAngWide = 3 };
 constexpr double kAngNearMax = 0.45, kAngFarMax = 1.13, kAngWideMax = 3.15;  // the largest reach (radians)
 
-__device__ constexpr double kAngleNear[9] = {
+// (theta / c)^2 as polynomials in c^2.  The first two reach the kernel multiplied by the q of a squared
+// angle (Pse64Args::ang).
+constexpr int kAngNearN = 9, kAngFarN = 16;
+constexpr double kAngleNear[9] = {
     1.0, 0x1.5555555555528p-4, 0x1.6c16c16c21e06p-7, 0x1.d41d41c32ba47p-10,
     0x1.4ce1a15af67f7p-12, 0x1.f85ad3dada806p-15, 0x1.8f6711cda66fbp-17, 0x1.3f8984fdb3592p-19,
     0x1.4ec6f7c8931fap-21};
-__device__ constexpr double kAngleFar[16] = {
+constexpr double kAngleFar[16] = {
     1.0, 0x1.555555555557dp-4, 0x1.6c16c16c11ab3p-7, 0x1.d41d41d8335acp-10,
     0x1.4ce19a0a71d18p-12, 0x1.f85dcd29033f7p-15, 0x1.8f0a574238fa0p-17, 0x1.46295d746cb2fp-19,
     0x1.0de9a232ae937p-21, 0x1.f9dd6ab3b186cp-24, 0x1.678acc7911957p-27, 0x1.3377469b31787p-26,
@@ -94,6 +96,7 @@ struct Pse64Src {
 
 struct Pse64Args {
   double c;               // q per squared distance (chord) or squared angle
+  double ang[kAngFarN];   // c times the near or the far angle polynomial
   double scale, unscale;  // what divides the kernel's polynomial (pi, powers of eps), and its inverse
   double reach;           // of the cutoff, in the test space
   int unit;               // 1: the test space is unit directions
@@ -155,26 +158,30 @@ __device__ __forceinline__ double horner(const double (&c)[N], double v) {
   return p;
 }
 
-// 4 asin^2(c / 2) from v = c^2.
+// q from the squared distance or squared chord v.
 template <int ANG>
-__device__ __forceinline__ double angle2(double v) {
-  if (ANG == kAngNone) return v;
-  if (ANG == kAngNear) return v * horner(kAngleNear, v);
-  if (ANG == kAngFar) return v * horner(kAngleFar, v);
-  if (v <= 2.0) return v * horner(kAngleWide, v);
+__device__ __forceinline__ double pse64_q(const Pse64Args& a, double v) {
+  if constexpr (ANG == kAngNear || ANG == kAngFar) {
+    constexpr int N = ANG == kAngNear ? kAngNearN : kAngFarN;
+    double p = a.ang[N - 1];
+#pragma unroll
+    for (int k = N - 2; k >= 0; --k) p = fma(p, v, a.ang[k]);
+    return __dmul_rn(v, p);
+  }
+  if (ANG == kAngNone) return __dmul_rn(v, a.c);
+  if (v <= 2.0) return __dmul_rn(v * horner(kAngleWide, v), a.c);
   // beyond 90 degrees: the supplement's angle (a kernel that reaches there has eps < 0.45, so
   // that near the antipode, where this loses digits, it is below e^-40)
   const double w = fmax(4.0 - v, 0.0);
   const double t = 3.14159265358979323846 - sqrt(w * horner(kAngleWide, w));
-  return t * t;
+  return __dmul_rn(t * t, a.c);
 }
 
-// The kernel (without what divides its polynomial) at q = c v.  The polynomial is in q, where its
+// The kernel (without what divides its polynomial) at q.  The polynomial is in q, where its
 // coefficients are exact: in s, their roundings were common to all pairs of a sum, whose moments cancel.
 template <class Op>
-__device__ __forceinline__ double pse64_kernel_value(double v, double c, const double* powers) {
+__device__ __forceinline__ double pse64_kernel_value(double q, const double* powers) {
   const double big = 6755399441055744.0;  // 1.5 x 2^52: the sum's low word is round(s)
-  const double q = __dmul_rn(v, c);
   const double t = fma(q, kPse64PerQ, big);
   const int i = __double2loint(t);
   const double f = fma(q, kPse64PerQ, __dsub_rn(big, t));
@@ -574,7 +581,7 @@ __global__ void __launch_bounds__(32) pse64_sweep_kernel(typename Op::Params p, 
       return;
     }
     const double3 d = offset(n);
-    const double w = pse64_kernel_value<Op>(angle2<ANG>(squared(n, d, regular(n))), a.c, powers);
+    const double w = pse64_kernel_value<Op>(pse64_q<ANG>(a, squared(n, d, regular(n))), powers);
     Op::add(t, n, d.x, d.y, d.z, w, acc);
   };
   int held = 0;  // entries of mine and tile_of that this lane holds
@@ -610,8 +617,8 @@ __global__ void __launch_bounds__(32) pse64_sweep_kernel(typename Op::Params p, 
         continue;
       }
       const double3 d0 = offset(n0), d1 = offset(n1);
-      const double w0 = pse64_kernel_value<Op>(angle2<ANG>(squared(n0, d0, true)), a.c, powers);
-      const double w1 = pse64_kernel_value<Op>(angle2<ANG>(squared(n1, d1, true)), a.c, powers);
+      const double w0 = pse64_kernel_value<Op>(pse64_q<ANG>(a, squared(n0, d0, true)), powers);
+      const double w1 = pse64_kernel_value<Op>(pse64_q<ANG>(a, squared(n1, d1, true)), powers);
       Op::add(t, n0, d0.x, d0.y, d0.z, w0, acc);
       Acc more = acc;
       Op::add(t, n1, d1.x, d1.y, d1.z, w1, more);

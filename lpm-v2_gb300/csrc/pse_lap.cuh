@@ -11,8 +11,8 @@
 //
 // Layout: sources and targets in curve order.  A group of kGroup sources has an origin o near its
 // centroid (in the plane with a low part: far from the coordinates' origin a float alone would make every
-// group wide, and at a shift of 1e8 a sum at quad nest 7 took 3.9 ms instead of 0.5); positions (unit directions for the great circle, x / a for the chord, x in the plane)
-// are held relative to it.  A pair needs only the exponent's base-2 argument y = -r^2 log2 e:
+// group wide, and at a shift of 1e8 a sum at quad nest 7 took 3.9 ms instead of 0.5); positions (unit directions for
+// the great circle, x / a for the chord, x in the plane) are held relative to it.  A pair needs only the exponent's base-2 argument y = -r^2 log2 e:
 //   v = |t - s|^2 from the offsets (3 + 3 packed FP32x2 operations; 2 + 2 in the plane),
 //   y = v (q0 + q1 v + ...)     for the great circle, theta^2 = 4 asin^2(sqrt(v) / 2) as a polynomial
 //                               interpolated at Chebyshev nodes (within 5e-9; v <= 0.2 or 1.3),

@@ -295,7 +295,8 @@ __global__ void finish_stream_kernel(const double* partial, int64_t nsplit, int6
   }
 }
 
-// The FP64 kinds whose kernel decays as exp(-r^2) (the PSE operators, pse64.cuh); *unit tells whether the distance is a great-circle one.
+// The FP64 kinds whose kernel decays as exp(-r^2) (the PSE operators, pse64.cuh); *unit tells whether the
+// distance is a great-circle one.
 bool fp64_cutoff(int kind, int* unit) {
   switch (kind) {
     case kSumPseK8Geo:
@@ -900,6 +901,8 @@ int launch_pse64(const SumJob& job, const SumPlan& plan, const typename Op::Para
     a.reach = 1e300;
     if (unit) ang = kAngWide;
   }
+  for (int k = 0; k < kAngFarN; ++k)
+    a.ang[k] = ang == kAngFar ? a.c * kAngleFar[k] : (k < kAngNearN ? a.c * kAngleNear[k] : 0.0);
   a.x = job.x;
   a.y = job.y;
   a.z = job.z;
